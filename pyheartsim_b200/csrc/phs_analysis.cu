@@ -406,6 +406,8 @@ __global__ void __launch_bounds__(kAThreads) cv_solve(long long ne, const long l
 
 }  // namespace
 
+using phs::dev_alloc;
+using phs::dev_free;
 using phs::set_last_error;
 
 extern "C" {
@@ -472,13 +474,13 @@ int phs_conduction_velocity(int64_t ne, const double* xyz, const double* lat, do
     long long* off = nullptr;
     double* ws = nullptr;
     auto done = [&](int rc) {
-        if (ws) cudaFreeAsync(ws, s);
-        if (off) cudaFreeAsync(off, s);
-        if (counts) cudaFreeAsync(counts, s);
+        dev_free(ws, s);
+        dev_free(off, s);
+        dev_free(counts, s);
         cudaStreamSynchronize(s);
         return rc;
     };
-    cudaError_t e = cudaMallocAsync((void**)&counts, (size_t)ne * sizeof(int32_t), s);
+    cudaError_t e = dev_alloc((void**)&counts, (size_t)ne * sizeof(int32_t), s);
     if (e == cudaSuccess) {
         cv_count<<<blocks_for(ne), kAThreads, 0, s>>>(ne, xyz, r2, counts);
         e = cudaGetLastError();
@@ -494,10 +496,10 @@ int phs_conduction_velocity(int64_t ne, const double* xyz, const double* lat, do
         h_off[(size_t)i] = total;
         total += h_counts[(size_t)i];
     }
-    e = cudaMallocAsync((void**)&off, (size_t)ne * sizeof(long long), s);
+    e = dev_alloc((void**)&off, (size_t)ne * sizeof(long long), s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(off, h_off.data(), (size_t)ne * sizeof(long long),
                                               cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&ws, (size_t)(5 * (total > 0 ? total : 1)) * sizeof(double), s);
+    if (e == cudaSuccess) e = dev_alloc((void**)&ws, (size_t)(5 * (total > 0 ? total : 1)) * sizeof(double), s);
     if (e == cudaSuccess) {
         cv_fill<<<blocks_for(ne), kAThreads, 0, s>>>(ne, xyz, lat, r2, off, counts, total, ws);
         cv_solve<<<(unsigned int)ne, kAThreads, 0, s>>>(ne, off, counts, total, ws, v_vec, v_mag);

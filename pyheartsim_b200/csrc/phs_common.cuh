@@ -17,6 +17,13 @@ void set_last_error(const char* where, cudaError_t e);
 // Record a plain error message for phs_last_error().
 void set_last_message(const char* msg);
 
+// Device memory from the library's pool of the current device, ordered on
+// `stream` (phs_pool.cu); dev_free accepts null.
+cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t stream);
+void dev_free(void* p, cudaStream_t stream);
+// Sets how much the pool keeps; `engines`: engines made (+1) or destroyed (-1).
+void pool_update(int engines);
+
 }  // namespace phs
 
 #define PHS_CUDA_TRY(expr)                                   \

@@ -166,14 +166,14 @@ int contract_f64(int64_t T, int64_t n_v, int64_t n_e, const double* V, int64_t l
     kchunk = ((kchunk + DG_BK - 1) / DG_BK) * DG_BK;
     splits = (n_v + kchunk - 1) / kchunk;
     double* P = nullptr;
-    PHS_CUDA_TRY(cudaMallocAsync((void**)&P, (size_t)splits * T * n_e * sizeof(double), stream));
+    PHS_CUDA_TRY(dev_alloc((void**)&P, (size_t)splits * T * n_e * sizeof(double), stream));
     dim3 grid((unsigned)tm, (unsigned)tn, (unsigned)splits);
     dgemm_tn_kernel<<<grid, 256, 0, stream>>>(T, n_e, n_v, V, ldv, Mt, n_v, P, kchunk);
     const int64_t MN = T * n_e;
     splitk_reduce_kernel<double><<<(unsigned)std::min<int64_t>((MN + 255) / 256, 4096), 256, 0, stream>>>(
         MN, (int)splits, P, egm);
     cudaError_t e = cudaGetLastError();
-    cudaFreeAsync(P, stream);
+    dev_free(P, stream);
     if (e != cudaSuccess) { set_last_error("contract_f64", e); return PHS_ERR_CUDA; }
     return PHS_OK;
 }
@@ -206,7 +206,7 @@ int contract_f64_into(int64_t T, int64_t n_v, int64_t n_e, const double* V, int6
 
 int normalize(int64_t T, int64_t n_e, void* egm, bool is_f64, cudaStream_t stream) {
     double* ptp = nullptr;
-    PHS_CUDA_TRY(cudaMallocAsync((void**)&ptp, (size_t)n_e * sizeof(double), stream));
+    PHS_CUDA_TRY(dev_alloc((void**)&ptp, (size_t)n_e * sizeof(double), stream));
     const int64_t total = T * n_e;
     const unsigned blocks = (unsigned)std::min<int64_t>((total + 255) / 256, 2048);
     if (is_f64) {
@@ -217,7 +217,7 @@ int normalize(int64_t T, int64_t n_e, void* egm, bool is_f64, cudaStream_t strea
         scale_kernel<float><<<blocks, 256, 0, stream>>>(total, n_e, ptp, (float*)egm);
     }
     cudaError_t e = cudaGetLastError();
-    cudaFreeAsync(ptp, stream);
+    dev_free(ptp, stream);
     if (e != cudaSuccess) { set_last_error("normalize", e); return PHS_ERR_CUDA; }
     return PHS_OK;
 }
@@ -305,12 +305,12 @@ int phs_electrogram(int64_t T, int64_t n_v, int64_t n_e, const double* V, const 
     std::vector<void*> bufs;
     auto alloc = [&](size_t bytes) -> void* {
         void* p = nullptr;
-        if (cudaMalloc(&p, std::max<size_t>(bytes, 16)) != cudaSuccess) return nullptr;
+        if (dev_alloc(&p, std::max<size_t>(bytes, 16), s) != cudaSuccess) return nullptr;
         bufs.push_back(p);
         return p;
     };
     auto cleanup = [&](int rc) {
-        for (void* p : bufs) cudaFree(p);
+        for (void* p : bufs) dev_free(p, s);
         return rc;
     };
     double* dV = (double*)alloc((size_t)T * n_v * 8);

@@ -1937,11 +1937,22 @@ struct InstHost {
     unsigned long long prof_ref[16] = {};
 };
 
+// The engine's device for as long as the guard lives (an engine may be
+// destroyed from a thread that has another device current).
+struct DeviceGuard {
+    int old = -1;
+    explicit DeviceGuard(int device) {
+        if (cudaGetDevice(&old) != cudaSuccess || old == device || cudaSetDevice(device) != cudaSuccess) old = -1;
+    }
+    ~DeviceGuard() {
+        if (old >= 0) cudaSetDevice(old);
+    }
+};
+
 void free_inst(InstHost& h) {
     void* ptrs[] = {h.nb, h.nbr, h.nbase, h.coef, h.cw, h.m6, h.enb, h.ecf, h.dx, h.vflags, h.vparams, h.stim, h.u, h.h0, h.h1, h.x, h.b, h.V,
                     h.hist_u, h.hist_h, h.lat, h.part, h.gpart, h.gcnt, h.sc, h.sync, h.st, h.prof};
-    for (void* p : ptrs)
-        if (p) cudaFree(p);
+    for (void* p : ptrs) dev_free(p, 0);
     h = InstHost();
 }
 
@@ -2117,7 +2128,7 @@ __global__ void nb_compact(long long n, const int32_t* nb, const T* coef, const 
 // alloc_n >= n elements (the tail is zero).
 template <typename T>
 int upload_converted(void** dst, const double* src, long long n, bool on_device, long long alloc_n) {
-    PHS_CUDA_TRY(cudaMalloc(dst, (size_t)alloc_n * sizeof(T)));
+    PHS_CUDA_TRY(dev_alloc(dst, (size_t)alloc_n * sizeof(T), 0));
     if (alloc_n > n) PHS_CUDA_TRY(cudaMemset((char*)*dst + (size_t)n * sizeof(T), 0, (size_t)(alloc_n - n) * sizeof(T)));
     if (sizeof(T) == 8) {
         PHS_CUDA_TRY(cudaMemcpy(*dst, src, (size_t)n * 8, cudaMemcpyDefault));
@@ -2126,7 +2137,7 @@ int upload_converted(void** dst, const double* src, long long n, bool on_device,
     double* tmp = nullptr;
     cudaError_t e = cudaSuccess;
     if (!on_device) {
-        PHS_CUDA_TRY(cudaMalloc(&tmp, (size_t)n * 8));
+        PHS_CUDA_TRY(dev_alloc((void**)&tmp, (size_t)n * 8, 0));
         e = cudaMemcpy(tmp, src, (size_t)n * 8, cudaMemcpyHostToDevice);
     }
     if (e == cudaSuccess) {
@@ -2134,7 +2145,7 @@ int upload_converted(void** dst, const double* src, long long n, bool on_device,
         convert_kernel<T><<<(unsigned)std::max<long long>(blocks, 1), 256>>>(on_device ? src : tmp, (T*)*dst, n);
         e = cudaDeviceSynchronize();
     }
-    if (tmp) cudaFree(tmp);
+    dev_free(tmp, 0);
     if (e != cudaSuccess) { set_last_error("upload_converted", e); return PHS_ERR_CUDA; }
     return PHS_OK;
 }
@@ -2176,7 +2187,7 @@ template <typename T>
 int build_compact_nb(InstHost& h) {
     const long long n = h.n;
     unsigned int* d_w = nullptr;
-    PHS_CUDA_TRY(cudaMalloc((void**)&d_w, 8 * sizeof(unsigned int)));
+    PHS_CUDA_TRY(dev_alloc((void**)&d_w, 8 * sizeof(unsigned int), 0));
     unsigned int w[8] = {};
     cudaError_t ce = cudaMemset(d_w, 0, 8 * sizeof(unsigned int));
     const long long blocks = std::max<long long>(1, std::min<long long>((n + 255) / 256, 4096));
@@ -2188,8 +2199,8 @@ int build_compact_nb(InstHost& h) {
     if (ce == cudaSuccess) ce = cudaMemcpy(w, d_w, 8 * sizeof(unsigned int), cudaMemcpyDeviceToHost);
     if (ce == cudaSuccess && !(w[0] & 1u) && !(w[1] & 2u)) {
         const long long nblk = h.ldv / 512;
-        ce = cudaMalloc((void**)&h.nbr, (size_t)h.ldv * 4 * sizeof(int16_t));
-        if (ce == cudaSuccess) ce = cudaMalloc((void**)&h.nbase, (size_t)nblk * 4 * sizeof(int32_t));
+        ce = dev_alloc((void**)&h.nbr, (size_t)h.ldv * 4 * sizeof(int16_t), 0);
+        if (ce == cudaSuccess) ce = dev_alloc((void**)&h.nbase, (size_t)nblk * 4 * sizeof(int32_t), 0);
         if (ce == cudaSuccess) ce = cudaMemset(d_w + 6, 0, sizeof(unsigned int));
         if (ce == cudaSuccess) {
             nb_compact<T><<<(unsigned)nblk, 256>>>(n, (const int32_t*)h.nb, (const T*)h.coef, (const T*)h.cw,
@@ -2198,13 +2209,13 @@ int build_compact_nb(InstHost& h) {
         }
         if (ce == cudaSuccess) ce = cudaMemcpy(w + 6, d_w + 6, sizeof(unsigned int), cudaMemcpyDeviceToHost);
         if (ce != cudaSuccess || w[6] != 0u) {
-            if (h.nbr) cudaFree(h.nbr);
-            if (h.nbase) cudaFree(h.nbase);
+            dev_free(h.nbr, 0);
+            dev_free(h.nbase, 0);
             h.nbr = nullptr;
             h.nbase = nullptr;
         }
     }
-    cudaFree(d_w);
+    dev_free(d_w, 0);
     if (ce != cudaSuccess) { set_last_error("build_compact_nb", ce); return PHS_ERR_CUDA; }
     return PHS_OK;
 }
@@ -2229,8 +2240,8 @@ int add_instance(phs_engine* e, const phs_instance_desc* d, int* slot) {
     auto fail = [&](int code) { free_inst(h); return code; };
 #define PHS_ALLOC(ptr, bytes)                                            \
     do {                                                                 \
-        cudaError_t _e = cudaMalloc((void**)&(ptr), (bytes));            \
-        if (_e != cudaSuccess) { set_last_error("cudaMalloc", _e); return fail(PHS_ERR_OOM); } \
+        cudaError_t _e = dev_alloc((void**)&(ptr), (bytes), 0);          \
+        if (_e != cudaSuccess) { set_last_error("dev_alloc", _e); return fail(PHS_ERR_OOM); } \
     } while (0)
     // tables: host arrays, or device arrays when device_tables (cudaMemcpyDefault)
     const bool dev = d->device_tables != 0;
@@ -2263,7 +2274,7 @@ int add_instance(phs_engine* e, const phs_instance_desc* d, int* slot) {
     if (dev) {
         // the checks validate_desc makes on host tables, on the copies
         unsigned int* d_err = nullptr;
-        if (cudaMalloc((void**)&d_err, sizeof(unsigned int)) != cudaSuccess) return fail(PHS_ERR_OOM);
+        if (dev_alloc((void**)&d_err, sizeof(unsigned int), 0) != cudaSuccess) return fail(PHS_ERR_OOM);
         unsigned int h_err = 0;
         cudaError_t ce = cudaMemset(d_err, 0, sizeof(unsigned int));
         if (ce == cudaSuccess) {
@@ -2274,7 +2285,7 @@ int add_instance(phs_engine* e, const phs_instance_desc* d, int* slot) {
             ce = cudaGetLastError();
         }
         if (ce == cudaSuccess) ce = cudaMemcpy(&h_err, d_err, sizeof(h_err), cudaMemcpyDeviceToHost);
-        cudaFree(d_err);
+        dev_free(d_err, 0);
         if (ce != cudaSuccess) { set_last_error("check_tables", ce); return fail(PHS_ERR_CUDA); }
         if (h_err) return fail(PHS_ERR_BAD_TABLE);
     }
@@ -2340,10 +2351,11 @@ int add_instance(phs_engine* e, const phs_instance_desc* d, int* slot) {
         if (!e->inst[i].used) { s = (int)i; break; }
     if (s < 0) { s = (int)e->inst.size(); e->inst.push_back(InstHost()); }
     if (e->profile) {
-        if (cudaMalloc((void**)&h.prof, kProfSlots * sizeof(unsigned long long)) == cudaSuccess)
+        if (dev_alloc((void**)&h.prof, kProfSlots * sizeof(unsigned long long), 0) == cudaSuccess)
             cudaMemset(h.prof, 0, kProfSlots * sizeof(unsigned long long));
     }
     e->inst[s] = h;
+    pool_update(0);
     e->dirty = true;
     e->auto_left = 2;
     e->auto_mark = e->launches;
@@ -2510,8 +2522,10 @@ int build_plan(phs_engine* e, int cps, bool edge) {
     for (int i : act) descs.push_back(make_dev<T>(e->inst[i], e->group_sums, vpt, e->compact_nb));
     size_t bytes = descs.size() * sizeof(InstDev<T>);
     if (bytes > e->d_desc_bytes) {
-        if (e->d_desc) cudaFree(e->d_desc);
-        PHS_CUDA_TRY(cudaMalloc(&e->d_desc, bytes));
+        dev_free(e->d_desc, 0);
+        e->d_desc = nullptr;
+        e->d_desc_bytes = 0;
+        PHS_CUDA_TRY(dev_alloc(&e->d_desc, bytes, 0));
         e->d_desc_bytes = bytes;
     }
     PHS_CUDA_TRY(cudaMemcpy(e->d_desc, descs.data(), bytes, cudaMemcpyHostToDevice));
@@ -2548,8 +2562,10 @@ int build_plan(phs_engine* e, int cps, bool edge) {
         waves.push_back({off, grid});
     }
     if (map_all.size() > e->d_map_n) {
-        if (e->d_map) cudaFree(e->d_map);
-        PHS_CUDA_TRY(cudaMalloc(&e->d_map, map_all.size() * sizeof(int4)));
+        dev_free(e->d_map, 0);
+        e->d_map = nullptr;
+        e->d_map_n = 0;
+        PHS_CUDA_TRY(dev_alloc((void**)&e->d_map, map_all.size() * sizeof(int4), 0));
         e->d_map_n = map_all.size();
     }
     PHS_CUDA_TRY(cudaMemcpy(e->d_map, map_all.data(), map_all.size() * sizeof(int4), cudaMemcpyHostToDevice));
@@ -2672,27 +2688,30 @@ int phs_engine_create(int precision, phs_engine** out) {
     e->prec = precision;
     cudaError_t ce = cudaGetDevice(&e->device);
     if (ce == cudaSuccess) ce = cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, e->device);
-    if (ce == cudaSuccess) ce = cudaMalloc(&e->abort_word, sizeof(unsigned int));
+    if (ce == cudaSuccess) ce = dev_alloc((void**)&e->abort_word, sizeof(unsigned int), 0);
     if (ce == cudaSuccess) ce = cudaMemset(e->abort_word, 0, sizeof(unsigned int));
     if (ce != cudaSuccess) {
         set_last_error("phs_engine_create", ce);
-        if (e->abort_word) cudaFree(e->abort_word);
+        dev_free(e->abort_word, 0);
         delete e;
         return PHS_ERR_CUDA;
     }
+    pool_update(1);
     *out = e;
     return PHS_OK;
 }
 
 int phs_engine_destroy(phs_engine* e) {
     if (!e) return PHS_ERR_BAD_ARG;
+    DeviceGuard guard(e->device);
     cudaDeviceSynchronize();
     drop_graphs(e);
     for (auto& h : e->inst)
         if (h.used) free_inst(h);
-    if (e->abort_word) cudaFree(e->abort_word);
-    if (e->d_desc) cudaFree(e->d_desc);
-    if (e->d_map) cudaFree(e->d_map);
+    dev_free(e->abort_word, 0);
+    dev_free(e->d_desc, 0);
+    dev_free(e->d_map, 0);
+    pool_update(-1);
     delete e;
     return PHS_OK;
 }
@@ -2704,8 +2723,10 @@ int phs_instance_add(phs_engine* e, const phs_instance_desc* d, int* slot) {
 
 int phs_instance_remove(phs_engine* e, int slot) {
     if (!e || slot < 0 || slot >= (int)e->inst.size() || !e->inst[slot].used) return PHS_ERR_BAD_ARG;
+    DeviceGuard guard(e->device);
     cudaDeviceSynchronize();
     free_inst(e->inst[slot]);
+    pool_update(0);
     e->dirty = true;
     e->auto_left = 2;
     e->auto_mark = e->launches;
@@ -2842,11 +2863,11 @@ int set_profile(phs_engine* e, bool on) {
     for (auto& h : e->inst) {
         if (!h.used) continue;
         if (e->profile && !h.prof) {
-            if (cudaMalloc((void**)&h.prof, kProfSlots * sizeof(unsigned long long)) != cudaSuccess)
+            if (dev_alloc((void**)&h.prof, kProfSlots * sizeof(unsigned long long), 0) != cudaSuccess)
                 return PHS_ERR_OOM;
         }
         if (h.prof) cudaMemset(h.prof, 0, kProfSlots * sizeof(unsigned long long));
-        if (!e->profile && h.prof) { cudaFree(h.prof); h.prof = nullptr; }
+        if (!e->profile && h.prof) { dev_free(h.prof, 0); h.prof = nullptr; }
         for (int i = 0; i < kProfSlots; ++i) h.prof_ref[i] = 0;
     }
     e->dirty = true;

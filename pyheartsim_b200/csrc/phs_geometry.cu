@@ -321,6 +321,8 @@ __global__ void pacing_bits(const int64_t* __restrict__ ids, long long count, lo
 
 }  // namespace
 
+using phs::dev_alloc;
+using phs::dev_free;
 using phs::set_last_error;
 using phs::set_last_message;
 
@@ -336,10 +338,10 @@ int phs_lattice_neighbors(int64_t n, const int32_t* ijk, int32_t* nb18, int32_t*
     int32_t* counts = nullptr;
     int rc = PHS_OK;
     auto cleanup = [&]() {
-        if (counts) cudaFreeAsync(counts, s);
-        if (grid) cudaFreeAsync(grid, s);
-        if (d_err) cudaFreeAsync(d_err, s);
-        if (d_mm) cudaFreeAsync(d_mm, s);
+        dev_free(counts, s);
+        dev_free(grid, s);
+        dev_free(d_err, s);
+        dev_free(d_mm, s);
         cudaStreamSynchronize(s);
     };
 #define GEO_TRY(expr)                                                  \
@@ -351,8 +353,8 @@ int phs_lattice_neighbors(int64_t n, const int32_t* ijk, int32_t* nb18, int32_t*
             return _e == cudaErrorMemoryAllocation ? PHS_ERR_OOM : PHS_ERR_CUDA; \
         }                                                              \
     } while (0)
-    GEO_TRY(cudaMallocAsync((void**)&d_mm, sizeof(h_mm), s));
-    GEO_TRY(cudaMallocAsync((void**)&d_err, sizeof(unsigned int), s));
+    GEO_TRY(dev_alloc((void**)&d_mm, sizeof(h_mm), s));
+    GEO_TRY(dev_alloc((void**)&d_err, sizeof(unsigned int), s));
     GEO_TRY(cudaMemcpyAsync(d_mm, h_mm, sizeof(h_mm), cudaMemcpyHostToDevice, s));
     GEO_TRY(cudaMemsetAsync(d_err, 0, sizeof(unsigned int), s));
     bbox_kernel<<<grid_for(n), kGeoThreads, 0, s>>>(ijk, n, d_mm);
@@ -379,14 +381,14 @@ int phs_lattice_neighbors(int64_t n, const int32_t* ijk, int32_t* nb18, int32_t*
         return PHS_ERR_UNSUPPORTED;
     }
     const long long cells = span[0] * span[1] * span[2];
-    GEO_TRY(cudaMallocAsync((void**)&grid, (size_t)cells * sizeof(int32_t), s));
+    GEO_TRY(dev_alloc((void**)&grid, (size_t)cells * sizeof(int32_t), s));
     fill_i32<<<grid_for(cells), kGeoThreads, 0, s>>>(grid, cells, -1);
     scatter_kernel<<<grid_for(n), kGeoThreads, 0, s>>>(ijk, n, b, grid, d_err);
     gather_kernel<<<grid_for(n), kGeoThreads, 0, s>>>(ijk, n, b, grid, nb18);
     GEO_TRY(cudaGetLastError());
     if (order) {
         const long long chunks = (cells + kChunkCells - 1) / kChunkCells;
-        GEO_TRY(cudaMallocAsync((void**)&counts, (size_t)chunks * sizeof(int32_t), s));
+        GEO_TRY(dev_alloc((void**)&counts, (size_t)chunks * sizeof(int32_t), s));
         chunk_count<<<(unsigned int)chunks, kGeoThreads, 0, s>>>(grid, cells, counts);
         scan_counts<<<1, kGeoThreads, 0, s>>>(counts, chunks);
         chunk_order<<<(unsigned int)chunks, kGeoThreads, 0, s>>>(grid, cells, counts, order);
@@ -417,7 +419,7 @@ int phs_operator_flags(int64_t n, const double* P, int32_t* out3, void* stream) 
     if (n <= 0 || !P || !out3) return PHS_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     unsigned int* d = nullptr;
-    PHS_CUDA_TRY(cudaMallocAsync((void**)&d, sizeof(unsigned int), s));
+    PHS_CUDA_TRY(dev_alloc((void**)&d, sizeof(unsigned int), s));
     unsigned int h = 0;
     cudaError_t e = cudaMemsetAsync(d, 0, sizeof(unsigned int), s);
     if (e == cudaSuccess) {
@@ -425,7 +427,7 @@ int phs_operator_flags(int64_t n, const double* P, int32_t* out3, void* stream) 
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, s);
-    cudaFreeAsync(d, s);
+    dev_free(d, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { set_last_error("phs_operator_flags", e); return PHS_ERR_CUDA; }
     out3[0] = (h & 1u) != 0;
@@ -442,7 +444,7 @@ int phs_operator_tables(phs_operator_tables_args* a) {
     cudaStream_t s = (cudaStream_t)a->stream;
     const long long n = a->n_voxel;
     unsigned int* d_err = nullptr;
-    PHS_CUDA_TRY(cudaMallocAsync((void**)&d_err, sizeof(unsigned int), s));
+    PHS_CUDA_TRY(dev_alloc((void**)&d_err, sizeof(unsigned int), s));
     unsigned int h_err = 0, one = 1u;
     cudaError_t e = cudaMemsetAsync(d_err, 0, sizeof(unsigned int), s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(a->iso_word, &one, sizeof(one), cudaMemcpyHostToDevice, s);
@@ -463,7 +465,7 @@ int phs_operator_tables(phs_operator_tables_args* a) {
     unsigned int iso = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h_err, d_err, sizeof(h_err), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&iso, a->iso_word, sizeof(iso), cudaMemcpyDeviceToHost, s);
-    cudaFreeAsync(d_err, s);
+    dev_free(d_err, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { set_last_error("phs_operator_tables", e); return PHS_ERR_CUDA; }
     a->iso = iso != 0;
