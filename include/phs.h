@@ -82,7 +82,9 @@ typedef struct phs_instance_desc {
     int32_t n_samples;        /* history length S                                           */
     int32_t save_h;           /* also keep the gate history                                 */
     int32_t full_cycles;      /* 1: CuPy GMRES semantics (full restart cycles, true-residual
-                                 test at each cycle start); 0: Givens early exit            */
+                                 test at each cycle start; a cycle whose residual estimate
+                                 is below rounding level, half a unit roundoff of ||b||, ends
+                                 there as on a breakdown); 0: Givens early exit             */
     double u0, h0;            /* initial state (MS: 0,1; AP: 0,0)                           */
     double tol, atol;         /* stop when ||r|| <= max(atol, tol*||b||)                    */
     int32_t maxiter;          /* Arnoldi steps per solve before giving up (reference 10000) */
