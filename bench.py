@@ -30,7 +30,7 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "voxel-steps/s batched FP32 vs plain FP64 on 1 B200 at LAT err<=dt; p99 latency"
-DEFAULT_F32_VARIANT = 2        # the engine's FP32 default when the autotuner is off
+DEFAULT_F32_VARIANT = 7        # the engine's FP32 default when the autotuner is off
 # DRAM bytes per voxel-step of step_kernel measured by ncu (dram__bytes_read.sum +
 # dram__bytes_write.sum of the two timed full-size launches of this batch, 2.71
 # Arnoldi steps per step, profiles/step_kernel_64shells_dram_fullsize.md), for

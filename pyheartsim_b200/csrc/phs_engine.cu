@@ -42,8 +42,8 @@ namespace phs {
 
 // ------------------------------------------------------------------ device types
 struct alignas(128) TeamSync {
-    unsigned int count;
-    unsigned int gen;
+    unsigned int count;    // arrivals since the launch began
+    unsigned int exits;    // CTAs that have left
     unsigned int pad[30];
 };
 
@@ -64,23 +64,9 @@ enum Phase : int { PH_PLAIN = 0, PH_RHS = 1, PH_DOTS = 2, PH_NORM = 3, PH_CHECK 
 enum ProfSlot : int {
     PF_RHS = 0, PF_RHS_WAIT, PF_A, PF_A_WAIT, PF_C, PF_C_WAIT, PF_X, PF_CHECK, PF_CHECK_WAIT,
     PF_COPY, PF_RHS1, PF_STEPS, PF_SOLVE_ITERS, PF_TEAM,
-    PF_LEADER,      // time in the leader bodies of the team's barriers (whichever CTA led)
+    PF_LEADER,      // time between a barrier's end and its decision: sums of the partials, solver scalars
     PF_BARRIERS,    // team barriers passed
     kProfSlots = 16
-};
-
-struct Scalars {
-    double R[(kMaxRestart + 1) * kMaxRestart];  // column j at R[j*(kMaxRestart+1) + i]
-    double cs[kMaxRestart];
-    double sn[kMaxRestart];
-    double g[kMaxRestart + 1];
-    double s[kMaxRestart + 1];      // v_j = s_j * V_j
-    double coef[kMaxRestart + 1];   // coefficients published for the next phase
-    double bnorm, atol_eff, rnorm, est;
-    int action;
-    int k;
-    int iters_solve;                // Arnoldi steps of the current solve
-    int iters_cap;                  // CuPy-style iteration count (restart per cycle)
 };
 
 struct InstState {
@@ -115,27 +101,31 @@ struct InstDev {
     T* x;
     T* b;
     T* V;                   // [(m+1)*n]
-    T* dx;                  // [n] last diffusion increment (extrapolated initial guess), or nullptr
+    T* ud;                  // [ldv*2] pairs (u*, last diffusion increment; 0 without the extrapolated guess)
     T* hist_u;              // [S*n]
     T* hist_h;              // [S*n] or nullptr
     int32_t* lat;           // [n]
-    double* part;           // [n_tiles*kSlots]
-    double* gpart;          // FP64: [n_groups*kSlots] sums of kGroupTiles consecutive tiles, or nullptr
-    unsigned int* gcnt;     // FP64: [n_groups] arrivals of the current phase at each group
-    Scalars* sc;
+    double* part;           // two buffers of part_half partial sums, [group][slot]
     TeamSync* sync;
     InstState* st;
     unsigned long long* prof;  // [kProfSlots] phase timers (CTA rank 0 of the team), or nullptr
     T params[5];
     T dt, half_dt, jmag;
     double tol, atol;
+    // Chebyshev basis: interval centre and half width, T_1(-theta / delta), and
+    // K_1 = (A - theta) K_0 / delta = cheb_a K_0 + cheb_b L K_0
+    double theta, delta, t1;
+    T cheb_a, cheb_b;
     long long n;
     long long ldv;          // padded voxel count (multiple of kPadVoxels): stride of V, length of per-voxel arrays
     long long n_steps;
     long long tb_steps;
+    long long part_half;
     int n_tiles;
-    int n_groups;           // ceil(n_tiles / kGroupTiles)
-    int ps;                 // partial slots per (tile, warp): m + 2
+    int gt;                 // consecutive tiles of a group (the unit of the partial sums and of the CTAs' work)
+    int n_groups;           // ceil(n_tiles / gt)
+    int cheb;               // solves use the Chebyshev basis (cheb_rule), else Arnoldi
+    int guess;
     int model;
     int m;                  // restart length actually used: min(restart, n)
     int maxiter;
@@ -239,13 +229,13 @@ __device__ __forceinline__ void prefetch_l2(const void* p, unsigned int bytes) {
 
 // ------------------------------------------------------------------ staging ring
 // Staged step kernels (RING > 0) add one producer warp to the 256 consumer
-// threads.  For every tile loop of a phase the consumers publish a job (the
-// arrays the phase streams and their bytes per voxel); the producer copies
-// each of the CTA's tiles' contiguous slices of every array into a stage of a
-// shared-memory ring with 1-D cp.async.bulk, signalled on the stage's "full"
-// mbarrier, and refills a stage once all consumer warps have arrived on its
-// "empty" mbarrier.  Consumers read the tile from shared memory; the stencil's
-// neighbour gathers and the scattered accesses stay on global memory.
+// threads.  For the update pass the consumers publish a job (the arrays the pass
+// streams and their bytes per voxel); the producer copies each of the CTA's
+// tiles' contiguous slices of every array into a stage of a shared-memory ring
+// with 1-D cp.async.bulk, signalled on the stage's "full" mbarrier, and refills
+// a stage once all consumer warps have arrived on its "empty" mbarrier.
+// Consumers read the tile from shared memory; the passes that gather neighbours
+// and the scattered accesses stay on global memory.
 constexpr int kStageMaxArr = 12;    // arrays per stage
 constexpr int kMaxStages = 6;       // ring depth limit
 constexpr int kRingHeader = 1024;   // barriers and jobs ahead of the ring in dynamic shared memory
@@ -257,7 +247,7 @@ struct StageJob {
     int n_arr;
     int stage_bytes;
     int n_stages;
-    int tile0, step, n_tiles;       // the CTA's tiles: tile0, tile0 + step, ... < n_tiles
+    int tile0, step, gt, n_tiles;   // the CTA's groups of gt tiles: tile0, tile0 + step, ...; tiles < n_tiles
     int quit;
 };
 struct RingHeader {
@@ -364,10 +354,10 @@ struct Stager {
         const int c = (RING / 2 - lay_off) / (TILE * (int)sizeof(T));
         return max(0, min(c, kStageMaxArr - lay_n));
     }
-    __device__ __forceinline__ int publish(int rank, int P, int n_tiles) {
+    __device__ __forceinline__ int publish(int rank, int P, int n_tiles, int n_groups, int gt) {
         nst = (lay_off > 0 && lay_n <= kStageMaxArr) ? RING / lay_off : 0;
         if (nst > kMaxStages) nst = kMaxStages;
-        if (rank >= n_tiles) nst = 0;
+        if (rank >= n_groups) nst = 0;
         if (nst == 0) return 0;
         if (threadIdx.x == 0) {
             StageJob& J = rh->job[job_buf];
@@ -376,6 +366,7 @@ struct Stager {
             J.n_stages = nst;
             J.tile0 = rank;
             J.step = P;
+            J.gt = gt;
             J.n_tiles = n_tiles;
             J.quit = 0;
         }
@@ -405,78 +396,48 @@ struct Stager {
 };
 
 struct SharedCtl {
-    int last;
-    unsigned int gen;
-    int action;
-    int k;
     int abort;
-    double sj;
-    double bnorm;
+    int action;
+    int k;            // basis vectors of the update that follows
+    int settled;      // the cycle's estimate is below rounding level (kSettled)
+    double bnorm, atol_eff;
+    double sj;        // Arnoldi: scale of the column the next pass applies A to
+    double sz;        // Chebyshev basis: sum of z_i^2
 };
 
-// Bounded team barrier.  The last CTA to arrive runs `leader` (whole CTA)
-// before releasing the others.  Returns false when the wait gave up or another
-// team aborted; the kernel then leaves all loops.
+// Bounded team barrier: every CTA of the team arrives on one counter and polls
+// it until the team's `target` is reached.  No CTA leads: what a barrier
+// combines (partial sums, solver scalars) every CTA computes for itself from
+// the partials, in the same order and so to the same bits.  That takes three
+// dependent L2 round trips out of a barrier (the leader's read of the partials,
+// its release and the waiters' read of its results): 5.3-7.5 us with a leader
+// that reduced, 3.0-4.2 us now, the reduction included (40 to 157 CTAs).
 //
-// The release word carries, besides a barrier counter (bits 9-31), the
-// action (bits 0-2) and cycle length k (bits 3-8) the leader left in `sc`, so
-// the waiting CTAs learn them from the load that releases them (ctl.action,
-// ctl.k).  Ordering: the arrival is an acq_rel RMW (the CTA's writes, made
-// visible to thread 0 by the CTA barrier and the fence, precede it; the
-// leader's RMW acquires every earlier arrival); the release is a release store
-// and the waiters' polls are acquire loads.
-constexpr unsigned int kGenShift = 9;
-template <bool ST, typename Leader>
-__device__ __forceinline__ bool team_sync(TeamSync* ts, int P, unsigned int* abort_word, SharedCtl& ctl,
-                                          const Scalars* sc, unsigned long long* prof, Leader&& leader) {
+// Ordering: the arrival is a release RMW after a CTA barrier (cumulative over
+// the CTA's writes), the poll an acquire load, followed by a CTA barrier.
+// Returns false when the wait gave up or another team aborted; the kernel then
+// leaves all loops.  A team of one CTA needs its own CTA barrier only.
+template <bool ST>
+__device__ __forceinline__ bool team_barrier(TeamSync* ts, int P, unsigned int target, unsigned int* abort_word,
+                                             SharedCtl& ctl) {
     csync<ST>();
+    if (P == 1) return true;
     if (threadIdx.x == 0) {
-        cuda::atomic_ref<unsigned int, cuda::thread_scope_device> gen(ts->gen);
         cuda::atomic_ref<unsigned int, cuda::thread_scope_device> cnt(ts->count);
-        unsigned int g = gen.load(cuda::memory_order_relaxed);
-        __threadfence();
-        unsigned int a = cnt.fetch_add(1u, cuda::memory_order_acq_rel);
-        ctl.last = (a == (unsigned int)(P - 1));
-        ctl.gen = g;
-        ctl.abort = 0;
-    }
-    csync<ST>();
-    if (ctl.last) {
-        const unsigned long long tl = (prof && threadIdx.x == 0) ? global_ns() : 0ull;
-        leader();
-        csync<ST>();
-        if (threadIdx.x == 0) {
-            if (prof) {
-                atomicAdd(prof + PF_LEADER, global_ns() - tl);
-                atomicAdd(prof + PF_BARRIERS, 1ull);
-            }
-            cuda::atomic_ref<unsigned int, cuda::thread_scope_device> gen(ts->gen);
-            cuda::atomic_ref<unsigned int, cuda::thread_scope_device> cnt(ts->count);
-            const int act = __ldcg(&sc->action), k = __ldcg(&sc->k);
-            ctl.action = act;
-            ctl.k = k;
-            cnt.store(0u, cuda::memory_order_relaxed);
-            const unsigned int word = ((((ctl.gen >> kGenShift) + 1u) << kGenShift)) | ((unsigned int)(k & 63) << 3) |
-                                      (unsigned int)(act & 7);
-            gen.store(word, cuda::memory_order_release);
-        }
-    } else if (threadIdx.x == 0) {
-        cuda::atomic_ref<unsigned int, cuda::thread_scope_device> gen(ts->gen);
-        cuda::atomic_ref<unsigned int, cuda::thread_scope_device> ab(*abort_word);
-        unsigned long long t0 = global_ns();
-        unsigned int polls = 0;
-        unsigned int word;
-        while ((word = gen.load(cuda::memory_order_acquire)) == ctl.gen) {
+        cnt.fetch_add(1u, cuda::memory_order_release);
+        unsigned long long t0 = 0;
+        for (unsigned int polls = 0; (int)(cnt.load(cuda::memory_order_acquire) - target) < 0; ++polls) {
+            if ((polls & 63u) != 63u) continue;
+            cuda::atomic_ref<unsigned int, cuda::thread_scope_device> ab(*abort_word);
+            const unsigned long long now = global_ns();
+            if (t0 == 0) t0 = now;
             if (ab.load(cuda::memory_order_relaxed) != 0u) { ctl.abort = 1; break; }
-            if (++polls > kWaitPolls || global_ns() - t0 > kWaitNs) {
+            if (polls > kWaitPolls || now - t0 > kWaitNs) {
                 ab.fetch_or(1u, cuda::memory_order_relaxed);
                 ctl.abort = 1;
                 break;
             }
-            __nanosleep(64);
         }
-        ctl.action = (int)(word & 7u);
-        ctl.k = (int)((word >> 3) & 63u);
     }
     csync<ST>();
     return ctl.abort == 0;
@@ -515,84 +476,206 @@ __device__ __forceinline__ void decode_nb(short4 r, int4 b, long long n, int32_t
     q[5] = nn + b.w + r.w;
 }
 
-// Coefficients of row n: one common value and a presence mask for isotropic
-// rows (D0 = I gives c_n / Delta^2 on every present neighbour), else six values.
+// One value, or the pair (u*, last diffusion increment), per voxel.
 template <typename T>
-__device__ __forceinline__ void row_coef(const T* coef, const T* cw, const uint8_t* m6, long long n, T (&c)[6]) {
-    if (cw) {
-        const T w = cw[n];
-        const unsigned mk = __ldg(m6 + n);
+struct Pair;
+template <>
+struct Pair<float> { using type = float2; };
+template <>
+struct Pair<double> { using type = double2; };
+template <typename T>
+using PairT = typename Pair<T>::type;
+
+__device__ __forceinline__ float lap_zero(float) { return 0.f; }
+__device__ __forceinline__ double lap_zero(double) { return 0.0; }
+__device__ __forceinline__ float2 lap_zero(float2) { return make_float2(0.f, 0.f); }
+__device__ __forceinline__ double2 lap_zero(double2) { return make_double2(0.0, 0.0); }
+// s += g - o
+__device__ __forceinline__ void add_diff(float& s, float g, float o) { s += g - o; }
+__device__ __forceinline__ void add_diff(double& s, double g, double o) { s += g - o; }
+__device__ __forceinline__ void add_diff(float2& s, float2 g, float2 o) { s.x += g.x - o.x; s.y += g.y - o.y; }
+__device__ __forceinline__ void add_diff(double2& s, double2 g, double2 o) { s.x += g.x - o.x; s.y += g.y - o.y; }
+// s += c * (g - o)
+template <typename T>
+__device__ __forceinline__ void add_scaled(T& s, T c, T g, T o) { s += c * (g - o); }
+__device__ __forceinline__ void add_scaled(float2& s, float c, float2 g, float2 o) {
+    s.x += c * (g.x - o.x);
+    s.y += c * (g.y - o.y);
+}
+__device__ __forceinline__ void add_scaled(double2& s, double c, double2 g, double2 o) {
+    s.x += c * (g.x - o.x);
+    s.y += c * (g.y - o.y);
+}
+template <typename T>
+__device__ __forceinline__ T times(T c, T s) { return c * s; }
+__device__ __forceinline__ float2 times(float c, float2 s) { return make_float2(c * s.x, c * s.y); }
+__device__ __forceinline__ double2 times(double c, double2 s) { return make_double2(c * s.x, c * s.y); }
+
+// Matrix-free rows of L applied to `vec` at the thread's voxels n0 + v * kThreads
+// of a tile (own[v] = vec there).  Nothing is stored in between, so the loads
+// of all VPT voxels (tables, then gathers) are in flight together: with a store
+// after each voxel, as this was written before, every voxel waited for its own
+// table and gathers in turn.  No bounds test: the per-voxel arrays are padded
+// to whole tiles with zeros, and a row of zero coefficients reads itself.
+// Isotropic rows (D0 = I: one coefficient c_n / Delta^2 on every present
+// neighbour) sum the differences first; other rows have six coefficients, and
+// the edge cross terms of simulation/simulation_gpu.py:199-217 as six
+// antisymmetric pairs.  NB: 0 int32 table, 1 compact table, 2 the instance's.
+template <typename T, int VPT, bool EDGE, int NB, typename V>
+__device__ __forceinline__ void tile_lap(const InstDev<T>& I, const V* vec, long long n0, bool tb, const V (&own)[VPT],
+                                         V (&lap)[VPT]) {
+    const bool compact = NB == 1 || (NB == 2 && I.nbr != nullptr);
+    if (I.cw) {
+        unsigned mk[VPT];
+        T w[VPT];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) c[k] = ((mk >> k) & 1u) ? w : T(0);
+        for (int v = 0; v < VPT; ++v) {
+            const long long n = n0 + v * kThreads;
+            mk[v] = __ldg(I.m6 + n);
+            w[v] = __ldg(I.cw + n);
+            // a zero coefficient reads nothing: its stored offset may be anything
+            if (w[v] == T(0) || (tb && (__ldg(I.vflags + n) & PHS_VFLAG_TBLOCK))) mk[v] = 0u;
+        }
+#pragma unroll
+        for (int v = 0; v < VPT; ++v) {
+            const long long n = n0 + v * kThreads;
+            int32_t q[6];
+            if (compact)
+                decode_nb(__ldg(reinterpret_cast<const short4*>(I.nbr) + n),
+                          __ldg(reinterpret_cast<const int4*>(I.nbase) + (n >> 9)), n, q);
+            else
+                load_nb(I.nb, n, q);
+            V g[6];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) g[k] = vec[((mk[v] >> k) & 1u) ? q[k] : (int32_t)n];
+            V s = lap_zero(own[v]);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) add_diff(s, g[k], own[v]);
+            lap[v] = times(w[v], s);
+        }
     } else {
-        load_coef(coef, n, c);
+#pragma unroll
+        for (int v = 0; v < VPT; ++v) {
+            const long long n = n0 + v * kThreads;
+            int32_t q[6];
+            T c[6];
+            if (compact)
+                decode_nb(__ldg(reinterpret_cast<const short4*>(I.nbr) + n),
+                          __ldg(reinterpret_cast<const int4*>(I.nbase) + (n >> 9)), n, q);
+            else
+                load_nb(I.nb, n, q);
+            load_coef(I.coef, n, c);
+            V g[6];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) g[k] = vec[c[k] != T(0) ? q[k] : (int32_t)n];
+            V s = lap_zero(own[v]);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) add_scaled(s, c[k], g[k], own[v]);
+            if (EDGE && I.ecf) {
+                const int4* pi = reinterpret_cast<const int4*>(I.enb + 12 * n);
+                const int4 i0 = __ldg(pi), i1 = __ldg(pi + 1), i2 = __ldg(pi + 2);
+                const int32_t e[12] = {i0.x, i0.y, i0.z, i0.w, i1.x, i1.y, i1.z, i1.w, i2.x, i2.y, i2.z, i2.w};
+                load_coef(I.ecf, n, c);
+                V a[6], b[6];
+#pragma unroll
+                for (int p = 0; p < 6; ++p) {
+                    a[p] = vec[c[p] != T(0) ? e[2 * p] : (int32_t)n];
+                    b[p] = vec[c[p] != T(0) ? e[2 * p + 1] : (int32_t)n];
+                }
+#pragma unroll
+                for (int p = 0; p < 6; ++p) add_scaled(s, c[p], a[p], b[p]);
+            }
+            if (tb && (__ldg(I.vflags + n) & PHS_VFLAG_TBLOCK)) s = lap_zero(own[v]);
+            lap[v] = s;
+        }
     }
 }
 
-// Matrix-free row of L applied to `vec` at voxel n (coefficients already loaded);
-// all six gathers are issued before they are combined.
-template <typename T>
-__device__ __forceinline__ T lap_row(const T* vec, T vn, const int32_t (&q)[6], const T (&c)[6]) {
-    T g[6];
+// Sums of N values over a warp, N a power of two: the halves of the value list
+// go to the halves of the warp at each exchange, so N sums take N - 1 + 5 -
+// log2(N) exchanges instead of 5 N.  Lane l returns the sum of value
+// l >> (5 - log2(N)); the order of the additions is fixed.
+template <int N>
+__device__ __forceinline__ double warp_sums(double (&v)[N], int lane) {
+    int off = 16;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) g[k] = (c[k] != T(0)) ? vec[q[k]] : vn;
-    T acc = T(0);
+    for (int h = N / 2; h >= 1; h /= 2) {
+        const bool up = (lane & off) != 0;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) acc += c[k] * (g[k] - vn);
-    return acc;
-}
-
-// Edge cross terms of an anisotropic row n (simulation/simulation_gpu.py:199-217):
-// six antisymmetric pairs ecf[p] * (vec[a_p] - vec[b_p]); all gathers first.
-template <typename T>
-__device__ __forceinline__ T edge_row(const T* vec, const int32_t* enb, const T* ecf, long long n) {
-    const int4* pi = reinterpret_cast<const int4*>(enb + 12 * n);
-    const int4 i0 = __ldg(pi), i1 = __ldg(pi + 1), i2 = __ldg(pi + 2);
-    const int32_t q[12] = {i0.x, i0.y, i0.z, i0.w, i1.x, i1.y, i1.z, i1.w, i2.x, i2.y, i2.z, i2.w};
-    T g[6];
-    load_coef(ecf, n, g);
-    T va[6], vb[6];
-#pragma unroll
-    for (int p = 0; p < 6; ++p) {
-        va[p] = (g[p] != T(0)) ? vec[q[2 * p]] : T(0);
-        vb[p] = (g[p] != T(0)) ? vec[q[2 * p + 1]] : T(0);
+        for (int i = 0; i < h; ++i) {
+            const double send = up ? v[i] : v[i + h];
+            const double keep = up ? v[i + h] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+        off /= 2;
     }
-    T acc = T(0);
-#pragma unroll
-    for (int p = 0; p < 6; ++p) acc += g[p] * (va[p] - vb[p]);
-    return acc;
+    for (; off >= 1; off /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+    return v[0];
 }
+__host__ __device__ constexpr int log2_of(int n) { return n <= 1 ? 0 : 1 + log2_of(n / 2); }
 
-
-// Basis vectors whose loads are issued together: FP32 tiles hold four voxels
-// per thread (four loads per vector already), FP64 tiles one, and the FP64
-// plain form's GMRES(50) cycles pass over up to 50 vectors per phase, so its
-// chunks are four times longer to keep as many loads in flight.
+// Basis vectors whose loads are issued together: FP32 tiles hold two or four
+// voxels per thread (as many loads per vector), FP64 tiles one, and the FP64
+// plain form passes over some twenty vectors per column.
 template <typename T>
 constexpr int kChunkOf = sizeof(T) == 8 ? 16 : 4;
-template <typename T>
-constexpr bool kWarpParts = sizeof(T) == 4;
 // A full GMRES cycle ends early once its residual estimate is at most this
 // fraction of ||b||: half a unit roundoff of the stored type.  A is I - dt/2 L
 // with eigenvalues of 1 and above, so what the remaining columns could add to x
 // is below a rounding of x; besides, classical Gram-Schmidt has lost the basis'
 // orthogonality by then (|v_0 . v_j| of 0.1 to 1 where the estimate passes this
 // line) and those columns are rounding noise.  On the sheet and shell runs the
-// line is crossed after 18-23 of 50 columns with the error against the exact
+// line is crossed after 18-26 of 50 columns with the error against the exact
 // solution unchanged (2.5e-16 relative at column 21 and at column 50); at
 // larger steps (dt/2 max(-L_nn) above ~5) it is not reached and the cycle runs
 // to its end.
 template <typename T>
 constexpr double kSettled = sizeof(T) == 8 ? 5.5511151231257827e-17 : 2.9802322387695312e-08;
-// FP64 partial sums are combined in fixed groups of this many consecutive tiles
-// by whichever CTA finishes a group's last tile, so the leader reads one
-// partial per group (GMRES(50) reduces up to 51 slots per barrier).
-constexpr int kGroupTiles = 8;
-constexpr int kMaxGroupWalk = 32;   // tiles a CTA counts in per pass
+
+// A full cycle in the Chebyshev basis whose true residual is above this fraction
+// of ||b|| (rounding level of the residual itself is 1-2e-16 ||b||) is followed by
+// a few columns more: where r0 is near ||b|| (the edges of a fresh stimulus) the
+// roundings of the three-term recurrence, which scale with r0, are above those
+// of b (1.4e-15 ||b|| at r0 = 0.3 ||b||, 2e-16 after).
+template <typename T>
+constexpr double kRefine = sizeof(T) == 8 ? 4.4408920985006262e-16 : 2.384185791015625e-07;
+
+// Partial sums are kept per group of consecutive tiles (one tile, more for
+// instances of more than this many tiles), whatever CTA a group falls to, so
+// that no team has to read many of them: every CTA sums all groups.
+constexpr int kMaxGroupsF32 = 640, kMaxGroupsF64 = 444;
+constexpr int kRedDoubles = 16 * kSlots;      // warp sums a CTA holds back before it combines them
+constexpr int kTri = (kMaxRestart + 1) * (kMaxRestart + 2) / 2;
+__device__ __forceinline__ int tri(int row) { return row * (row + 1) / 2; }
+
+// Below this share of <K_j, K_j> the part of K_j outside the span of the
+// earlier vectors is zero (breakdown) or lost to rounding.
+constexpr double kPivot = 1e-12;
 
 // ------------------------------------------------------------------ the kernel
+// Each solve (I - dt/2 L) x = b is restarted GMRES, in one of two forms:
+//
+//  Chebyshev basis (I.cheb, the rule is cheb_rule's): the Krylov vectors are
+//  K_j = T_j((A - theta) / delta) r0 for the interval [theta - delta, theta +
+//  delta] that Gershgorin's theorem gives for A, a basis well enough conditioned
+//  to be used without orthogonalising it.  Column j is ONE pass over the voxels
+//  (K_{j+1} from K_j and K_{j-1}, and its dots with every K_i) and ONE team
+//  barrier.  From the Gram matrix G of the dots (FP64) every CTA keeps
+//  W = R^-T, G = R^T R, and z = W t, t_i = T_i(-theta / delta): with the
+//  residuals written as sum c_i K_i under sum c_i t_i = 1 (a polynomial that is
+//  1 at 0), the GMRES residual is 1 / ||z|| and its coefficients W^T z /
+//  ||z||^2.  The iterates, estimates and column counts are those of Arnoldi
+//  GMRES (FP32: solutions agree to 1e-8, estimates to 3 digits at tol 1e-7;
+//  FP64: to 1e-15), which needed two passes and two barriers per column, the
+//  second pass to orthogonalise.  200 x 200 sheet: FP32 70 -> 33 us per step of
+//  3 columns, FP64 460 -> 190 us per step of 21.
+//
+//  Arnoldi with classical Gram-Schmidt (the others: stiff steps with long
+//  cycles): phase A applies A and takes the dots, phase C orthogonalises.
+//
 // EDGE: the launch carries anisotropic instances (edge cross terms); the
-// isotropic launches compile without that code.
+// isotropic launches compile without that code.  RING > 0: a producer warp
+// copies the update pass's slices into a shared-memory ring.
 template <typename T, int VPT, int MINB, bool EDGE, int RING, bool NBC>
 __global__ void __launch_bounds__(kThreads + (RING > 0 ? 32 : 0), MINB)
 step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_map,
@@ -601,17 +684,26 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
     static_assert(!ST || sizeof(T) == 4, "staged kernels are FP32");
     // NBC: every instance of the launch has a compact neighbour table (decode_nb)
     static_assert(!(ST && NBC), "staged kernels choose the table per instance");
+    constexpr int NB = ST ? 2 : (NBC ? 1 : 0);
     constexpr int TILE = kThreads * VPT;
     constexpr int kChunk = kChunkOf<T>;
+    using P2 = PairT<T>;
     const int4 cm = cta_map[blockIdx.x];
     const int rank = cm.y;
     const int P = cm.z;
 
     __shared__ InstDev<T> I;
     __shared__ SharedCtl ctl;
-    __shared__ double shc[kMaxRestart + 1];
     __shared__ long long sh_step0;
     __shared__ int sh_id_save, sh_pending, sh_hbuf, sh_status;
+    // solver scalars: R^-T of the Gram matrix or R of the Hessenberg QR (both
+    // triangular), vectors over the columns
+    __shared__ double tm[kTri];
+    __shared__ double va[kMaxRestart + 2], vb[kMaxRestart + 2], vc[kMaxRestart + 2], vd[kMaxRestart + 2];
+    __shared__ double gsum[kSlots];                 // sums of the barrier that just ended
+    __shared__ double shc[kMaxRestart + 1];         // coefficients of the next pass
+    __shared__ double red[kRedDoubles];
+    __shared__ double bs[kThreads];
     // staged kernels: ring header (mbarriers, jobs) and the ring itself
     extern __shared__ __align__(128) unsigned char dyn_smem[];
     RingHeader* const rh = reinterpret_cast<RingHeader*>(dyn_smem);
@@ -624,6 +716,7 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
         sh_pending = __ldcg(&I.st->pending);
         sh_hbuf = __ldcg(&I.st->hbuf);
         sh_status = __ldcg(&I.st->status);
+        ctl.abort = 0;
         if constexpr (ST) {
             for (int q = 0; q < kMaxStages; ++q) {
                 mbar_init(smem_u32(&rh->full[q]), 1u);
@@ -653,27 +746,32 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
                 if (J->quit) break;
                 fence_proxy_async_global();
                 const int na = J->n_arr, sbytes = J->stage_bytes, nst = J->n_stages;
-                const int tstep = J->step, nt = J->n_tiles;
+                const int tstep = J->step, nt = J->n_tiles, gt = J->gt;
                 const char* src = pl < na ? J->src[pl] : nullptr;
                 const int bytes = pl < na ? J->bytes[pl] : 0;
                 const int off = pl < na ? J->off[pl] : 0;
                 int sg = 0;
-                for (int tile = J->tile0; tile < nt && !dead; tile += tstep) {
-                    const uint32_t fb = smem_u32(&rh->full[sg]);
-                    bool ok = true;
-                    if (pl == 0) ok = mbar_wait(smem_u32(&rh->empty[sg]), (epar >> sg) & 1u, stop, abort_word);
-                    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-                    if (!ok) {
-                        dead = true;
-                        break;
+                for (int grp = J->tile0; grp * gt < nt && !dead; grp += tstep) {
+                    const int tend = min(nt, (grp + 1) * gt);
+                    for (int tile = grp * gt; tile < tend && !dead; ++tile) {
+                        const uint32_t fb = smem_u32(&rh->full[sg]);
+                        bool ok = true;
+                        if (pl == 0) ok = mbar_wait(smem_u32(&rh->empty[sg]), (epar >> sg) & 1u, stop, abort_word);
+                        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                        if (!ok) {
+                            dead = true;
+                            break;
+                        }
+                        epar ^= 1u << sg;
+                        if (pl == 0) mbar_expect_tx(fb, (uint32_t)sbytes);
+                        __syncwarp();
+                        if (pl < na)
+                            bulk_g2s(ring_u32 + (uint32_t)(sg * sbytes + off), src + (size_t)tile * bytes,
+                                     (uint32_t)bytes, fb);
+                        fpar ^= 1u << sg;
+                        used |= 1u << sg;
+                        if (++sg == nst) sg = 0;
                     }
-                    epar ^= 1u << sg;
-                    if (pl == 0) mbar_expect_tx(fb, (uint32_t)sbytes);
-                    __syncwarp();
-                    if (pl < na) bulk_g2s(ring_u32 + (uint32_t)(sg * sbytes + off), src + (size_t)tile * bytes, (uint32_t)bytes, fb);
-                    fpar ^= 1u << sg;
-                    used |= 1u << sg;
-                    if (++sg == nst) sg = 0;
                 }
             }
             // every copy this CTA issued has landed before it exits
@@ -686,13 +784,10 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
     }
 
     const long long N = I.n;
-    const int ps = I.ps;
-    const bool grouped = !kWarpParts<T> && I.gpart != nullptr;
-    const int nparts = kWarpParts<T> ? I.n_tiles * kWarps : (grouped ? I.n_groups : I.n_tiles);
-    const double* psum = grouped ? I.gpart : I.part;   // what the leader sums
+    const int gt = I.gt, n_groups = I.n_groups, n_tiles = I.n_tiles;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    Scalars* sc = I.sc;
+    const bool cheb = I.cheb != 0;
     long long step = sh_step0;
     long long step_end = step + n_steps_launch;
     if (step_end > I.n_steps) step_end = I.n_steps;
@@ -701,6 +796,13 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
     int hbuf = sh_hbuf;
     bool retired = (sh_status == PHS_ERR_NONFINITE);
     bool aborted = false;
+    // solve statistics of this launch (thread 0 of rank 0)
+    __shared__ long long st_arnoldi, st_arnoldi_sq, st_solves;
+    __shared__ int st_max_arnoldi, st_nonconv;
+    if (threadIdx.x == 0) {
+        st_arnoldi = st_arnoldi_sq = st_solves = 0;
+        st_max_arnoldi = st_nonconv = 0;
+    }
     // optional phase timer: thread 0 of CTA rank 0 of each team
     __shared__ unsigned long long pf[kProfSlots];
     __shared__ unsigned long long pf_t;
@@ -716,114 +818,97 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
             pf_t = t;
         }
     };
+    unsigned int target = 0;
+    auto barrier = [&]() -> bool {
+        target += (unsigned int)P;
+        const bool ok = team_barrier<ST>(I.sync, P, target, abort_word, ctl);
+        if (prof_on && threadIdx.x == 0) pf[PF_BARRIERS] += 1;
+        return ok;
+    };
 
-    // Partial sums of one tile.  FP32: one entry per (tile, warp), written by
-    // lane 0 after a warp reduction.  FP64 (long GMRES(50) cycles): the warps of
-    // a tile are first combined in shared memory, one entry per tile, so the
-    // leader reads 8x fewer values.  Both orders are fixed.
-    __shared__ double red[2][kWarps][kSlots];
-    int red_buf = 0;
-    auto put = [&](int tile, int slot, double v) {
-        if constexpr (kWarpParts<T>) {
-            if (lane == 0) I.part[(size_t)(tile * kWarps + warp) * ps + slot] = v;
-        } else {
-            if (lane == 0) red[red_buf][warp][slot] = v;
-        }
+    // ---- partial sums.  A warp's sum of a tile goes to red[entry][warp][slot]
+    // (entry: the CTA's groups since the last flush; the tiles of a group add
+    // up), flush() adds the warps in order into the group's partials in global
+    // memory.  Two partial buffers alternate: a CTA may write the next phase's
+    // partials while another still reads this one's.
+    int pbuf = 0;
+    int entries = 0, group0 = 0;
+    double* const part0 = I.part;
+    auto phase_begin = [&]() {
+        entries = 0;
+        group0 = rank;
     };
-    auto tile_done = [&](int tile, int nslot) {
-        if constexpr (!kWarpParts<T>) {
-            csync<ST>();
-            for (int t = threadIdx.x; t < nslot; t += kThreads) {
-                double a = 0.0;
+    auto flush = [&](int ns, bool more) {
+        csync<ST>();
+        double* dst = part0 + (size_t)pbuf * I.part_half;
+        for (int e = threadIdx.x; e < entries * ns; e += kThreads) {
+            const int q = e / ns, s = e - q * ns;
+            double a = 0.0;
 #pragma unroll
-                for (int w = 0; w < kWarps; ++w) a += red[red_buf][w][t];
-                I.part[(size_t)tile * ps + t] = a;
-            }
-            red_buf ^= 1;
+            for (int w = 0; w < kWarps; ++w) a += red[(q * kWarps + w) * ns + s];
+            dst[(size_t)(group0 + q * P) * ns + s] = a;
         }
+        if (more) csync<ST>();
+        group0 += entries * P;
+        entries = 0;
     };
-    // After a CTA's tiles of a phase (FP64 with group sums): one fence, then
-    // the CTA counts its tiles in at their groups; the CTA whose tile completes
-    // a group sums that group's tiles in order.  Every tile of a group arrives
-    // once per phase and the next phase's arrivals follow the team barrier, so
-    // the completing CTA resets the counter.
-    __shared__ int sh_glast[kMaxGroupWalk];
-    __shared__ int sh_nlast;
-    auto groups_done = [&](int nslot) {
-        if constexpr (!kWarpParts<T>) {
-            if (I.gpart == nullptr) return;
-            for (int base = rank; base < I.n_tiles; base += kMaxGroupWalk * P) {
-                csync<ST>();
-                if (threadIdx.x == 0) {
-                    __threadfence();
-                    int nl = 0;
-                    for (int q = 0; q < kMaxGroupWalk; ++q) {
-                        const int tile = base + q * P;
-                        if (tile >= I.n_tiles) break;
-                        const int g = tile / kGroupTiles;
-                        const int gsz = min(kGroupTiles, I.n_tiles - g * kGroupTiles);
-                        if (atomicAdd(I.gcnt + g, 1u) == (unsigned int)(gsz - 1)) sh_glast[nl++] = g;
-                    }
-                    sh_nlast = nl;
-                    __threadfence();
-                }
-                csync<ST>();
-                for (int q = 0; q < sh_nlast; ++q) {
-                    const int g = sh_glast[q];
-                    const int t0 = g * kGroupTiles;
-                    const int t1 = min(t0 + kGroupTiles, I.n_tiles);
-                    for (int t = threadIdx.x; t < nslot; t += kThreads) {
-                        double a = 0.0;
-                        for (int u = t0; u < t1; ++u) a += __ldcg(I.part + (size_t)u * ps + t);
-                        I.gpart[(size_t)g * ps + t] = a;
-                    }
-                    if (threadIdx.x == 0) I.gcnt[g] = 0u;
-                }
-            }
+    // a lane's sums of slot s for the current group
+    auto put = [&](int ns, int s, double v, bool first) {
+        double* p = &red[(entries * kWarps + warp) * ns + s];
+        *p = first ? v : *p + v;
+    };
+    auto group_done = [&](int ns) {
+        ++entries;
+        if ((entries + 1) * kWarps * ns > kRedDoubles) flush(ns, true);
+    };
+    // sums over all groups into gsum[0..ns), in an order that depends on the
+    // number of groups alone: thread t adds slot t % ns over every
+    // (256 / ns)-th group, then a warp per slot adds the threads.
+    auto reduce = [&](int ns) {
+        const double* src = part0 + (size_t)pbuf * I.part_half;
+        const int stride = kThreads / ns;
+        const int q0 = threadIdx.x / ns, s = threadIdx.x - q0 * ns;
+        double a = 0.0;
+        if (q0 < stride) {
+#pragma unroll 8
+            for (int q = q0; q < n_groups; q += stride) a += __ldcg(src + (size_t)q * ns + s);
         }
+        bs[threadIdx.x] = a;
+        csync<ST>();
+        const int live = min(stride, n_groups);
+        for (int t = warp; t < ns; t += kWarps) {
+            double b = 0.0;
+            for (int l = lane; l < live; l += 32) b += bs[l * ns + t];
+            b = warp_sum(b);
+            if (lane == 0) gsum[t] = b;
+        }
+        csync<ST>();
+        pbuf ^= 1;
+    };
+    // the barrier of a phase that summed ns slots
+    unsigned long long t_red = 0;
+    auto barrier_sums = [&](int ns) -> bool {
+        flush(ns, false);
+        if (!barrier()) return false;
+        if (prof_on && threadIdx.x == 0) t_red = global_ns();
+        reduce(ns);
+        return true;
+    };
+    auto decided = [&]() {   // after every CTA's own decision
+        csync<ST>();
+        if (prof_on && threadIdx.x == 0) pf[PF_LEADER] += global_ns() - t_red;
     };
     auto voxel = [&](int tile, int v) -> long long { return (long long)tile * TILE + v * kThreads + threadIdx.x; };
 
     // ---- consumer side of the staging ring (ST)
     Stager<RING, TILE, T> stg{rh, ring, 0, 0, 0, 0, 0, 0u};
-    // row coefficients of local voxel li from a stage (cw + m6, or coef)
-    auto stage_coef = [&](const unsigned char* sb, int o_c, int o_m, int li, T (&c)[6]) {
-        if (o_m >= 0) {
-            const T w = reinterpret_cast<const T*>(sb + o_c)[li];
-            const unsigned mk = sb[o_m + li];
-#pragma unroll
-            for (int k = 0; k < 6; ++k) c[k] = ((mk >> k) & 1u) ? w : T(0);
-        } else {
-            const T* cf = reinterpret_cast<const T*>(sb + o_c) + 6 * li;
-#pragma unroll
-            for (int k = 0; k < 6; ++k) c[k] = cf[k];
-        }
-    };
-    // neighbour indices of voxel n (local li) from a stage's compact table, or
-    // the int32 table in global memory when the instance has none
-    auto stage_nb = [&](const unsigned char* sb, int o_nb, int li, long long n, int32_t (&q)[6]) {
-        if (o_nb >= 0)
-            decode_nb(reinterpret_cast<const short4*>(sb + o_nb)[li], __ldg(reinterpret_cast<const int4*>(I.nbase) + (n >> 9)),
-                      n, q);
-        else
-            load_nb(I.nb, n, q);
-    };
-    // neighbour indices of row n (unstaged loops)
-    auto row_nb = [&](long long n, int32_t (&q)[6]) {
-        if constexpr (NBC) {
-            decode_nb(__ldg(reinterpret_cast<const short4*>(I.nbr) + n), __ldg(reinterpret_cast<const int4*>(I.nbase) + (n >> 9)),
-                      n, q);
-        } else {
-            load_nb(I.nb, n, q);
-        }
-    };
 
     // Prefetch into L2 the slice of an array (elem bytes per voxel) that `tile`
     // will read, so that the loads of the CTA's next tile find it there.  Start
     // and end are rounded down to 16 bytes: every prefetched byte lies inside
     // the array (whose allocation starts 256-byte aligned).
     auto pf_slice = [&](const void* arr, int elem, int tile) {
-        if (arr == nullptr || tile >= I.n_tiles) return;
+        if (arr == nullptr || tile >= n_tiles) return;
         const long long v0 = (long long)tile * TILE;
         const long long v1 = (v0 + TILE < N) ? v0 + TILE : N;
         uintptr_t a = reinterpret_cast<uintptr_t>(arr) + (uintptr_t)(v0 * elem);
@@ -835,16 +920,19 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
     // the row tables of the operator (neighbours, coefficients, flags, edges)
     auto pf_rows = [&](int t, int tile) {
         switch (t) {
-            case 0: if (NBC) pf_slice(I.nbr, 8, tile); else pf_slice(I.nb, 24, tile); break;
+            case 0: if (NB == 1 || (NB == 2 && I.nbr)) pf_slice(I.nbr, 8, tile); else pf_slice(I.nb, 24, tile); break;
             case 1: pf_slice(I.cw ? (const void*)I.cw : (const void*)I.coef, I.cw ? (int)sizeof(T) : 6 * (int)sizeof(T), tile); break;
             case 2: pf_slice(I.m6, 1, tile); break;
-            case 3: pf_slice(I.vflags, 1, tile); break;
-            case 4: if (EDGE) pf_slice(I.enb, 48, tile); break;
-            case 5: if (EDGE) pf_slice(I.ecf, 6 * (int)sizeof(T), tile); break;
+            case 3: if (EDGE) pf_slice(I.enb, 48, tile); break;
+            case 4: if (EDGE) pf_slice(I.ecf, 6 * (int)sizeof(T), tile); break;
             default: break;
         }
     };
-    constexpr int kRowArrays = 6;
+    constexpr int kRowArrays = 5;
+    // the CTA's tile after `tile` of group `grp`
+    auto tile_after = [&](int grp, int tile) {
+        return (tile + 1 < min(n_tiles, (grp + 1) * gt)) ? tile + 1 : (grp + P) * gt;
+    };
 
     auto params_of = [&](long long n, T* p) {
         if (I.vparams) {
@@ -858,245 +946,260 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
         }
     };
 
-    // ---- leader bodies ------------------------------------------------------
-    // Deterministic sums of partial slots slot0 .. slot0+ns-1 over all partials,
-    // by the whole leader CTA; results in bsum_out[0..ns).  The order depends
-    // only on the partial count, not on the team size.
-    //  FP32 (a partial per tile and warp: many partials, few slots): thread t
-    //  adds partials t, t+256, ... in order, four slots per pass with their loads
-    //  issued together, then a fixed xor tree per warp.
-    //  FP64 (a partial per group of tiles: few partials, up to 51 slots in a
-    //  GMRES(50) cycle): lane l of warp w adds slot l (and l + 32) over partials
-    //  w, w+8, ... in order, its loads issued together, so one pass of loads
-    //  serves every slot.
-    //  Both end with the warp results added in warp order.
-    __shared__ double bsum_w[kMaxRestart + 1][kWarps];
-    __shared__ double bsum_out[kMaxRestart + 1];
-    constexpr int kSumW = 4;
-    auto block_sum = [&](int slot0, int ns) {
-        if constexpr (kWarpParts<T>) {
-            for (int s0 = 0; s0 < ns; s0 += kSumW) {
-                double a[kSumW];
-#pragma unroll
-                for (int u = 0; u < kSumW; ++u) a[u] = 0.0;
-#pragma unroll 4
-                for (int q = threadIdx.x; q < nparts; q += kThreads) {
-                    const double* pq = psum + (size_t)q * ps + slot0 + s0;
-#pragma unroll
-                    for (int u = 0; u < kSumW; ++u)
-                        if (s0 + u < ns) a[u] += __ldcg(pq + u);
-                }
-#pragma unroll
-                for (int u = 0; u < kSumW; ++u) {
-                    const double v = warp_sum(a[u]);
-                    if (lane == 0 && s0 + u < ns) bsum_w[s0 + u][warp] = v;
-                }
-            }
-        } else {
-            for (int s0 = 0; s0 < ns; s0 += 32) {
-                const int sl = s0 + lane;
-                if (sl < ns) {
-                    const double* pq = psum + slot0 + sl;
-                    double a = 0.0;
-#pragma unroll 8
-                    for (int q = warp; q < nparts; q += kWarps) a += __ldcg(pq + (size_t)q * ps);
-                    bsum_w[sl][warp] = a;
-                }
-            }
-        }
-        csync<ST>();
-        for (int i = threadIdx.x; i < ns; i += kThreads) {
-            double t = 0.0;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) t += bsum_w[i][w];
-            bsum_out[i] = t;
-        }
-        csync<ST>();
-    };
+    T* const Vb = I.V;
+    P2* const UD = reinterpret_cast<P2*>(I.ud);
+    const size_t ldV = (size_t)I.ldv;
 
-    // statistics of a solve that iterated, recorded by the leader that ends it
+    // ---- what every CTA decides from the sums of a barrier ------------------
+    int iters_solve = 0, iters_cap = 0, cols = 0;   // columns: of the solve, CuPy's count, of the cycle
+    bool refined = false;
+    auto fail = [&]() {
+        ctl.action = ACT_FAIL;
+        if (rank == 0) I.st->status = PHS_ERR_NONFINITE;
+    };
     auto account_solve = [&]() {
-        const int it = sc->iters_solve;
-        if (it > 0) {
-            I.st->arnoldi += it;
-            I.st->arnoldi_sq += (long long)it * it;
-            I.st->solves += 1;
-            if (it > I.st->max_arnoldi) I.st->max_arnoldi = it;
+        if (rank == 0 && threadIdx.x == 0 && iters_solve > 0) {
+            st_arnoldi += iters_solve;
+            st_arnoldi_sq += (long long)iters_solve * iters_solve;
+            st_solves += 1;
+            st_max_arnoldi = max(st_max_arnoldi, iters_solve);
         }
     };
-
-    auto leader_rhs = [&]() {
-        block_sum(0, 2);
-        if (warp == 0) {
-            double b2 = bsum_out[0];
-            double r2 = bsum_out[1];
-            if (lane == 0) {
-                double bn = sqrt(b2), rn = sqrt(r2);
-                double atol_eff = fmax(I.atol, I.tol * bn);
-                int act;
-                if (!isfinite(bn) || !isfinite(rn)) act = ACT_FAIL;
-                else if (bn == 0.0) act = ACT_ZERO_B;
-                else if (rn <= atol_eff) act = ACT_DONE;
-                else {
-                    act = ACT_CYCLE;
-                    sc->g[0] = rn;
-                    sc->s[0] = 1.0 / rn;
-                    sc->iters_solve = 0;
-                    sc->iters_cap = 0;
-                }
-                sc->bnorm = bn;
-                sc->rnorm = rn;
-                sc->atol_eff = atol_eff;
-                sc->action = act;
-                if (act == ACT_FAIL) I.st->status = PHS_ERR_NONFINITE;
-            }
+    // start of a cycle from the residual in column 0, norm rn (thread 0)
+    auto start_cycle = [&](double rn) {
+        ctl.action = ACT_CYCLE;
+        if (cheb) {
+            const double w0 = 1.0 / rn;
+            tm[0] = w0;            // W
+            va[0] = w0;            // z
+            vb[0] = 1.0;           // t
+            ctl.sz = w0 * w0;
+        } else {
+            va[0] = rn;            // g
+            vb[0] = 1.0 / rn;      // s
+            ctl.sj = vb[0];
         }
     };
-
-    auto leader_dots = [&](int j) {
-        // h_ij = s_i * sum <V_i, w>;  published coef_i = h_ij * s_i
-        block_sum(0, j + 1);
-        for (int i = threadIdx.x; i <= j; i += kThreads) {
-            double si = sc->s[i];
-            double h = si * bsum_out[i];
-            sc->R[j * (kMaxRestart + 1) + i] = h;
-            sc->coef[i] = h * si;
-        }
-    };
-
-    // Givens update of Hessenberg column j and, when the cycle ends, the back
-    // substitution R y = g.  The rotations, the column, g, s and (at a cycle
-    // end) the k x k triangle of R are first loaded into shared memory by the
-    // whole CTA, so the sequential parts run on shared memory instead of a
-    // chain of dependent L2 round trips; the arithmetic and its order are
-    // those of a plain sequential Givens QR.
-    __shared__ double gv_cs[kMaxRestart], gv_sn[kMaxRestart], gv_col[kMaxRestart + 2];
-    __shared__ double gv_g[kMaxRestart + 1], gv_s[kMaxRestart + 1], gv_y[kMaxRestart + 1];
-    __shared__ double gv_R[kMaxRestart * (kMaxRestart + 1) / 2];   // column l, rows 0..l at l(l+1)/2 + i
-    __shared__ int gv_act;
-    auto leader_norm = [&](int j) {
-        block_sum(0, 1);
-        double* Rc = sc->R + j * (kMaxRestart + 1);
-        for (int i = threadIdx.x; i < j; i += kThreads) {
-            gv_cs[i] = __ldcg(sc->cs + i);
-            gv_sn[i] = __ldcg(sc->sn + i);
-        }
-        for (int i = threadIdx.x; i <= j; i += kThreads) {
-            gv_col[i] = __ldcg(Rc + i);
-            gv_g[i] = __ldcg(sc->g + i);
-            gv_s[i] = __ldcg(sc->s + i);
-        }
-        csync<ST>();
+    auto decide_rhs = [&]() {
         if (threadIdx.x == 0) {
-            const double hn = sqrt(bsum_out[0]);
-            gv_col[j + 1] = hn;
-            // apply the previous rotations to column j
-            for (int i = 0; i < j; ++i) {
-                const double c = gv_cs[i], s = gv_sn[i];
-                const double a = gv_col[i], bb = gv_col[i + 1];
-                gv_col[i] = c * a + s * bb;
-                gv_col[i + 1] = -s * a + c * bb;
+            const double bn = sqrt(gsum[0]), rn = sqrt(gsum[1]);
+            const double atol_eff = fmax(I.atol, I.tol * bn);
+            ctl.bnorm = bn;
+            ctl.atol_eff = atol_eff;
+            if (!isfinite(bn) || !isfinite(rn)) fail();
+            else if (bn == 0.0) ctl.action = ACT_ZERO_B;
+            else if (rn <= atol_eff) ctl.action = ACT_DONE;
+            else start_cycle(rn);
+        }
+        decided();
+    };
+    // Chebyshev basis, column j (K_0..K_{j+1} there, gsum[i] = <K_{j+1}, K_i>):
+    // the next row of W and entry of z, the residual estimate, and at the end of
+    // a cycle the coefficients of x = x0 + sum y_i K_i.  One warp.
+    auto decide_cheb = [&](int j, int cycle_cols) {
+        if (warp == 0) {
+            const double gjj = gsum[j + 1];
+            // x = W g, the new column of R
+            double xs[2], s2 = 0.0, sx = 0.0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = lane + 32 * h;
+                double a = 0.0;
+                if (i <= j) {
+                    const double* wr = tm + tri(i);
+                    for (int l = 0; l <= i; ++l) a += wr[l] * gsum[l];
+                    s2 += a * a;
+                    sx += a * va[i];
+                    vd[i] = a;
+                }
+                xs[h] = a;
             }
-            const double a = gv_col[j], bb = gv_col[j + 1];
+            s2 = warp_sum(s2);
+            sx = warp_sum(sx);
+            __syncwarp();
+            const double tj = (j == 0) ? I.t1 : 2.0 * I.t1 * vb[j] - vb[j - 1];
+            double p2 = gjj - s2;
+            const bool finite = isfinite(gjj) && isfinite(s2);
+            const bool dependent = fabs(p2) <= kPivot * gjj;        // breakdown: K_{j+1} in the span
+            const bool lost = !dependent && !(p2 > 0.0);            // G no longer positive definite
+            if (dependent) p2 = fmax(1e-30 * gjj, 1e-200);
+            int act, k = j + 1;
+            bool settled = false;
+            if (!finite) {
+                act = ACT_FAIL;
+            } else if (lost) {
+                act = ACT_UPDATE_CHECK;
+                k = j;                                             // without the column that failed
+            } else {
+                const double pinv = (p2 > 0.0) ? 1.0 / sqrt(p2) : 0.0;
+                double* wn = tm + tri(j + 1);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int l = lane + 32 * h;
+                    if (l <= j) {
+                        double a = 0.0;
+                        for (int i = l; i <= j; ++i) a += vd[i] * tm[tri(i) + l];
+                        wn[l] = -a * pinv;
+                    }
+                }
+                const double zn = (tj - sx) * pinv;
+                const double sz = ctl.sz + zn * zn;
+                __syncwarp();
+                if (lane == 0) {
+                    wn[j + 1] = pinv;
+                    va[j + 1] = zn;
+                    vb[j + 1] = tj;
+                    ctl.sz = sz;
+                }
+                const double est = 1.0 / sqrt(sz);
+                settled = I.full_cycles && est <= kSettled<T> * ctl.bnorm;
+                if (!isfinite(est)) act = ACT_FAIL;
+                else if (!I.full_cycles && est <= ctl.atol_eff && !dependent) act = ACT_UPDATE_FINAL;
+                else if (j + 1 >= cycle_cols || dependent || settled) act = ACT_UPDATE_CHECK;
+                else act = ACT_NEXT_J;
+                __syncwarp();
+            }
+            if (act == ACT_UPDATE_FINAL || act == ACT_UPDATE_CHECK) {
+                // residual coefficients c = W^T z / ||z||^2 over K_0..K_k
+                const double isz = 1.0 / ctl.sz;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int l = lane + 32 * h;
+                    if (l <= k) {
+                        double a = 0.0;
+                        for (int i = l; i <= k; ++i) a += tm[tri(i) + l] * va[i];
+                        vc[l] = a * isz;
+                    }
+                }
+                __syncwarp();
+                // sum c_i K_i = r0 - A sum y_i K_i with A K_0 = theta K_0 + delta K_1,
+                // A K_i = theta K_i + delta/2 (K_{i+1} + K_{i-1}): rows k..1 give y
+                if (lane == 0) {
+                    double y1 = 0.0, y2 = 0.0;      // y_i, y_{i+1}
+                    for (int i = k; i >= 1; --i) {
+                        const double y0 = -(vc[i] + I.theta * y1 + 0.5 * I.delta * y2) /
+                                          (i == 1 ? I.delta : 0.5 * I.delta);
+                        shc[i - 1] = y0;
+                        y2 = y1;
+                        y1 = y0;
+                    }
+                }
+            }
+            if (lane == 0) {
+                ctl.action = act;
+                ctl.k = k;
+                ctl.settled = settled ? 1 : 0;
+                if (act == ACT_FAIL) fail();
+            }
+        }
+        decided();
+    };
+    // Arnoldi, phase A of column j: h_ij = s_i <V_i, w> and the coefficients
+    // h_ij s_i that phase C subtracts
+    auto decide_dots = [&](int j) {
+        for (int i = threadIdx.x; i <= j; i += kThreads) {
+            const double si = vb[i];
+            const double h = si * gsum[i];
+            vc[i] = h;
+            shc[i] = h * si;
+        }
+        decided();
+    };
+    // Arnoldi, phase C of column j: Givens update of the Hessenberg column and,
+    // when the cycle ends, the back substitution R y = g (g in va, s in vb,
+    // the rotations in gv_cs and vd, the column in vc)
+    __shared__ double gv_cs[kMaxRestart];
+    auto decide_norm = [&](int j) {
+        if (threadIdx.x == 0) {
+            const double hn = sqrt(gsum[0]);
+            vc[j + 1] = hn;
+            for (int i = 0; i < j; ++i) {
+                const double c = gv_cs[i], s = vd[i];
+                const double a = vc[i], bb = vc[i + 1];
+                vc[i] = c * a + s * bb;
+                vc[i + 1] = -s * a + c * bb;
+            }
+            const double a = vc[j], bb = vc[j + 1];
             const double r = hypot(a, bb);
             const double c = (r == 0.0) ? 1.0 : a / r;
             const double s = (r == 0.0) ? 0.0 : bb / r;
-            sc->cs[j] = c;
-            sc->sn[j] = s;
-            gv_col[j] = r;
-            gv_col[j + 1] = 0.0;
-            const double gj = gv_g[j];
-            gv_g[j] = c * gj;
-            gv_g[j + 1] = -s * gj;
-            sc->g[j] = gv_g[j];
-            sc->g[j + 1] = gv_g[j + 1];
-            const double est = fabs(gv_g[j + 1]);
-            sc->est = est;
-            sc->iters_solve += 1;
-            int act;
-            const bool finite = isfinite(hn) && isfinite(r);
+            gv_cs[j] = c;
+            vd[j] = s;
+            vc[j] = r;
+            for (int i = 0; i <= j; ++i) tm[tri(j) + i] = vc[i];
+            const double gj = va[j];
+            va[j] = c * gj;
+            va[j + 1] = -s * gj;
+            const double est = fabs(va[j + 1]);
             const bool breakdown = (hn == 0.0);
-            const bool conv = (!I.full_cycles) && (est <= sc->atol_eff);
-            // a full cycle whose estimate is below rounding level (kSettled) is over:
-            // the columns still to come cannot change x
-            const bool settled = I.full_cycles && est <= kSettled<T> * sc->bnorm;
-            if (!finite) {
+            const bool conv = (!I.full_cycles) && (est <= ctl.atol_eff);
+            const bool settled = I.full_cycles && est <= kSettled<T> * ctl.bnorm;
+            int act;
+            if (!isfinite(hn) || !isfinite(r)) {
                 act = ACT_FAIL;
-                I.st->status = PHS_ERR_NONFINITE;
             } else if (conv || (breakdown && !I.full_cycles)) {
                 act = ACT_UPDATE_FINAL;
             } else if (j + 1 >= I.m || breakdown || settled) {
                 act = ACT_UPDATE_CHECK;
             } else {
                 act = ACT_NEXT_J;
-                sc->s[j + 1] = 1.0 / hn;
+                vb[j + 1] = 1.0 / hn;
+                ctl.sj = vb[j + 1];
             }
-            if (act == ACT_UPDATE_FINAL || act == ACT_UPDATE_CHECK) sc->k = j + 1;
-            if (act == ACT_UPDATE_FINAL) account_solve();
-            sc->action = act;
-            gv_act = act;
+            ctl.action = act;
+            ctl.k = j + 1;
+            ctl.settled = 1;    // nothing is left of the cycle
+            if (act == ACT_FAIL) fail();
         }
         csync<ST>();
-        for (int i = threadIdx.x; i <= j + 1; i += kThreads) Rc[i] = gv_col[i];
-        const int act = gv_act;
-        if (act != ACT_UPDATE_FINAL && act != ACT_UPDATE_CHECK) return;
-        // back substitution R y = g (k x k upper triangular), k = j + 1
-        const int k = j + 1;
-        for (int l = warp; l < k; l += kWarps)
-            for (int i = lane; i <= l; i += 32)
-                gv_R[l * (l + 1) / 2 + i] = (l == j) ? gv_col[i] : __ldcg(sc->R + l * (kMaxRestart + 1) + i);
-        csync<ST>();
-        if (warp == 0) {
+        if ((ctl.action == ACT_UPDATE_FINAL || ctl.action == ACT_UPDATE_CHECK) && warp == 0) {
+            const int k = j + 1;
             for (int i = k - 1; i >= 0; --i) {
                 double acc = 0.0;
-                for (int l = i + 1 + lane; l < k; l += 32) acc += gv_R[l * (l + 1) / 2 + i] * gv_y[l];
+                for (int l = i + 1 + lane; l < k; l += 32) acc += tm[tri(l) + i] * vc[l];
                 acc = warp_sum(acc);
-                if (lane == 0) gv_y[i] = (gv_g[i] - acc) / gv_R[i * (i + 1) / 2 + i];
+                if (lane == 0) vc[i] = (va[i] - acc) / tm[tri(i) + i];
                 __syncwarp();
             }
-            // scale: x += sum_j y_j v_j = sum_j (y_j s_j) V_j
-            for (int i = lane; i < k; i += 32) sc->coef[i] = gv_y[i] * gv_s[i];
+            // x += sum_j y_j v_j = sum_j (y_j s_j) V_j
+            for (int i = lane; i < k; i += 32) shc[i] = vc[i] * vb[i];
         }
+        decided();
     };
-
-    auto leader_check = [&]() {
-        block_sum(0, 1);
-        if (warp == 0) {
-            double r2 = bsum_out[0];
-            if (lane == 0) {
-                double rn = sqrt(r2);
-                sc->rnorm = rn;
-                sc->iters_cap += I.m;
-                int act;
-                if (!isfinite(rn)) {
-                    act = ACT_FAIL;
-                    I.st->status = PHS_ERR_NONFINITE;
-                } else if (rn <= sc->atol_eff) {
-                    act = ACT_DONE;
-                    account_solve();
-                } else if (sc->iters_cap >= I.maxiter) {
-                    act = ACT_DONE;
-                    account_solve();
-                    I.st->nonconv += 1;
-                    if (I.st->status == PHS_OK) I.st->status = PHS_WARN_NO_CONVERGE;
-                } else {
-                    act = ACT_CYCLE;
-                    sc->g[0] = rn;
-                    sc->s[0] = 1.0 / rn;
-                }
-                sc->action = act;
+    auto decide_check = [&]() {
+        // columns the logical cycle of I.m still has: when its Gram matrix gave out
+        // early, or once more when it ended settled (kRefine)
+        const int left = I.m - cols;
+        const double rn = sqrt(gsum[0]);
+        const bool more = cheb && I.full_cycles && left > 0 && rn > kRefine<T> * ctl.bnorm && !refined;
+        if (more && ctl.settled) refined = true;
+        if (!more) iters_cap += I.m;
+        bool over = false;
+        csync<ST>();
+        if (threadIdx.x == 0) {
+            if (!isfinite(rn)) {
+                fail();
+            } else if (more) {
+                start_cycle(rn);
+            } else if (rn <= ctl.atol_eff) {
+                ctl.action = ACT_DONE;
+            } else if (iters_cap >= I.maxiter) {
+                ctl.action = ACT_DONE;
+                over = true;
+            } else {
+                start_cycle(rn);
             }
         }
-    };
-
-
-    // the action and cycle length of the barrier that just ended (team_sync)
-    auto read_action = [&]() { return ctl.action; };
-
-    auto load_shc = [&](int cnt) {
-        csync<ST>();
-        for (int i = threadIdx.x; i < cnt; i += kThreads) shc[i] = __ldcg(sc->coef + i);
-        csync<ST>();
+        decided();
+        if (!more) {
+            cols = 0;
+            refined = false;
+        }
+        if (ctl.action == ACT_DONE) account_solve();
+        if (over) {
+            st_nonconv += 1;
+            if (rank == 0 && I.st->status == PHS_OK) I.st->status = PHS_WARN_NO_CONVERGE;
+        }
     };
 
     // ---- sample / activation bookkeeping of the state in u (after step s-1)
@@ -1108,17 +1211,14 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
         if (done_step >= 0 && un >= T(0.5) && I.lat[n] < 0) I.lat[n] = (int32_t)done_step;
     };
 
-    T* Vb = I.V;
-    const size_t ldV = (size_t)I.ldv;
-
     // End-of-step work of voxel n whose new state un is known (the state after
     // step done_step): its sample into history slot `slot` (-1: none), its
     // activation entry (lat_n loaded when un >= 0.5), then the RK4 reaction of
     // the next step (stimulus bits stim_next) -> h of the step after it into
-    // hdst, u* into the basis column 1.  This is the reaction pass of the next
-    // step, done while the voxel's new state is still in registers.
+    // hdst, u* returned.  This is the reaction pass of the next step, done while
+    // the voxel's new state is still in registers.
     auto react_voxel = [&](long long n, T un, T hn, int32_t lat_n, long long done_step, int slot, uint8_t fl,
-                           uint8_t stim_next, T* hdst) {
+                           uint8_t stim_next, T* hdst) -> T {
         if (slot >= 0) {
             I.hist_u[(size_t)slot * N + n] = un;
             if (I.save_h) I.hist_h[(size_t)slot * N + n] = hn;
@@ -1130,29 +1230,7 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
         T us, hs;
         rk4(I.model, un, hn, J, p, I.dt, us, hs);
         hdst[n] = hs;
-        Vb[ldV + n] = us;
-    };
-
-    // acc[v] += sum_{i < cnt} coef[i] * Vb[i][n_v], loads issued kChunk vectors at a time
-    auto axpy_basis = [&](int tile, int cnt, const double* coef, double (&acc)[VPT]) {
-        for (int i0 = 0; i0 < cnt; i0 += kChunk) {
-            T vv[kChunk][VPT];
-#pragma unroll
-            for (int ii = 0; ii < kChunk; ++ii)
-#pragma unroll
-                for (int v = 0; v < VPT; ++v) {
-                    long long n = voxel(tile, v);
-                    vv[ii][v] = (i0 + ii < cnt && n < N) ? Vb[(size_t)(i0 + ii) * ldV + n] : T(0);
-                }
-#pragma unroll
-            for (int ii = 0; ii < kChunk; ++ii) {
-                if (i0 + ii < cnt) {
-                    const double cf = coef[i0 + ii];
-#pragma unroll
-                    for (int v = 0; v < VPT; ++v) acc[v] += cf * (double)vv[ii][v];
-                }
-            }
-        }
+        return us;
     };
 
     // the reaction pass of the current step was done at the end of the previous
@@ -1165,162 +1243,86 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
         T* hout = hbuf ? I.h0 : I.h1;
 
         // ================= RHS phase.  Pass 1: RK4 reaction of every voxel of the
-        // team; u* goes to basis column 1 (unused until the first Arnoldi step).
-        // Except in the first step of a launch and after a full-cycle solve, it
-        // ran at the end of the previous step (react_voxel in the update and copy
-        // passes), so it costs no pass of its own.
-        // Pass 2, after a team barrier: b = u* + dt/2 L u*, the initial guess and
-        // r0 = b - A x0 -> V0, gathering u* of the neighbours from memory.  (A
-        // fused form that kept a tile's u* in shared memory and recomputed the RK4
-        // of neighbours outside the tile did three RK4 per voxel in row order and
-        // was 17 % slower over the batch.)
-        T* Us = Vb + ldV;
-        for (int tile = prepared ? I.n_tiles : rank; tile < I.n_tiles; tile += P) {
-            if (threadIdx.x < 4) {
-                const int t = threadIdx.x;
-                if (t == 0) pf_slice(I.u, sizeof(T), tile + P);
-                else if (t == 1) pf_slice(hin, sizeof(T), tile + P);
-                else if (t == 2) pf_slice(I.vflags, 1, tile + P);
-                else pf_slice(I.vparams, 5 * sizeof(T), tile + P);
-            }
-            // every load of the tile before its first store: plain loads cannot
-            // move across stores the compiler must assume may alias them
-            T un[VPT], hn[VPT];
-            uint8_t fl[VPT];
-            int32_t lt[VPT];
+        // team, u* into the pairs.  Except in the first step of a launch and after
+        // a full-cycle solve, it ran at the end of the previous step (react_voxel
+        // in the update and copy passes), so it costs no pass of its own.
+        // Pass 2, after a team barrier: b = u* + dt/2 L u*, the initial guess
+        // x0 = u* + dx and r0 = b - A x0 -> V0.  u* and the increment dx lie side by
+        // side, so one gather per neighbour brings both; x0 and b are not stored
+        // (x0 is u* + dx again in the update; only full cycles read b).
+        for (int grp = prepared ? n_groups : rank; grp < n_groups; grp += P) {
+            for (int tile = grp * gt; tile < min(n_tiles, (grp + 1) * gt); ++tile) {
+                const int nxt = tile_after(grp, tile);
+                if (threadIdx.x < 4) {
+                    const int t = threadIdx.x;
+                    if (t == 0) pf_slice(I.u, sizeof(T), nxt);
+                    else if (t == 1) pf_slice(hin, sizeof(T), nxt);
+                    else if (t == 2) pf_slice(I.vflags, 1, nxt);
+                    else pf_slice(I.vparams, 5 * sizeof(T), nxt);
+                }
+                // every load of the tile before its first store: plain loads cannot
+                // move across stores the compiler must assume may alias them
+                T un[VPT], hn[VPT];
+                uint8_t fl[VPT];
+                int32_t lt[VPT];
 #pragma unroll
-            for (int v = 0; v < VPT; ++v) {
-                const long long n = voxel(tile, v);
-                un[v] = T(0);
-                hn[v] = T(0);
-                fl[v] = 0;
-                lt[v] = 0;
-                if (n < N) {
+                for (int v = 0; v < VPT; ++v) {
+                    const long long n = voxel(tile, v);
                     un[v] = I.u[n];
                     hn[v] = hin[n];
                     fl[v] = __ldg(I.vflags + n);
                 }
-            }
 #pragma unroll
-            for (int v = 0; v < VPT; ++v) {
-                const long long n = voxel(tile, v);
-                if (n < N && step > 0 && un[v] >= T(0.5)) lt[v] = I.lat[n];
-            }
+                for (int v = 0; v < VPT; ++v)
+                    lt[v] = (step > 0 && un[v] >= T(0.5)) ? I.lat[voxel(tile, v)] : 0;
 #pragma unroll
-            for (int v = 0; v < VPT; ++v) {
-                const long long n = voxel(tile, v);
-                if (n < N) react_voxel(n, un[v], hn[v], lt[v], step - 1, pending, fl[v], stim_bits, hout);
+                for (int v = 0; v < VPT; ++v) {
+                    const long long n = voxel(tile, v);
+                    if (n < N) UD[n].x = react_voxel(n, un[v], hn[v], lt[v], step - 1, pending, fl[v], stim_bits, hout);
+                }
             }
         }
         pending = -1;
         mark(PF_RHS1);
-        if (!team_sync<ST>(I.sync, P, abort_word, ctl, sc, I.prof, [&]() {})) { aborted = true; break; }
+        if (!barrier()) { aborted = true; break; }
         mark(PF_RHS_WAIT);
-        int nst = 0;
-        if constexpr (ST) {
-            stg.begin();
-            const int o_us = stg.add(Us, sizeof(T));
-            const int o_nb = I.nbr ? stg.add(I.nbr, 8) : -1;
-            const int o_cw = I.cw ? stg.add(I.cw, sizeof(T)) : stg.add(I.coef, 6 * sizeof(T));
-            const int o_m6 = I.cw ? stg.add(I.m6, 1) : -1;
-            const int o_dx = I.dx ? stg.add(I.dx, sizeof(T)) : -1;
-            const int o_fl = tb ? stg.add(I.vflags, 1) : -1;
-            nst = stg.publish(rank, P, I.n_tiles);
-            for (int tile = rank; nst > 0 && tile < I.n_tiles; tile += P) {
-                const unsigned char* sb = stg.acquire(abort_word);
-                double ab = 0.0, ar = 0.0;
+        phase_begin();
+        for (int grp = rank; grp < n_groups; grp += P) {
+            for (int tile = grp * gt; tile < min(n_tiles, (grp + 1) * gt); ++tile) {
+                const int nxt = tile_after(grp, tile);
+                if (threadIdx.x < kRowArrays) pf_rows(threadIdx.x, nxt);
+                else if (threadIdx.x == kRowArrays) pf_slice(UD, sizeof(P2), nxt);
+                const long long n0 = voxel(tile, 0);
+                P2 own[VPT], lap[VPT];
+#pragma unroll
+                for (int v = 0; v < VPT; ++v) own[v] = UD[n0 + v * kThreads];
+                tile_lap<T, VPT, EDGE, NB>(I, UD, n0, tb, own, lap);
+                double s[2] = {0.0, 0.0};
 #pragma unroll
                 for (int v = 0; v < VPT; ++v) {
-                    const int li = v * kThreads + threadIdx.x;
-                    const long long n = (long long)tile * TILE + li;
-                    if (n < N) {
-                        const T us = reinterpret_cast<const T*>(sb + o_us)[li];
-                        const bool rz = tb && (sb[o_fl + li] & PHS_VFLAG_TBLOCK);
-                        int32_t q[6];
-                        T c[6];
-                        stage_nb(sb, o_nb, li, n, q);
-                        stage_coef(sb, o_cw, o_m6, li, c);
-                        T lap = T(0), dp = T(0), lapd = T(0);
-                        if (!rz) {
-                            lap = lap_row(Us, us, q, c);
-                            if (EDGE && I.ecf) lap += edge_row(Us, I.enb, I.ecf, n);
-                        }
-                        if (o_dx >= 0) {
-                            dp = reinterpret_cast<const T*>(sb + o_dx)[li];
-                            if (!rz) {
-                                lapd = lap_row(I.dx, dp, q, c);
-                                if (EDGE && I.ecf) lapd += edge_row(I.dx, I.enb, I.ecf, n);
-                            }
-                        }
-                        const T x0 = us + dp;
-                        const T bn = us + I.half_dt * lap;
-                        const T ax = x0 - I.half_dt * (lap + lapd);
-                        const T rn = bn - ax;
-                        I.x[n] = x0;
-                        I.b[n] = bn;
-                        Vb[n] = rn;
-                        ab += (double)bn * (double)bn;
-                        ar += (double)rn * (double)rn;
-                    }
-                }
-                stg.release();
-                ab = warp_sum(ab);
-                ar = warp_sum(ar);
-                put(tile, 0, ab);
-                put(tile, 1, ar);
-                tile_done(tile, 2);
-            }
-        }
-        for (int tile = rank; nst == 0 && tile < I.n_tiles; tile += P) {
-            if (threadIdx.x < kRowArrays) pf_rows(threadIdx.x, tile + P);
-            else if (threadIdx.x == kRowArrays) pf_slice(Us, sizeof(T), tile + P);
-            else if (threadIdx.x == kRowArrays + 1) pf_slice(I.dx, sizeof(T), tile + P);
-            double ab = 0.0, ar = 0.0;
-#pragma unroll
-            for (int v = 0; v < VPT; ++v) {
-                const long long n = voxel(tile, v);
-                if (n < N) {
-                    const T us = __ldcg(Us + n);
-                    const bool rz = tb && (__ldg(I.vflags + n) & PHS_VFLAG_TBLOCK);
-                    int32_t q[6];
-                    T c[6];
-                    row_nb(n, q);
-                    row_coef(I.coef, I.cw, I.m6, n, c);
-                    T lap = T(0), dp = T(0), lapd = T(0);
-                    if (!rz) {
-                        lap = lap_row(Us, us, q, c);
-                        if (EDGE && I.ecf) lap += edge_row(Us, I.enb, I.ecf, n);
-                    }
-                    // initial guess: u* (the reference's x0), or u* plus the previous
-                    // step's diffusion increment when dx is kept
-                    if (I.dx) {
-                        dp = I.dx[n];
-                        if (!rz) {
-                            lapd = lap_row(I.dx, dp, q, c);
-                            if (EDGE && I.ecf) lapd += edge_row(I.dx, I.enb, I.ecf, n);
-                        }
-                    }
-                    const T x0 = us + dp;
-                    const T bn = us + I.half_dt * lap;
-                    const T ax = x0 - I.half_dt * (lap + lapd);
+                    const long long n = n0 + v * kThreads;
+                    const T x0 = own[v].x + own[v].y;
+                    const T bn = own[v].x + I.half_dt * lap[v].x;
+                    const T ax = x0 - I.half_dt * (lap[v].x + lap[v].y);
                     const T rn = bn - ax;
-                    I.x[n] = x0;
-                    I.b[n] = bn;
+                    if (I.full_cycles) I.b[n] = bn;
                     Vb[n] = rn;
-                    ab += (double)bn * (double)bn;
-                    ar += (double)rn * (double)rn;
+                    s[0] += (double)bn * (double)bn;
+                    s[1] += (double)rn * (double)rn;
                 }
+                const double w = warp_sums<2>(s, lane);
+                if ((lane & 15) == 0) put(2, lane >> 4, w, tile == grp * gt);
             }
-            ab = warp_sum(ab);
-            ar = warp_sum(ar);
-            put(tile, 0, ab);
-            put(tile, 1, ar);
-            tile_done(tile, 2);
+            group_done(2);
         }
-        groups_done(2);
         mark(PF_RHS);
-        if (!team_sync<ST>(I.sync, P, abort_word, ctl, sc, I.prof, leader_rhs)) { aborted = true; break; }
-        int act = read_action();
+        if (!barrier_sums(2)) { aborted = true; break; }
+        iters_solve = 0;
+        iters_cap = 0;
+        cols = 0;
+        refined = false;
+        decide_rhs();
+        int act = ctl.action;
         mark(PF_RHS_WAIT);
         // end of this step: its history slot, and whether the pass that writes
         // the new state also runs the next step's reaction (not after the last
@@ -1332,368 +1334,303 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
         bool fused = false;
 
         if (act == ACT_CYCLE) {
-            bool leave_solve = false;
-            while (!leave_solve) {
-                int j = 0;
-                for (;;) {
-                    // ============ phase A: w = A (s_j V_j) -> V_{j+1}; dots <V_i, w>
-                    if (threadIdx.x == 0) ctl.sj = __ldcg(&sc->s[j]);
-                    csync<ST>();
-                    const T sj = (T)ctl.sj;
-                    const T* Vj = Vb + (size_t)j * ldV;
-                    T* Vn = Vb + (size_t)(j + 1) * ldV;
-                    int nsa = 0;
-                    if constexpr (ST) {
-                        stg.begin();
-                        const int o_vj = stg.add(Vj, sizeof(T));
-                        const int o_nb = I.nbr ? stg.add(I.nbr, 8) : -1;
-                        const int o_cw = I.cw ? stg.add(I.cw, sizeof(T)) : stg.add(I.coef, 6 * sizeof(T));
-                        const int o_m6 = I.cw ? stg.add(I.m6, 1) : -1;
-                        const int o_fl = tb ? stg.add(I.vflags, 1) : -1;
-                        const int nvs = min(j, stg.vec_cap());      // V_0 .. V_{nvs-1} staged too
-                        const int o_v = stg.lay_off;
-                        for (int i = 0; i < nvs; ++i) stg.add(Vb + (size_t)i * ldV, sizeof(T));
-                        nsa = stg.publish(rank, P, I.n_tiles);
-                        for (int tile = rank; nsa > 0 && tile < I.n_tiles; tile += P) {
-                            const unsigned char* sb = stg.acquire(abort_word);
-                            const T* vjs = reinterpret_cast<const T*>(sb + o_vj);
-                            T wr[VPT];
-#pragma unroll
-                            for (int v = 0; v < VPT; ++v) {
-                                const int li = v * kThreads + threadIdx.x;
-                                const long long n = (long long)tile * TILE + li;
-                                wr[v] = T(0);
-                                if (n < N) {
-                                    const T vj = vjs[li];
-                                    const bool rz = tb && (sb[o_fl + li] & PHS_VFLAG_TBLOCK);
-                                    int32_t q[6];
-                                    T c[6];
-                                    stage_nb(sb, o_nb, li, n, q);
-                                    stage_coef(sb, o_cw, o_m6, li, c);
-                                    T lap = rz ? T(0) : lap_row(Vj, vj, q, c);
-                                    if (EDGE && I.ecf && !rz) lap += edge_row(Vj, I.enb, I.ecf, n);
-                                    const T w = sj * (vj - I.half_dt * lap);
-                                    Vn[n] = w;
-                                    wr[v] = w;
-                                }
-                            }
-                            for (int i0 = 0; i0 <= j; i0 += kChunk) {
-                                T vv[kChunk][VPT];
-#pragma unroll
-                                for (int ii = 0; ii < kChunk; ++ii)
-#pragma unroll
-                                    for (int v = 0; v < VPT; ++v) {
-                                        const int li = v * kThreads + threadIdx.x;
-                                        const long long n = (long long)tile * TILE + li;
-                                        const int i = i0 + ii;
-                                        T val = T(0);
-                                        if (i <= j && n < N)
-                                            val = (i == j) ? vjs[li]
-                                                  : (i < nvs) ? reinterpret_cast<const T*>(sb + o_v + i * TILE * (int)sizeof(T))[li]
-                                                              : Vb[(size_t)i * ldV + n];
-                                        vv[ii][v] = val;
-                                    }
-#pragma unroll
-                                for (int ii = 0; ii < kChunk; ++ii) {
-                                    double d = 0.0;
-#pragma unroll
-                                    for (int v = 0; v < VPT; ++v) d += (double)vv[ii][v] * (double)wr[v];
-                                    if (i0 + ii <= j) {          // uniform over the warp
-                                        d = warp_sum(d);
-                                        put(tile, i0 + ii, d);
-                                    }
-                                }
-                            }
-                            stg.release();
-                            tile_done(tile, j + 1);
-                        }
-                    }
-                    for (int tile = rank; nsa == 0 && tile < I.n_tiles; tile += P) {
-                        if (threadIdx.x < kRowArrays) pf_rows(threadIdx.x, tile + P);
-                        else if (threadIdx.x <= kRowArrays + j)
-                            pf_slice(Vb + (size_t)(threadIdx.x - kRowArrays) * ldV, sizeof(T), tile + P);
-                        T wr[VPT];
-#pragma unroll
-                        for (int v = 0; v < VPT; ++v) {
-                            const long long n = voxel(tile, v);
-                            wr[v] = T(0);
-                            if (n < N) {
-                                const T vj = Vj[n];
-                                const bool rz = tb && (__ldg(I.vflags + n) & PHS_VFLAG_TBLOCK);
-                                int32_t q[6];
-                                T c[6];
-                                row_nb(n, q);
-                                row_coef(I.coef, I.cw, I.m6, n, c);
-                                T lap = rz ? T(0) : lap_row(Vj, vj, q, c);
-                                if (EDGE && I.ecf && !rz) lap += edge_row(Vj, I.enb, I.ecf, n);
-                                const T w = sj * (vj - I.half_dt * lap);
-                                Vn[n] = w;
-                                wr[v] = w;
-                            }
-                        }
-                        for (int i0 = 0; i0 <= j; i0 += kChunk) {
-                            T vv[kChunk][VPT];
-#pragma unroll
-                            for (int ii = 0; ii < kChunk; ++ii)
+            bool first_cycle = true;
+            for (;;) {
+                if (cheb) {
+                    const int cycle_cols = I.m - cols;
+                    for (int j = 0;; ++j) {
+                        // ======== column j: K_{j+1} = 2/delta (A - theta) K_j - K_{j-1}, dots
+                        const T* Kj = Vb + (size_t)j * ldV;
+                        const T* Kp = Vb + (size_t)max(j - 1, 0) * ldV;
+                        T* Kn = Vb + (size_t)(j + 1) * ldV;
+                        const int ns = j + 2;
+                        const T ca = (j == 0) ? I.cheb_a : T(2) * I.cheb_a;   // (1 - theta)/delta, doubled
+                        const T cb = (j == 0) ? I.cheb_b : T(2) * I.cheb_b;   // -dt/2 / delta, doubled
+                        const T cc = (j == 0) ? T(0) : T(1);
+                        phase_begin();
+                        for (int grp = rank; grp < n_groups; grp += P) {
+                            for (int tile = grp * gt; tile < min(n_tiles, (grp + 1) * gt); ++tile) {
+                                const int nxt = tile_after(grp, tile);
+                                if (threadIdx.x < kRowArrays) pf_rows(threadIdx.x, nxt);
+                                else if (threadIdx.x <= kRowArrays + j)
+                                    pf_slice(Vb + (size_t)(threadIdx.x - kRowArrays) * ldV, sizeof(T), nxt);
+                                const bool first = tile == grp * gt;
+                                const long long n0 = voxel(tile, 0);
+                                T own[VPT], lap[VPT], prev[VPT], kn[VPT];
+                                T vv[kChunk][VPT];      // K_{j-2}, K_{j-3}, ... (in the slots 3.. of the first sums)
 #pragma unroll
                                 for (int v = 0; v < VPT; ++v) {
-                                    const long long n = voxel(tile, v);
-                                    vv[ii][v] = (i0 + ii <= j && n < N) ? Vb[(size_t)(i0 + ii) * ldV + n] : T(0);
+                                    own[v] = Kj[n0 + v * kThreads];
+                                    prev[v] = Kp[n0 + v * kThreads];
                                 }
 #pragma unroll
-                            for (int ii = 0; ii < kChunk; ++ii) {
-                                double d = 0.0;
+                                for (int e = 3; e < kChunk; ++e)
 #pragma unroll
-                                for (int v = 0; v < VPT; ++v) d += (double)vv[ii][v] * (double)wr[v];
-                                if (i0 + ii <= j) {          // uniform over the warp
-                                    d = warp_sum(d);
-                                    put(tile, i0 + ii, d);
+                                    for (int v = 0; v < VPT; ++v)
+                                        vv[e][v] = (j + 1 >= e) ? Vb[(size_t)(j + 1 - e) * ldV + n0 + v * kThreads] : T(0);
+                                tile_lap<T, VPT, EDGE, NB>(I, Kj, n0, tb, own, lap);
+#pragma unroll
+                                for (int v = 0; v < VPT; ++v) {
+                                    kn[v] = (ca * own[v] + cb * lap[v]) - cc * prev[v];
+                                    vv[0][v] = kn[v];
+                                    vv[1][v] = own[v];
+                                    vv[2][v] = prev[v];
                                 }
+                                double s[kChunk];
+#pragma unroll
+                                for (int e = 0; e < kChunk; ++e) {
+                                    s[e] = 0.0;
+#pragma unroll
+                                    for (int v = 0; v < VPT; ++v) s[e] += (double)vv[e][v] * (double)kn[v];
+                                }
+                                {
+                                    const double w = warp_sums<kChunk>(s, lane);
+                                    const int i = j + 1 - (lane >> (5 - log2_of(kChunk)));
+                                    if ((lane & (32 / kChunk - 1)) == 0 && i >= 0) put(ns, i, w, first);
+                                }
+                                for (int i0 = j + 1 - kChunk; i0 >= 0; i0 -= kChunk) {   // K_{i0}, K_{i0-1}, ...
+#pragma unroll
+                                    for (int e = 0; e < kChunk; ++e)
+#pragma unroll
+                                        for (int v = 0; v < VPT; ++v)
+                                            vv[e][v] = (i0 >= e) ? Vb[(size_t)(i0 - e) * ldV + n0 + v * kThreads] : T(0);
+#pragma unroll
+                                    for (int e = 0; e < kChunk; ++e) {
+                                        s[e] = 0.0;
+#pragma unroll
+                                        for (int v = 0; v < VPT; ++v) s[e] += (double)vv[e][v] * (double)kn[v];
+                                    }
+                                    const double w = warp_sums<kChunk>(s, lane);
+                                    const int i = i0 - (lane >> (5 - log2_of(kChunk)));
+                                    if ((lane & (32 / kChunk - 1)) == 0 && i >= 0) put(ns, i, w, first);
+                                }
+#pragma unroll
+                                for (int v = 0; v < VPT; ++v) Kn[n0 + v * kThreads] = kn[v];
                             }
+                            group_done(ns);
                         }
-                        tile_done(tile, j + 1);
+                        mark(PF_A);
+                        if (!barrier_sums(ns)) { aborted = true; break; }
+                        iters_solve += 1;
+                        cols += 1;
+                        decide_cheb(j, cycle_cols);
+                        act = ctl.action;
+                        mark(PF_A_WAIT);
+                        if (prof_on && threadIdx.x == 0) pf[PF_SOLVE_ITERS] += 1;
+                        if (act != ACT_NEXT_J) break;
                     }
-                    groups_done(j + 1);
-                    mark(PF_A);
-                    if (!team_sync<ST>(I.sync, P, abort_word, ctl, sc, I.prof, [&]() { leader_dots(j); })) { aborted = true; break; }
-                    load_shc(j + 1);
-                    mark(PF_A_WAIT);
-                    // ============ phase C: u = w - sum_i c_i V_i  (in place), ||u||^2
-                    int nsc = 0;
-                    if constexpr (ST) {
-                        stg.begin();
-                        const int o_w = stg.add(Vn, sizeof(T));
-                        const int nvs = min(j + 1, stg.vec_cap());
-                        const int o_v = stg.lay_off;
-                        for (int i = 0; i < nvs; ++i) stg.add(Vb + (size_t)i * ldV, sizeof(T));
-                        nsc = stg.publish(rank, P, I.n_tiles);
-                        for (int tile = rank; nsc > 0 && tile < I.n_tiles; tile += P) {
-                            const unsigned char* sb = stg.acquire(abort_word);
-                            double acc[VPT];
+                } else {
+                    for (int j = 0;; ++j) {
+                        // ======== phase A: w = A (s_j V_j) -> V_{j+1}; dots <V_i, w>
+                        const T sj = (T)ctl.sj;
+                        const T* Vj = Vb + (size_t)j * ldV;
+                        T* Vn = Vb + (size_t)(j + 1) * ldV;
+                        const int ns = j + 1;
+                        phase_begin();
+                        for (int grp = rank; grp < n_groups; grp += P) {
+                            for (int tile = grp * gt; tile < min(n_tiles, (grp + 1) * gt); ++tile) {
+                                const bool first = tile == grp * gt;
+                                const long long n0 = voxel(tile, 0);
+                                T own[VPT], lap[VPT], wr[VPT];
 #pragma unroll
-                            for (int v = 0; v < VPT; ++v) {
-                                const int li = v * kThreads + threadIdx.x;
-                                const long long n = (long long)tile * TILE + li;
-                                acc[v] = (n < N) ? (double)reinterpret_cast<const T*>(sb + o_w)[li] : 0.0;
-                            }
-                            for (int i0 = 0; i0 <= j; i0 += kChunk) {
-                                T vv[kChunk][VPT];
+                                for (int v = 0; v < VPT; ++v) own[v] = Vj[n0 + v * kThreads];
+                                tile_lap<T, VPT, EDGE, NB>(I, Vj, n0, tb, own, lap);
 #pragma unroll
-                                for (int ii = 0; ii < kChunk; ++ii)
+                                for (int v = 0; v < VPT; ++v) {
+                                    wr[v] = sj * (own[v] - I.half_dt * lap[v]);
+                                    Vn[n0 + v * kThreads] = wr[v];
+                                }
+                                for (int i0 = 0; i0 <= j; i0 += kChunk) {
+                                    double s[kChunk];
 #pragma unroll
-                                    for (int v = 0; v < VPT; ++v) {
-                                        const int li = v * kThreads + threadIdx.x;
-                                        const long long n = (long long)tile * TILE + li;
-                                        const int i = i0 + ii;
-                                        T val = T(0);
-                                        if (i <= j && n < N)
-                                            val = (i < nvs) ? reinterpret_cast<const T*>(sb + o_v + i * TILE * (int)sizeof(T))[li]
-                                                            : Vb[(size_t)i * ldV + n];
-                                        vv[ii][v] = val;
+                                    for (int e = 0; e < kChunk; ++e) {
+                                        s[e] = 0.0;
+#pragma unroll
+                                        for (int v = 0; v < VPT; ++v)
+                                            if (i0 + e <= j)
+                                                s[e] += (double)Vb[(size_t)(i0 + e) * ldV + n0 + v * kThreads] *
+                                                        (double)wr[v];
                                     }
-#pragma unroll
-                                for (int ii = 0; ii < kChunk; ++ii) {
-                                    if (i0 + ii <= j) {
-                                        const double cf = shc[i0 + ii];
-#pragma unroll
-                                        for (int v = 0; v < VPT; ++v) acc[v] -= cf * (double)vv[ii][v];
-                                    }
+                                    const double w = warp_sums<kChunk>(s, lane);
+                                    const int i = i0 + (lane >> (5 - log2_of(kChunk)));
+                                    if ((lane & (32 / kChunk - 1)) == 0 && i <= j) put(ns, i, w, first);
                                 }
                             }
-                            stg.release();
-                            double a2 = 0.0;
+                            group_done(ns);
+                        }
+                        mark(PF_A);
+                        if (!barrier_sums(ns)) { aborted = true; break; }
+                        decide_dots(j);
+                        mark(PF_A_WAIT);
+                        // ======== phase C: u = w - sum_i c_i V_i  (in place), ||u||^2
+                        phase_begin();
+                        for (int grp = rank; grp < n_groups; grp += P) {
+                            for (int tile = grp * gt; tile < min(n_tiles, (grp + 1) * gt); ++tile) {
+                                const long long n0 = voxel(tile, 0);
+                                double acc[VPT], s[1] = {0.0};
 #pragma unroll
-                            for (int v = 0; v < VPT; ++v) {
-                                const long long n = voxel(tile, v);
-                                if (n < N) {
+                                for (int v = 0; v < VPT; ++v) acc[v] = (double)Vn[n0 + v * kThreads];
+#pragma unroll 4
+                                for (int i = 0; i <= j; ++i) {
+                                    const double cf = shc[i];
+#pragma unroll
+                                    for (int v = 0; v < VPT; ++v)
+                                        acc[v] -= cf * (double)Vb[(size_t)i * ldV + n0 + v * kThreads];
+                                }
+#pragma unroll
+                                for (int v = 0; v < VPT; ++v) {
                                     const T ut = (T)acc[v];
-                                    Vn[n] = ut;
-                                    a2 += (double)ut * (double)ut;
+                                    Vn[n0 + v * kThreads] = ut;
+                                    s[0] += (double)ut * (double)ut;
                                 }
+                                const double w = warp_sums<1>(s, lane);
+                                if (lane == 0) put(1, 0, w, tile == grp * gt);
                             }
-                            a2 = warp_sum(a2);
-                            put(tile, 0, a2);
-                            tile_done(tile, 1);
+                            group_done(1);
                         }
+                        mark(PF_C);
+                        if (!barrier_sums(1)) { aborted = true; break; }
+                        iters_solve += 1;
+                        decide_norm(j);
+                        act = ctl.action;
+                        mark(PF_C_WAIT);
+                        if (prof_on && threadIdx.x == 0) pf[PF_SOLVE_ITERS] += 1;
+                        if (act != ACT_NEXT_J) break;
                     }
-                    for (int tile = rank; nsc == 0 && tile < I.n_tiles; tile += P) {
-                        if (threadIdx.x <= j + 1) pf_slice(Vb + (size_t)threadIdx.x * ldV, sizeof(T), tile + P);
-                        double acc[VPT];
-#pragma unroll
-                        for (int v = 0; v < VPT; ++v) {
-                            const long long n = voxel(tile, v);
-                            acc[v] = (n < N) ? (double)Vn[n] : 0.0;
-                        }
-                        // acc -= sum_i shc[i] V_i
-                        for (int i0 = 0; i0 <= j; i0 += kChunk) {
-                            T vv[kChunk][VPT];
-#pragma unroll
-                            for (int ii = 0; ii < kChunk; ++ii)
-#pragma unroll
-                                for (int v = 0; v < VPT; ++v) {
-                                    const long long n = voxel(tile, v);
-                                    vv[ii][v] = (i0 + ii <= j && n < N) ? Vb[(size_t)(i0 + ii) * ldV + n] : T(0);
-                                }
-#pragma unroll
-                            for (int ii = 0; ii < kChunk; ++ii) {
-                                if (i0 + ii <= j) {
-                                    const double cf = shc[i0 + ii];
-#pragma unroll
-                                    for (int v = 0; v < VPT; ++v) acc[v] -= cf * (double)vv[ii][v];
-                                }
-                            }
-                        }
-                        double a2 = 0.0;
-#pragma unroll
-                        for (int v = 0; v < VPT; ++v) {
-                            const long long n = voxel(tile, v);
-                            if (n < N) {
-                                const T ut = (T)acc[v];
-                                Vn[n] = ut;
-                                a2 += (double)ut * (double)ut;
-                            }
-                        }
-                        a2 = warp_sum(a2);
-                        put(tile, 0, a2);
-                        tile_done(tile, 1);
-                    }
-                    groups_done(1);
-                    mark(PF_C);
-                    if (!team_sync<ST>(I.sync, P, abort_word, ctl, sc, I.prof, [&]() { leader_norm(j); })) { aborted = true; break; }
-                    act = read_action();
-                    mark(PF_C_WAIT);
-                    if (prof_on && threadIdx.x == 0) pf[PF_SOLVE_ITERS] += 1;
-                    if (act != ACT_NEXT_J) break;
-                    ++j;
                 }
                 if (aborted) break;
                 if (act == ACT_FAIL) { retired = true; break; }
                 // ============ phase X: x += sum_j c_j V_j
                 const int k = ctl.k;
-                load_shc(k);
                 const bool final = (act == ACT_UPDATE_FINAL);
                 const bool react = final && fuse_next;
+                if (final) account_solve();
                 int nsx = 0;
                 if constexpr (ST) {
                     stg.begin();
-                    const int o_x = stg.add(I.x, sizeof(T));
-                    const int o_dx = (final && I.dx) ? stg.add(I.dx, sizeof(T)) : -1;
+                    const int o_ud = stg.add(UD, sizeof(P2));
+                    const int o_x = first_cycle ? -1 : stg.add(I.x, sizeof(T));
                     const int o_h = react ? stg.add(hout, sizeof(T)) : -1;
                     const int o_fl = react ? stg.add(I.vflags, 1) : -1;
                     const int nvs = min(k, stg.vec_cap());
                     const int o_v = stg.lay_off;
                     for (int i = 0; i < nvs; ++i) stg.add(Vb + (size_t)i * ldV, sizeof(T));
-                    nsx = stg.publish(rank, P, I.n_tiles);
-                    for (int tile = rank; nsx > 0 && tile < I.n_tiles; tile += P) {
-                        const unsigned char* sb = stg.acquire(abort_word);
-                        const T* xs = reinterpret_cast<const T*>(sb + o_x);
-                        double acc[VPT];
-#pragma unroll
-                        for (int v = 0; v < VPT; ++v) {
-                            const int li = v * kThreads + threadIdx.x;
-                            acc[v] = ((long long)tile * TILE + li < N) ? (double)xs[li] : 0.0;
-                        }
-                        for (int i0 = 0; i0 < k; i0 += kChunk) {
-                            T vv[kChunk][VPT];
-#pragma unroll
-                            for (int ii = 0; ii < kChunk; ++ii)
-#pragma unroll
-                                for (int v = 0; v < VPT; ++v) {
-                                    const int li = v * kThreads + threadIdx.x;
-                                    const long long n = (long long)tile * TILE + li;
-                                    const int i = i0 + ii;
-                                    T val = T(0);
-                                    if (i < k && n < N)
-                                        val = (i < nvs) ? reinterpret_cast<const T*>(sb + o_v + i * TILE * (int)sizeof(T))[li]
-                                                        : Vb[(size_t)i * ldV + n];
-                                    vv[ii][v] = val;
-                                }
-#pragma unroll
-                            for (int ii = 0; ii < kChunk; ++ii) {
-                                if (i0 + ii < k) {
-                                    const double cf = shc[i0 + ii];
-#pragma unroll
-                                    for (int v = 0; v < VPT; ++v) acc[v] += cf * (double)vv[ii][v];
-                                }
-                            }
-                        }
-#pragma unroll
-                        for (int v = 0; v < VPT; ++v) {
-                            const int li = v * kThreads + threadIdx.x;
-                            const long long n = (long long)tile * TILE + li;
-                            if (n < N) {
-                                if (final) {
-                                    I.u[n] = (T)acc[v];
-                                    if (o_dx >= 0) {
-                                        const double dxo = (double)reinterpret_cast<const T*>(sb + o_dx)[li];
-                                        I.dx[n] = (T)(dxo + (acc[v] - (double)xs[li]));
-                                    }
-                                } else {
-                                    I.x[n] = (T)acc[v];
-                                }
-                            }
-                        }
-                        if (react) {
+                    nsx = stg.publish(rank, P, n_tiles, n_groups, gt);
+                    for (int grp = rank; nsx > 0 && grp < n_groups; grp += P) {
+                        for (int tile = grp * gt; tile < min(n_tiles, (grp + 1) * gt); ++tile) {
+                            const unsigned char* sb = stg.acquire(abort_word);
+                            double acc[VPT];
+                            T x0[VPT], dxo[VPT], hn[VPT];
+                            uint8_t fl[VPT];
                             int32_t lt[VPT];
 #pragma unroll
                             for (int v = 0; v < VPT; ++v) {
-                                const long long n = voxel(tile, v);
-                                lt[v] = (n < N && (T)acc[v] >= T(0.5)) ? I.lat[n] : 0;
+                                const int li = v * kThreads + threadIdx.x;
+                                const P2 p = reinterpret_cast<const P2*>(sb + o_ud)[li];
+                                dxo[v] = p.y;
+                                x0[v] = first_cycle ? p.x + p.y : reinterpret_cast<const T*>(sb + o_x)[li];
+                                acc[v] = (double)x0[v];
+                                hn[v] = react ? reinterpret_cast<const T*>(sb + o_h)[li] : T(0);
+                                fl[v] = react ? sb[o_fl + li] : (uint8_t)0;
                             }
+                            for (int i = 0; i < k; ++i) {
+                                const double cf = shc[i];
+#pragma unroll
+                                for (int v = 0; v < VPT; ++v) {
+                                    const int li = v * kThreads + threadIdx.x;
+                                    const T val = (i < nvs) ? reinterpret_cast<const T*>(sb + o_v + i * TILE * (int)sizeof(T))[li]
+                                                            : Vb[(size_t)i * ldV + (long long)tile * TILE + li];
+                                    acc[v] += cf * (double)val;
+                                }
+                            }
+                            stg.release();
+#pragma unroll
+                            for (int v = 0; v < VPT; ++v)
+                                lt[v] = (react && (T)acc[v] >= T(0.5)) ? I.lat[voxel(tile, v)] : 0;
 #pragma unroll
                             for (int v = 0; v < VPT; ++v) {
-                                const int li = v * kThreads + threadIdx.x;
-                                const long long n = (long long)tile * TILE + li;
-                                if (n < N)
-                                    react_voxel(n, (T)acc[v], reinterpret_cast<const T*>(sb + o_h)[li], lt[v], step, slot_now,
-                                                sb[o_fl + li], stim_next, hin);
+                                const long long n = voxel(tile, v);
+                                if (n >= N) continue;
+                                const T un = (T)acc[v];
+                                if (!final) {
+                                    I.x[n] = un;
+                                    continue;
+                                }
+                                I.u[n] = un;
+                                const T dx = I.guess ? (T)((double)dxo[v] + (acc[v] - (double)x0[v])) : T(0);
+                                if (react) {
+                                    P2 p;
+                                    p.x = react_voxel(n, un, hn[v], lt[v], step, slot_now, fl[v], stim_next, hin);
+                                    p.y = dx;
+                                    UD[n] = p;
+                                } else {
+                                    UD[n].y = dx;
+                                }
                             }
                         }
-                        stg.release();
                     }
                 }
-                for (int tile = rank; nsx == 0 && tile < I.n_tiles; tile += P) {
-                    if (threadIdx.x < k) pf_slice(Vb + (size_t)threadIdx.x * ldV, sizeof(T), tile + P);
-                    else if (threadIdx.x == k) pf_slice(I.x, sizeof(T), tile + P);
-                    else if (threadIdx.x == k + 1 && final) pf_slice(I.dx, sizeof(T), tile + P);
-                    else if (threadIdx.x == k + 2 && react) pf_slice(hout, sizeof(T), tile + P);
-                    else if (threadIdx.x == k + 3 && react) pf_slice(I.vflags, 1, tile + P);
-                    double acc[VPT], x_in[VPT];
-                    T hn[VPT];
-                    uint8_t fl[VPT];
-#pragma unroll
-                    for (int v = 0; v < VPT; ++v) {
-                        const long long n = voxel(tile, v);
-                        acc[v] = (n < N) ? (double)I.x[n] : 0.0;
-                        x_in[v] = acc[v];
-                        hn[v] = (react && n < N) ? hout[n] : T(0);
-                        fl[v] = (react && n < N) ? __ldg(I.vflags + n) : (uint8_t)0;
-                    }
-                    axpy_basis(tile, k, shc, acc);
-#pragma unroll
-                    for (int v = 0; v < VPT; ++v) {
-                        const long long n = voxel(tile, v);
-                        if (n < N) {
-                            if (final) {
-                                I.u[n] = (T)acc[v];
-                                // increment u_next - u* for the next step's initial guess
-                                if (I.dx) I.dx[n] = (T)((double)I.dx[n] + (acc[v] - x_in[v]));
-                            } else {
-                                I.x[n] = (T)acc[v];
-                            }
-                        }
-                    }
-                    if (react) {
+                for (int grp = rank; nsx == 0 && grp < n_groups; grp += P) {
+                    for (int tile = grp * gt; tile < min(n_tiles, (grp + 1) * gt); ++tile) {
+                        const int nxt = tile_after(grp, tile);
+                        if (threadIdx.x < k) pf_slice(Vb + (size_t)threadIdx.x * ldV, sizeof(T), nxt);
+                        else if (threadIdx.x == k) pf_slice(UD, sizeof(P2), nxt);
+                        else if (threadIdx.x == k + 1 && react) pf_slice(hout, sizeof(T), nxt);
+                        else if (threadIdx.x == k + 2 && react) pf_slice(I.vflags, 1, nxt);
+                        double acc[VPT];
+                        T x0[VPT], dxo[VPT], hn[VPT];
+                        uint8_t fl[VPT];
                         int32_t lt[VPT];
 #pragma unroll
                         for (int v = 0; v < VPT; ++v) {
                             const long long n = voxel(tile, v);
-                            lt[v] = (n < N && (T)acc[v] >= T(0.5)) ? I.lat[n] : 0;
+                            const P2 p = UD[n];
+                            dxo[v] = p.y;
+                            x0[v] = first_cycle ? p.x + p.y : I.x[n];
+                            acc[v] = (double)x0[v];
+                            hn[v] = react ? hout[n] : T(0);
+                            fl[v] = react ? __ldg(I.vflags + n) : (uint8_t)0;
                         }
+                        // kChunk vectors' loads at a time
+                        for (int i0 = 0; i0 < k; i0 += kChunk) {
+                            T vv[kChunk][VPT];
+#pragma unroll
+                            for (int e = 0; e < kChunk; ++e)
+#pragma unroll
+                                for (int v = 0; v < VPT; ++v)
+                                    vv[e][v] = (i0 + e < k) ? Vb[(size_t)(i0 + e) * ldV + voxel(tile, v)] : T(0);
+#pragma unroll
+                            for (int e = 0; e < kChunk; ++e) {
+                                if (i0 + e < k) {
+                                    const double cf = shc[i0 + e];
+#pragma unroll
+                                    for (int v = 0; v < VPT; ++v) acc[v] += cf * (double)vv[e][v];
+                                }
+                            }
+                        }
+#pragma unroll
+                        for (int v = 0; v < VPT; ++v)
+                            lt[v] = (react && (T)acc[v] >= T(0.5)) ? I.lat[voxel(tile, v)] : 0;
 #pragma unroll
                         for (int v = 0; v < VPT; ++v) {
                             const long long n = voxel(tile, v);
-                            if (n < N) react_voxel(n, (T)acc[v], hn[v], lt[v], step, slot_now, fl[v], stim_next, hin);
+                            if (n >= N) continue;
+                            const T un = (T)acc[v];
+                            if (!final) {
+                                I.x[n] = un;
+                                continue;
+                            }
+                            I.u[n] = un;
+                            // increment u_next - u* for the next step's initial guess
+                            const T dx = I.guess ? (T)((double)dxo[v] + (acc[v] - (double)x0[v])) : T(0);
+                            if (react) {
+                                P2 p;
+                                p.x = react_voxel(n, un, hn[v], lt[v], step, slot_now, fl[v], stim_next, hin);
+                                p.y = dx;
+                                UD[n] = p;
+                            } else {
+                                UD[n].y = dx;
+                            }
                         }
                     }
                 }
@@ -1702,40 +1639,47 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
                     fused = react;
                     break;
                 }
+                first_cycle = false;
                 // ============ true residual of the new iterate (start of the next cycle)
-                if (!team_sync<ST>(I.sync, P, abort_word, ctl, sc, I.prof, [&]() {})) { aborted = true; break; }
-                for (int tile = rank; tile < I.n_tiles; tile += P) {
-                    if (threadIdx.x < kRowArrays) pf_rows(threadIdx.x, tile + P);
-                    else if (threadIdx.x == kRowArrays) pf_slice(I.x, sizeof(T), tile + P);
-                    else if (threadIdx.x == kRowArrays + 1) pf_slice(I.b, sizeof(T), tile + P);
-                    double a2 = 0.0;
+                if (!barrier()) { aborted = true; break; }
+                phase_begin();
+                for (int grp = rank; grp < n_groups; grp += P) {
+                    for (int tile = grp * gt; tile < min(n_tiles, (grp + 1) * gt); ++tile) {
+                        const long long n0 = voxel(tile, 0);
+                        T own[VPT], lap[VPT], bn[VPT];
 #pragma unroll
-                    for (int v = 0; v < VPT; ++v) {
-                        const long long n = voxel(tile, v);
-                        if (n < N) {
-                            const T xv = I.x[n];
-                            const bool rz = tb && (__ldg(I.vflags + n) & PHS_VFLAG_TBLOCK);
-                            int32_t q[6];
-                            T c[6];
-                            row_nb(n, q);
-                            row_coef(I.coef, I.cw, I.m6, n, c);
-                            T lap = rz ? T(0) : lap_row(I.x, xv, q, c);
-                            if (EDGE && I.ecf && !rz) lap += edge_row(I.x, I.enb, I.ecf, n);
-                            const T ax = xv - I.half_dt * lap;
-                            const T r = I.b[n] - ax;
-                            Vb[n] = r;
-                            I.u[n] = xv;
-                            a2 += (double)r * (double)r;
+                        for (int v = 0; v < VPT; ++v) own[v] = I.x[n0 + v * kThreads];
+                        if (I.full_cycles) {
+#pragma unroll
+                            for (int v = 0; v < VPT; ++v) bn[v] = I.b[n0 + v * kThreads];
+                        } else {
+                            // b again from u* (the pairs are untouched until the solve ends)
+                            P2 po[VPT], pl[VPT];
+#pragma unroll
+                            for (int v = 0; v < VPT; ++v) po[v] = UD[n0 + v * kThreads];
+                            tile_lap<T, VPT, EDGE, NB>(I, UD, n0, tb, po, pl);
+#pragma unroll
+                            for (int v = 0; v < VPT; ++v) bn[v] = po[v].x + I.half_dt * pl[v].x;
                         }
+                        tile_lap<T, VPT, EDGE, NB>(I, I.x, n0, tb, own, lap);
+                        double s[1] = {0.0};
+#pragma unroll
+                        for (int v = 0; v < VPT; ++v) {
+                            const long long n = n0 + v * kThreads;
+                            const T r = bn[v] - (own[v] - I.half_dt * lap[v]);
+                            Vb[n] = r;
+                            if (n < N) I.u[n] = own[v];
+                            s[0] += (double)r * (double)r;
+                        }
+                        const double w = warp_sums<1>(s, lane);
+                        if (lane == 0) put(1, 0, w, tile == grp * gt);
                     }
-                    a2 = warp_sum(a2);
-                    put(tile, 0, a2);
-                    tile_done(tile, 1);
+                    group_done(1);
                 }
-                groups_done(1);
                 mark(PF_CHECK);
-                if (!team_sync<ST>(I.sync, P, abort_word, ctl, sc, I.prof, leader_check)) { aborted = true; break; }
-                act = read_action();
+                if (!barrier_sums(1)) { aborted = true; break; }
+                decide_check();
+                act = ctl.action;
                 mark(PF_CHECK_WAIT);
                 if (act == ACT_DONE) break;
                 if (act == ACT_FAIL) { retired = true; break; }
@@ -1743,36 +1687,39 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
             }
             if (aborted || retired) break;
         } else if (act == ACT_ZERO_B || act == ACT_DONE) {
-            const T* src = (act == ACT_ZERO_B) ? I.b : I.x;
-            for (int tile = rank; tile < I.n_tiles; tile += P) {
-                if (threadIdx.x == 0) pf_slice(src, sizeof(T), tile + P);
-                else if (threadIdx.x == 1 && fuse_next) pf_slice(hout, sizeof(T), tile + P);
-                else if (threadIdx.x == 2 && fuse_next) pf_slice(I.vflags, 1, tile + P);
-                T cv[VPT], hn[VPT];
-                uint8_t fl[VPT];
-#pragma unroll
-                for (int v = 0; v < VPT; ++v) {
-                    const long long n = voxel(tile, v);
-                    cv[v] = (n < N) ? src[n] : T(0);
-                    hn[v] = (fuse_next && n < N) ? hout[n] : T(0);
-                    fl[v] = (fuse_next && n < N) ? __ldg(I.vflags + n) : (uint8_t)0;
-                }
-#pragma unroll
-                for (int v = 0; v < VPT; ++v) {
-                    const long long n = voxel(tile, v);
-                    if (n < N) I.u[n] = cv[v];
-                }
-                if (fuse_next) {
+            // no iteration: the solve returns x0 (or b = 0)
+            for (int grp = rank; grp < n_groups; grp += P) {
+                for (int tile = grp * gt; tile < min(n_tiles, (grp + 1) * gt); ++tile) {
+                    const int nxt = tile_after(grp, tile);
+                    if (threadIdx.x == 0) pf_slice(UD, sizeof(P2), nxt);
+                    else if (threadIdx.x == 1 && fuse_next) pf_slice(hout, sizeof(T), nxt);
+                    else if (threadIdx.x == 2 && fuse_next) pf_slice(I.vflags, 1, nxt);
+                    T un[VPT], dxo[VPT], hn[VPT];
+                    uint8_t fl[VPT];
                     int32_t lt[VPT];
 #pragma unroll
                     for (int v = 0; v < VPT; ++v) {
                         const long long n = voxel(tile, v);
-                        lt[v] = (n < N && cv[v] >= T(0.5)) ? I.lat[n] : 0;
+                        const P2 p = UD[n];
+                        dxo[v] = p.y;
+                        un[v] = (act == ACT_ZERO_B) ? T(0) : p.x + p.y;
+                        hn[v] = fuse_next ? hout[n] : T(0);
+                        fl[v] = fuse_next ? __ldg(I.vflags + n) : (uint8_t)0;
                     }
+#pragma unroll
+                    for (int v = 0; v < VPT; ++v)
+                        lt[v] = (fuse_next && un[v] >= T(0.5)) ? I.lat[voxel(tile, v)] : 0;
 #pragma unroll
                     for (int v = 0; v < VPT; ++v) {
                         const long long n = voxel(tile, v);
-                        if (n < N) react_voxel(n, cv[v], hn[v], lt[v], step, slot_now, fl[v], stim_next, hin);
+                        if (n >= N) continue;
+                        I.u[n] = un[v];
+                        if (fuse_next) {
+                            P2 p;
+                            p.x = react_voxel(n, un[v], hn[v], lt[v], step, slot_now, fl[v], stim_next, hin);
+                            p.y = dxo[v];
+                            UD[n] = p;
+                        }
                     }
                 }
             }
@@ -1782,9 +1729,9 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
             break;
         }
         mark(PF_COPY);
-        // No barrier at the end of the step: each voxel's u and h are written and
-        // read again (next RHS pass 1) by the same thread, and every cross-CTA read
-        // of the next step follows its mid-RHS barrier.
+        // No barrier at the end of the step: each voxel's u, h and pair are written
+        // and read again (next RHS pass 1) by the same thread, and every cross-CTA
+        // read of the next step follows its mid-RHS barrier.
         if (prof_on && threadIdx.x == 0) pf[PF_STEPS] += 1;
         hbuf ^= 1;
         if (slot_now >= 0) {
@@ -1798,30 +1745,41 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
     if (!aborted && !retired) {
         const T* hcur = hbuf ? I.h1 : I.h0;
         if (pending >= 0 || step > sh_step0) {
-            for (int tile = rank; tile < I.n_tiles; tile += P) {
+            for (int grp = rank; grp < n_groups; grp += P)
+                for (int tile = grp * gt; tile < min(n_tiles, (grp + 1) * gt); ++tile) {
 #pragma unroll
-                for (int v = 0; v < VPT; ++v) {
-                    const long long n = voxel(tile, v);
-                    if (n < N) sample_voxel(n, I.u[n], hcur[n], step - 1);
+                    for (int v = 0; v < VPT; ++v) {
+                        const long long n = voxel(tile, v);
+                        if (n < N) sample_voxel(n, I.u[n], hcur[n], step - 1);
+                    }
                 }
-            }
         }
         pending = -1;
     }
     if (prof_on && threadIdx.x == 0) {
-        for (int i = 0; i < PF_TEAM; ++i) atomicAdd(I.prof + i, pf[i]);
+        for (int i = 0; i < kProfSlots; ++i)
+            if (i != PF_TEAM) atomicAdd(I.prof + i, pf[i]);
         atomicExch(I.prof + PF_TEAM, (unsigned long long)P);
     }
-    if (!aborted) {
-        if (!team_sync<ST>(I.sync, P, abort_word, ctl, sc, I.prof, [&]() {
-                if (threadIdx.x == 0) {
-                    I.st->step = step;
-                    I.st->id_save = id_save;
-                    I.st->pending = pending;
-                    I.st->hbuf = hbuf;
-                }
-            })) {
-            aborted = true;
+    if (threadIdx.x == 0 && !aborted) {
+        InstState* st = I.st;
+        if (rank == 0) {
+            st->arnoldi += st_arnoldi;
+            st->arnoldi_sq += st_arnoldi_sq;
+            st->solves += st_solves;
+            if (st_max_arnoldi > st->max_arnoldi) st->max_arnoldi = st_max_arnoldi;
+            st->nonconv += st_nonconv;
+        }
+        // the last CTA to leave records the progress and clears the counters: every
+        // CTA has passed its last poll by then
+        cuda::atomic_ref<unsigned int, cuda::thread_scope_device> ex(I.sync->exits);
+        if (ex.fetch_add(1u, cuda::memory_order_acq_rel) == (unsigned int)(P - 1)) {
+            st->step = step;
+            st->id_save = id_save;
+            st->pending = pending;
+            st->hbuf = hbuf;
+            I.sync->count = 0u;
+            I.sync->exits = 0u;
         }
     }
     if constexpr (ST) stg.quit();   // the producer warp drains its copies and exits
@@ -1862,23 +1820,23 @@ constexpr int kVptF64 = 1;
 // without and with the anisotropic edge terms.
 using StepFnF = void (*)(const InstDev<float>*, const int4*, long long, unsigned int*);
 using StepFnD = void (*)(const InstDev<double>*, const int4*, long long, unsigned int*);
-constexpr int kRing3 = 56 * 1024, kRing2 = 88 * 1024;
+constexpr int kRing3 = 48 * 1024, kRing2 = 84 * 1024;
 const StepFnF kStepF32[] = {step_kernel<float, kVptF32, 2, false, 0, false>, step_kernel<float, kVptF32, 3, false, 0, false>,
                             step_kernel<float, kVptF32, 4, false, 0, false>, step_kernel<float, 2, 4, false, 0, false>,
                             step_kernel<float, 2, 5, false, 0, false>,       step_kernel<float, 2, 3, false, kRing3, false>,
-                            step_kernel<float, 4, 2, false, kRing2, false>,  step_kernel<float, 2, 5, false, 0, true>,
+                            step_kernel<float, 4, 2, false, kRing2, false>,  step_kernel<float, 2, 4, false, 0, true>,
                             step_kernel<float, kVptF32, 4, false, 0, true>};
 const StepFnF kStepF32Edge[] = {step_kernel<float, kVptF32, 2, true, 0, false>, step_kernel<float, kVptF32, 3, true, 0, false>,
                                 step_kernel<float, kVptF32, 4, true, 0, false>, step_kernel<float, 2, 4, true, 0, false>,
                                 step_kernel<float, 2, 5, true, 0, false>,       step_kernel<float, 2, 3, true, kRing3, false>,
-                                step_kernel<float, 4, 2, true, kRing2, false>,  step_kernel<float, 2, 5, true, 0, true>,
+                                step_kernel<float, 4, 2, true, kRing2, false>,  step_kernel<float, 2, 4, true, 0, true>,
                                 step_kernel<float, kVptF32, 4, true, 0, true>};
-const int kMinbF32[] = {2, 3, 4, 4, 5, 3, 2, 5, 4};
+const int kMinbF32[] = {2, 3, 4, 4, 5, 3, 2, 4, 4};
 const int kVptOfF32[] = {kVptF32, kVptF32, kVptF32, 2, 2, 2, 4, 2, kVptF32};
 const int kRingF32[] = {0, 0, 0, 0, 0, kRing3, kRing2, 0, 0};
 // variants that read the compact neighbour table of every instance, and their
 // int32-table twin (launched instead when an unfinished instance has none)
-const int kTwinF32[] = {-1, -1, -1, -1, -1, -1, -1, 4, 2};
+const int kTwinF32[] = {-1, -1, -1, -1, -1, -1, -1, 3, 2};
 const StepFnD kStepF64[] = {step_kernel<double, kVptF64, 2, false, 0, false>, step_kernel<double, kVptF64, 3, false, 0, false>};
 const StepFnD kStepF64Edge[] = {step_kernel<double, kVptF64, 2, true, 0, false>,
                                 step_kernel<double, kVptF64, 3, true, 0, false>};
@@ -1894,11 +1852,25 @@ int dyn_smem_of(int prec_bytes, int variant) {
 
 // Tiles of an instance of n voxels under a variant.
 int tiles_of(long long n, int vpt) { return (int)((n + (long long)kThreads * vpt - 1) / ((long long)kThreads * vpt)); }
+// Tiles per group of partial sums, and groups, of an instance of `tiles` tiles.
+template <typename T>
+int group_tiles(int tiles) {
+    const int most = sizeof(T) == 8 ? kMaxGroupsF64 : kMaxGroupsF32;
+    return std::max(1, (tiles + most - 1) / most);
+}
+template <typename T>
+int groups_of(int tiles) {
+    const int g = group_tiles<T>(tiles);
+    return (tiles + g - 1) / g;
+}
 int vpt_of(int prec_bytes, int variant) { return prec_bytes == 8 ? kVptF64 : kVptOfF32[variant]; }
-// FP32: 64 registers, 4 CTAs/SM (the autotuner's pick on B200); FP64: 80
-// registers, 3 CTAs/SM (plain GMRES(50) on a 157k-voxel shell: 2.06 ms per
-// step against 2.46 ms with 128 registers and 2 CTAs/SM)
-constexpr int kDefaultF32 = 2, kDefaultF64 = 1;
+// FP32: 512-voxel tiles, 64 registers, 4 CTAs/SM, compact table: a lone
+// instance spreads over twice the CTAs of 1024-voxel tiles (91k voxels: 6.5
+// against 8.0 ms per 300 steps, 40k: 5.5 against 6.7 per 200) and a batch of
+// 3.9M voxels takes the same (88-92 ms per 300 steps).  FP64: 80 registers, 3
+// CTAs/SM (plain form, 160k voxels: 11.9 ms per 30 steps against 14.3 ms with
+// 124 registers and 2 CTAs/SM).
+constexpr int kDefaultF32 = 7, kDefaultF64 = 1;
 
 template <typename T>
 const void* step_fn(int variant, bool edge = false) {
@@ -1931,15 +1903,13 @@ struct InstHost {
     void* x = nullptr;
     void* b = nullptr;
     void* V = nullptr;
-    void* dx = nullptr;
+    void* ud = nullptr;
     void* hist_u = nullptr;
     void* hist_h = nullptr;
     int32_t* lat = nullptr;
     double* part = nullptr;
-    double* gpart = nullptr;
-    unsigned int* gcnt = nullptr;
-    int n_groups = 0;
-    Scalars* sc = nullptr;
+    long long part_half = 0;
+    double bound = 0.0;          // largest eigenvalue Gershgorin's theorem allows -L
     TeamSync* sync = nullptr;
     InstState* st = nullptr;
     unsigned long long* prof = nullptr;
@@ -1965,8 +1935,8 @@ struct DeviceGuard {
 };
 
 void free_inst(InstHost& h) {
-    void* ptrs[] = {h.nb, h.nbr, h.nbase, h.coef, h.cw, h.m6, h.enb, h.ecf, h.dx, h.vflags, h.vparams, h.stim, h.u, h.h0, h.h1, h.x, h.b, h.V,
-                    h.hist_u, h.hist_h, h.lat, h.part, h.gpart, h.gcnt, h.sc, h.sync, h.st, h.prof};
+    void* ptrs[] = {h.nb, h.nbr, h.nbase, h.coef, h.cw, h.m6, h.enb, h.ecf, h.ud, h.vflags, h.vparams, h.stim, h.u, h.h0, h.h1, h.x, h.b, h.V,
+                    h.hist_u, h.hist_h, h.lat, h.part, h.sync, h.st, h.prof};
     for (void* p : ptrs) dev_free(p, 0);
     h = InstHost();
 }
@@ -2003,7 +1973,6 @@ struct phs_engine {
     bool test_overcount = false;  // test hook: first team waits for one CTA too many
     int default_cps = 0;     // CTAs per SM when advance() is given 0 (0: occupancy limit)
     int wave_instances = 0;  // instances per launch wave (0: as many as the grid holds)
-    bool group_sums = true;  // FP64: partial sums combined in groups of tiles before the leader
     bool compact_nb = true;  // instances read the compact neighbour table when they have one
 };
 
@@ -2075,6 +2044,30 @@ __global__ void nb_slot_kinds(long long n, const int32_t* nb, const T* coef, con
         for (int o = 16; o > 0; o >>= 1) a |= __shfl_xor_sync(0xffffffffu, a, o);
         if ((threadIdx.x & 31) == 0 && a) atomicOr(flags + k, a);
     }
+}
+
+// Largest over the rows of (diagonal of -L) + (sum of its off-diagonal
+// magnitudes), the bound Gershgorin's theorem gives for the eigenvalues of -L;
+// rounded up to FP32, whose bit patterns of non-negative values order as
+// integers (NaN above all).
+template <typename T>
+__global__ void row_bound(long long n, const T* coef, const T* cw, const uint8_t* m6, const T* ecf, unsigned int* out) {
+    float b = 0.f;
+    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
+        double diag = 0.0, off = 0.0;
+        for (int k = 0; k < 6; ++k) {
+            const double c = cw ? (((m6[v] >> k) & 1u) ? (double)cw[v] : 0.0) : (double)coef[6 * v + k];
+            diag += c;
+            off += fabs(c);
+            if (ecf) off += 2.0 * fabs((double)ecf[6 * v + k]);
+        }
+        const float r = __double2float_ru(diag + off);
+        if (!(r <= b)) b = r;
+    }
+    if (!(b >= 0.f)) b = __int_as_float(0x7fffffff);
+    unsigned int u = __float_as_uint(b);
+    for (int o = 16; o > 0; o >>= 1) u = max(u, __shfl_xor_sync(0xffffffffu, u, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(out, u);
 }
 
 // One CTA of 256 threads per 512-voxel block: for slots 2..5 the base offset
@@ -2194,8 +2187,8 @@ int validate_desc(const phs_instance_desc* d) {
     return PHS_OK;
 }
 
-// Build the compact neighbour table (decode_nb) of an instance whose tables
-// are on the device (h.nb with the coefficients).  Leaves h.nbr null when a
+// Build the compact neighbour table (decode_nb) and the eigenvalue bound of an
+// instance whose tables are on the device (h.nb with the coefficients).  Leaves h.nbr null when a
 // present neighbour of slot 0 is not n + 1, one of slot 1 not n - 1, or a
 // block's offsets of another slot do not fit int16.
 template <typename T>
@@ -2209,9 +2202,14 @@ int build_compact_nb(InstHost& h) {
     if (ce == cudaSuccess) {
         nb_slot_kinds<T><<<(unsigned)blocks, 256>>>(n, (const int32_t*)h.nb, (const T*)h.coef, (const T*)h.cw,
                                                     (const uint8_t*)h.m6, d_w);
+        row_bound<T><<<(unsigned)blocks, 256>>>(n, (const T*)h.coef, (const T*)h.cw, (const uint8_t*)h.m6,
+                                                (const T*)h.ecf, d_w + 7);
         ce = cudaGetLastError();
     }
     if (ce == cudaSuccess) ce = cudaMemcpy(w, d_w, 8 * sizeof(unsigned int), cudaMemcpyDeviceToHost);
+    float bound = 0.f;
+    memcpy(&bound, &w[7], sizeof(bound));
+    h.bound = (double)bound;
     if (ce == cudaSuccess && !(w[0] & 1u) && !(w[1] & 2u)) {
         const long long nblk = h.ldv / 512;
         ce = dev_alloc((void**)&h.nbr, (size_t)h.ldv * 4 * sizeof(int16_t), 0);
@@ -2318,19 +2316,13 @@ int add_instance(phs_engine* e, const phs_instance_desc* d, int* slot) {
     PHS_ALLOC(h.x, np * sizeof(T));
     PHS_ALLOC(h.b, np * sizeof(T));
     PHS_ALLOC(h.V, np * (size_t)(h.m + 1) * sizeof(T));
-    if (d->guess) PHS_ALLOC(h.dx, np * sizeof(T));
+    PHS_ALLOC(h.ud, np * 2 * sizeof(T));
     const size_t S = (size_t)std::max(d->n_samples, 1);
     PHS_ALLOC(h.hist_u, S * n * sizeof(T));
     if (d->save_h) PHS_ALLOC(h.hist_h, S * n * sizeof(T));
     PHS_ALLOC(h.lat, np * sizeof(int32_t));
-    const size_t nparts = (size_t)h.n_tiles * (kWarpParts<T> ? kWarps : 1);
-    PHS_ALLOC(h.part, nparts * (h.m + 2) * sizeof(double));
-    h.n_groups = (h.n_tiles + kGroupTiles - 1) / kGroupTiles;
-    if (!kWarpParts<T>) {
-        PHS_ALLOC(h.gpart, (size_t)h.n_groups * (h.m + 2) * sizeof(double));
-        PHS_ALLOC(h.gcnt, (size_t)h.n_groups * sizeof(unsigned int));
-    }
-    PHS_ALLOC(h.sc, sizeof(Scalars));
+    h.part_half = (long long)groups_of<T>(h.n_tiles) * (h.m + 2);
+    PHS_ALLOC(h.part, (size_t)h.part_half * 2 * sizeof(double));
     PHS_ALLOC(h.sync, sizeof(TeamSync));
     PHS_ALLOC(h.st, sizeof(InstState));
 #undef PHS_ALLOC
@@ -2340,14 +2332,11 @@ int add_instance(phs_engine* e, const phs_instance_desc* d, int* slot) {
     fill_dev<T>((T*)h.x, (long long)np, (T)0, 0);
     fill_dev<T>((T*)h.b, (long long)np, (T)0, 0);
     cudaMemset(h.V, 0, np * (size_t)(h.m + 1) * sizeof(T));
-    if (h.dx) cudaMemset(h.dx, 0, np * sizeof(T));
+    cudaMemset(h.ud, 0, np * 2 * sizeof(T));
     cudaMemset(h.hist_u, 0, S * n * sizeof(T));
     if (h.hist_h) cudaMemset(h.hist_h, 0, S * n * sizeof(T));
     cudaMemset(h.lat, 0xff, np * sizeof(int32_t));
-    cudaMemset(h.part, 0, nparts * (h.m + 2) * sizeof(double));
-    if (h.gpart) cudaMemset(h.gpart, 0, (size_t)h.n_groups * (h.m + 2) * sizeof(double));
-    if (h.gcnt) cudaMemset(h.gcnt, 0, (size_t)h.n_groups * sizeof(unsigned int));
-    cudaMemset(h.sc, 0, sizeof(Scalars));
+    cudaMemset(h.part, 0, (size_t)h.part_half * 2 * sizeof(double));
     cudaMemset(h.sync, 0, sizeof(TeamSync));
     InstState st{};
     st.step = 0;
@@ -2378,8 +2367,21 @@ int add_instance(phs_engine* e, const phs_instance_desc* d, int* slot) {
     return PHS_OK;
 }
 
+// Which solves use the Chebyshev basis.  hg: the half width of the interval
+// of A - I.  Its Gram matrix stays positive definite in FP64 for about 25
+// columns on the stiff side (hg 3 and 15: lost at column 22-30) and longer
+// than a solve needs where it converges by 4 and more per column.  Early exit:
+// restarts of up to 20 columns stay clear of that at any hg (hg 15, 20 columns:
+// estimate within 0.5 % of Arnoldi's).  Full cycles want rounding level: up to
+// hg 1.25 (Mitchell-Schaeffer at 0.05 ms and 0.4 mm: 0.94) that takes 21-28
+// columns; beyond, Arnoldi.
+bool cheb_rule(bool full_cycles, int m, double hg) {
+    if (!(hg >= 0.0) || !std::isfinite(hg)) return false;
+    return hg <= 1.25 || (!full_cycles && m <= 20);
+}
+
 template <typename T>
-InstDev<T> make_dev(const InstHost& h, bool group_sums, int vpt, bool compact_nb) {
+InstDev<T> make_dev(const InstHost& h, int vpt, bool compact_nb) {
     InstDev<T> I{};
     I.nb = (const int32_t*)h.nb;
     if (compact_nb && h.nbr) {
@@ -2401,15 +2403,13 @@ InstDev<T> make_dev(const InstHost& h, bool group_sums, int vpt, bool compact_nb
     I.b = (T*)h.b;
     I.V = (T*)h.V;
     I.ldv = h.ldv;
-    I.dx = (T*)h.dx;
+    I.ud = (T*)h.ud;
+    I.guess = h.d.guess;
     I.hist_u = (T*)h.hist_u;
     I.hist_h = (T*)h.hist_h;
     I.lat = h.lat;
     I.part = h.part;
-    I.gpart = group_sums ? h.gpart : nullptr;
-    I.gcnt = h.gcnt;
-    I.n_groups = (tiles_of(h.n, vpt) + kGroupTiles - 1) / kGroupTiles;
-    I.sc = h.sc;
+    I.part_half = h.part_half;
     I.sync = h.sync;
     I.st = h.st;
     I.prof = h.prof;
@@ -2425,7 +2425,8 @@ InstDev<T> make_dev(const InstHost& h, bool group_sums, int vpt, bool compact_nb
     I.n_steps = h.d.n_steps;
     I.tb_steps = h.d.tblock_steps;
     I.n_tiles = tiles_of(h.n, vpt);
-    I.ps = h.m + 2;
+    I.gt = group_tiles<T>(I.n_tiles);
+    I.n_groups = groups_of<T>(I.n_tiles);
     I.model = h.d.model;
     I.m = h.m;
     I.maxiter = h.d.maxiter;
@@ -2433,6 +2434,16 @@ InstDev<T> make_dev(const InstHost& h, bool group_sums, int vpt, bool compact_nb
     I.stride = h.d.sample_stride;
     I.n_samples = h.d.n_samples;
     I.save_h = h.d.save_h;
+    // A = I - dt/2 L has its eigenvalues in 1 + [0, 2 hg]
+    const double hg = 0.5 * (0.5 * h.d.dt) * h.bound;
+    const double delta = std::max(hg, 1.0 / 16), theta = 1.0 + hg;
+    I.cheb = cheb_rule(h.d.full_cycles != 0, h.m, hg) ? 1 : 0;
+    I.cheb_a = (T)((1.0 - theta) / delta);
+    I.cheb_b = (T)(-0.5 * h.d.dt / delta);
+    // the centre and width that the stored constants stand for
+    I.delta = -(double)I.half_dt / (double)I.cheb_b;
+    I.theta = 1.0 - I.delta * (double)I.cheb_a;
+    I.t1 = -I.theta / I.delta;
     return I;
 }
 
@@ -2534,7 +2545,7 @@ int build_plan(phs_engine* e, int cps, bool edge) {
     std::vector<InstDev<T>> descs;
     descs.reserve(act.size());
     const int vpt = vpt_of((int)sizeof(T), variant_of<T>(e));
-    for (int i : act) descs.push_back(make_dev<T>(e->inst[i], e->group_sums, vpt, e->compact_nb));
+    for (int i : act) descs.push_back(make_dev<T>(e->inst[i], vpt, e->compact_nb));
     size_t bytes = descs.size() * sizeof(InstDev<T>);
     if (bytes > e->d_desc_bytes) {
         dev_free(e->d_desc, 0);
@@ -2559,7 +2570,7 @@ int build_plan(phs_engine* e, int cps, bool edge) {
         for (size_t i = w0; i < w1; ++i) measured = measured && e->inst[act[i]].weight > 0.0;
         for (size_t i = w0; i < w1; ++i) {
             const InstHost& h = e->inst[act[i]];
-            tiles.push_back(tiles_of(h.n, vpt));
+            tiles.push_back(groups_of<T>(tiles_of(h.n, vpt)));
             weight.push_back(measured ? h.weight : (double)h.n * (1.6 + h.kavg));
         }
         std::vector<int> P = team_sizes(tiles, weight, G);
@@ -2939,11 +2950,7 @@ int phs_engine_config(phs_engine* e, int key, int64_t value) {
             e->auto_prof = false;
             return set_profile(e, value != 0);
         case PHS_CFG_GROUP_SUMS:
-            if (e->group_sums != (value != 0)) {
-                e->group_sums = value != 0;
-                e->dirty = true;
-            }
-            return PHS_OK;
+            return PHS_OK;   // partial sums are always kept per group of tiles
         case PHS_CFG_COMPACT_NB:
             if (e->compact_nb != (value != 0)) {
                 e->compact_nb = value != 0;

@@ -126,12 +126,12 @@ def footprint_bytes(inst):
     n = inst.n_voxel
     n_pad = math.ceil(n / 1024) * 1024
     m = min(inst.restart, n)
-    tiles = math.ceil(n / 512)
+    groups = min(math.ceil(n / 512), 640)
     cb = 5 if getattr(inst, "cw", None) is not None else 24
     eb = 72 if getattr(inst, "coef_edge", None) is not None else 0
-    per_voxel = 24 + 8 + cb + eb + 1 + 5 * 4 + (m + 1) * 4 + 4 + (4 if inst.guess else 0)
+    per_voxel = 24 + 8 + cb + eb + 1 + 5 * 4 + (m + 1) * 4 + 4 + 8
     hist = n * inst.n_samples * 4 * (2 if inst.save_h else 1)
-    return n_pad * per_voxel + hist + tiles * 8 * (m + 2) * 8 + inst.n_steps + 64 * 1024
+    return n_pad * per_voxel + hist + groups * 2 * (m + 2) * 8 + inst.n_steps + 64 * 1024
 
 
 class _Inline:
