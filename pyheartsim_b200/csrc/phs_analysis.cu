@@ -10,7 +10,7 @@
 //                            c z + d through the electrodes within the radius
 //                            (itself included); the minimum-norm solution, as
 //                            numpy.linalg.lstsq gives, from a one-sided Jacobi
-//                            SVD of the m x 4 system (one CTA per electrode);
+//                            SVD of the m x 4 system (one warp per electrode);
 //                            velocity grad/|grad|^2, speed 1/|grad|, NaN with
 //                            fewer than 4 points or |grad|^2 <= 1e-8
 //   phs_interpolate_lat      utility/lat_map.py:29-46 -- electrode LAT spread
@@ -54,38 +54,66 @@ __device__ __forceinline__ float neg_diff<float>(float cur, float prev) { return
 template <>
 __device__ __forceinline__ double neg_diff<double>(double cur, double prev) { return -__dsub_rn(cur, prev); }
 
-// One thread per electrode, walking down time (consecutive electrodes are
-// adjacent in memory, so each time step is one coalesced row).
+// A CTA takes kLatCols adjacent electrodes (a 128- or 256-byte piece of each time
+// step's row) and splits the time steps into kLatParts consecutive parts, one
+// per group of kLatCols threads; the parts' results are then combined in time
+// order: the first NaN wins, else the first of the largest.  One thread per
+// electrode over all time steps, as before, left 2048 threads with one load in
+// flight each (2048 electrodes x 1000 steps, FP64: the call 205 us, now 45 us
+// with its synchronisation).
+constexpr int kLatCols = 32, kLatParts = 32;
 template <typename T>
-__global__ void lat_kernel(long long nt, long long ne, const T* __restrict__ egm, int32_t* __restrict__ idx) {
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < ne; e += (long long)gridDim.x * blockDim.x) {
-        T prev = egm[e];
-        T best = T(0);
-        int bi = 0;
-        bool have = false, best_nan = false;
-        for (long long t = 0; t + 1 < nt; ++t) {
-            const T cur = egm[(t + 1) * ne + e];
+__global__ void __launch_bounds__(kLatCols* kLatParts) lat_kernel(long long nt, long long ne, const T* __restrict__ egm,
+                                                                  int32_t* __restrict__ idx) {
+    __shared__ T s_best[kLatParts][kLatCols];
+    __shared__ int s_at[kLatParts][kLatCols];      // -1: no difference in the part
+    __shared__ unsigned char s_nan[kLatParts][kLatCols];
+    const int col = threadIdx.x % kLatCols, part = threadIdx.x / kLatCols;
+    const long long e = (long long)blockIdx.x * kLatCols + col;
+    const long long nd = nt - 1, per = (nd + kLatParts - 1) / kLatParts;     // differences, and per part
+    const long long t0 = part * per, t1 = (t0 + per < nd) ? t0 + per : nd;
+    T best = T(0);
+    int at = INT32_MIN;                            // none yet
+    bool found_nan = false;
+    if (e < ne && t0 < t1) {
+        const T* p = egm + t0 * ne + e;
+        T prev = *p;
+#pragma unroll 8
+        for (long long t = t0; t < t1; ++t) {
+            p += ne;
+            const T cur = *p;
             const T d = neg_diff<T>(cur, prev);
             prev = cur;
-            if (best_nan) continue;                     // the first NaN is the argmax
-            if (isnan(d)) { best_nan = true; bi = (int)t; have = true; continue; }
-            if (!have || d > best) { best = d; bi = (int)t; have = true; }
+            if (found_nan) continue;               // the first NaN is the argmax
+            if (isnan(d)) { found_nan = true; at = (int)t; continue; }
+            if (at == INT32_MIN || d > best) { best = d; at = (int)t; }
         }
-        idx[e] = bi;
     }
+    s_best[part][col] = best;
+    s_at[part][col] = (at == INT32_MIN) ? -1 : at;
+    s_nan[part][col] = found_nan;
+    __syncthreads();
+    if (part != 0 || e >= ne) return;
+    int bi = 0;
+    bool have = false;
+    for (int q = 0; q < kLatParts; ++q) {
+        const int a = s_at[q][col];
+        if (a < 0) continue;
+        if (s_nan[q][col]) { bi = a; break; }
+        const T d = s_best[q][col];
+        if (!have || d > best) { best = d; bi = a; have = true; }
+    }
+    idx[e] = bi;
 }
 
-__global__ void shift_to_zero(long long ne, int32_t* idx) {
-    __shared__ int s[kAThreads];
+__global__ void __launch_bounds__(1024) shift_to_zero(long long ne, int32_t* idx) {
+    __shared__ int s[32];
     int m = INT32_MAX;
     for (long long e = threadIdx.x; e < ne; e += blockDim.x) m = min(m, idx[e]);
-    s[threadIdx.x] = m;
+    m = __reduce_min_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = m;
     __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) s[threadIdx.x] = min(s[threadIdx.x], s[threadIdx.x + o]);
-        __syncthreads();
-    }
-    const int mn = s[0];
+    const int mn = __reduce_min_sync(0xffffffffu, s[threadIdx.x & 31]);
     for (long long e = threadIdx.x; e < ne; e += blockDim.x) idx[e] -= mn;
 }
 
@@ -93,21 +121,34 @@ __global__ void shift_to_zero(long long ne, int32_t* idx) {
 // sample).  A crossing at sample s: u[s] >= thr and u[s-1] < thr, with the
 // state before sample 0 counted as below.  The first max_k crossing samples go
 // to times[v * max_k + i]; counts[v] is the number of crossings (it may exceed
-// max_k).
+// max_k).  The pass is bound by HBM: kRows samples are loaded before any of
+// them is looked at, so a thread keeps that many loads in flight (one at a time
+// before: 91k voxels x 1000 samples 172 us = 2.1 TB/s, now 78 us = 4.7 TB/s).
+constexpr int kRows = 16, kActThreads = 64;
 template <typename T>
 __global__ void activation_kernel(long long S, long long n, const T* __restrict__ hist, long long ld, T thr, int max_k,
                                   int32_t* __restrict__ times, int32_t* __restrict__ counts) {
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
         bool above = false;
         int c = 0;
-        for (long long s = 0; s < S; ++s) {
-            const bool a = hist[s * ld + v] >= thr;
+        auto look = [&](T u, long long s) {
+            const bool a = u >= thr;
             if (a && !above) {
                 if (c < max_k) times[v * max_k + c] = (int32_t)s;
                 ++c;
             }
             above = a;
+        };
+        const T* p = hist + v;
+        long long s = 0;
+        for (; s + kRows <= S; s += kRows, p += kRows * ld) {
+            T u[kRows];
+#pragma unroll
+            for (int i = 0; i < kRows; ++i) u[i] = __ldcs(p + i * ld);
+#pragma unroll
+            for (int i = 0; i < kRows; ++i) look(u[i], s + i);
         }
+        for (; s < S; ++s, p += ld) look(*p, s);
         counts[v] = c;
     }
 }
@@ -404,6 +445,170 @@ __global__ void __launch_bounds__(kAThreads) cv_solve(long long ne, const long l
     }
 }
 
+// One warp per electrode, everything in one launch: the electrodes within the
+// radius are collected into shared memory in index order (a ballot per 32
+// candidates), Householder reflections take the m x 4 system [x y z 1 | lat] to
+// R (4 x 4) and Q^T lat, and the minimum-norm solution comes from a one-sided
+// Jacobi SVD of R, whose singular values are those of the system.  Before, a
+// count, a download of the counts, an upload of offsets, a fill and a CTA-wide
+// Jacobi over the m rows (a block reduction per column pair) took 1.08 ms for
+// 2048 electrodes; now 0.2 ms, call and transfers included.  An electrode with
+// more than kCvRows rows sets *big and the caller falls back to that form, which
+// has no limit.
+constexpr int kCvRows = 512, kCvWarps = 2;
+__global__ void __launch_bounds__(32 * kCvWarps) cv_warp(long long ne, const double* __restrict__ xyz,
+                                                         const double* __restrict__ lat, double r2,
+                                                         double* __restrict__ vvec, double* __restrict__ vmag,
+                                                         unsigned int* __restrict__ big) {
+    __shared__ double sm[kCvWarps][5][kCvRows];
+    const int lane = threadIdx.x & 31;
+    double(*col)[kCvRows] = sm[threadIdx.x >> 5];
+    const long long i = (long long)blockIdx.x * kCvWarps + (threadIdx.x >> 5);
+    if (i >= ne) return;                       // whole warps
+    const double c[3] = {xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2]};
+    int m = 0;
+    for (long long j0 = 0; j0 < ne; j0 += 32) {
+        const long long j = j0 + lane;
+        double p[3] = {0.0, 0.0, 0.0};
+        bool in = false;
+        if (j < ne) {
+            p[0] = xyz[3 * j];
+            p[1] = xyz[3 * j + 1];
+            p[2] = xyz[3 * j + 2];
+            in = dist2(c, p) <= r2;
+        }
+        const unsigned int mask = __ballot_sync(0xffffffffu, in);
+        const int at = m + __popc(mask & ((1u << lane) - 1u));
+        if (in && at < kCvRows) {
+            col[0][at] = p[0];
+            col[1][at] = p[1];
+            col[2][at] = p[2];
+            col[3][at] = 1.0;
+            col[4][at] = lat[j];
+        }
+        m += __popc(mask);
+    }
+    if (m > kCvRows) {
+        if (lane == 0) atomicOr(big, 1u);
+        return;
+    }
+    const double none = nan("");
+    if (m < 4) {
+        if (lane < 3) vvec[3 * i + lane] = none;
+        if (lane == 3) vmag[i] = none;
+        return;
+    }
+    __syncwarp();
+    auto wsum = [](double v) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        return v;
+    };
+    // Householder QR: column q, rows q.. (m >= 4)
+    double R[4][4], y[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        double ss = 0.0;
+        for (int k = q + lane; k < m; k += 32) ss += col[q][k] * col[q][k];
+        ss = wsum(ss);
+        const double a0 = col[q][q];
+        const double alpha = (a0 > 0.0) ? -sqrt(ss) : sqrt(ss);
+        // v = column - alpha e_q, H = I - 2 v v^T / v^T v, v^T v = 2 (ss - alpha a0)
+        const double vv = ss - alpha * a0;
+        double d[5];
+#pragma unroll
+        for (int t = 0; t < 5; ++t) d[t] = 0.0;
+        for (int k = q + lane; k < m; k += 32) {
+            const double vk = col[q][k] - ((k == q) ? alpha : 0.0);
+#pragma unroll
+            for (int t = 0; t < 5; ++t)
+                if (t > q) d[t] += vk * col[t][k];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int t = 0; t < 5; ++t)
+            if (t > q) d[t] = (vv != 0.0) ? wsum(d[t]) / vv : 0.0;
+        for (int k = q + lane; k < m; k += 32) {
+            const double vk = col[q][k] - ((k == q) ? alpha : 0.0);
+#pragma unroll
+            for (int t = 0; t < 5; ++t)
+                if (t > q) col[t][k] -= d[t] * vk;
+        }
+        __syncwarp();
+        R[q][q] = (vv != 0.0) ? alpha : a0;
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            if (t > q) R[q][t] = col[t][q];
+            else if (t < q) R[q][t] = 0.0;
+        y[q] = col[4][q];
+        __syncwarp();
+    }
+    if (lane != 0) return;
+    // one-sided Jacobi of R: rotate column pairs until they are orthogonal to
+    // machine precision, the rotations collected in V
+    double V[4][4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) V[r][q] = (r == q) ? 1.0 : 0.0;
+    for (int sweep = 0; sweep < 60; ++sweep) {
+        int rotated = 0;
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+#pragma unroll
+            for (int q = 1; q < 4; ++q) {
+                if (q <= p) continue;
+                double al = 0.0, be = 0.0, ga = 0.0;
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    al += R[r][p] * R[r][p];
+                    be += R[r][q] * R[r][q];
+                    ga += R[r][p] * R[r][q];
+                }
+                if (ga == 0.0 || fabs(ga) <= kEps * sqrt(al * be)) continue;
+                ++rotated;
+                const double zeta = (be - al) / (2.0 * ga);
+                const double t = copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
+                const double cs = 1.0 / sqrt(1.0 + t * t), sn = cs * t;
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const double x = R[r][p], w = R[r][q], vx = V[r][p], vw = V[r][q];
+                    R[r][p] = cs * x - sn * w;
+                    R[r][q] = sn * x + cs * w;
+                    V[r][p] = cs * vx - sn * vw;
+                    V[r][q] = sn * vx + cs * vw;
+                }
+            }
+        }
+        if (rotated == 0) break;
+    }
+    double sig2[4], ub[4], smax = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        sig2[q] = ub[q] = 0.0;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            sig2[q] += R[r][q] * R[r][q];
+            ub[q] += R[r][q] * y[r];
+        }
+        smax = fmax(smax, sqrt(sig2[q]));
+    }
+    const double tol = kEps * (double)(m > 4 ? m : 4) * smax;   // numpy lstsq rcond=None
+    double coef[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (!(sqrt(sig2[q]) > tol)) continue;
+        const double w = ub[q] / sig2[q];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) coef[r] += V[r][q] * w;
+    }
+    const double g2 = coef[0] * coef[0] + coef[1] * coef[1] + coef[2] * coef[2];
+    const bool ok = g2 > 1e-8;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) vvec[3 * i + r] = ok ? coef[r] / g2 : none;
+    vmag[i] = ok ? 1.0 / sqrt(g2) : none;
+}
+
 }  // namespace
 
 using phs::dev_alloc;
@@ -414,12 +619,14 @@ extern "C" {
 
 int phs_electrode_lat(int64_t nt, int64_t ne, const void* egm, int is_f64, int32_t* lat_out, void* stream) {
     if (nt < 2 || ne <= 0 || nt > INT32_MAX || !egm || !lat_out) return PHS_ERR_BAD_ARG;
+    if ((ne + kLatCols - 1) / kLatCols > INT32_MAX) return PHS_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
+    const unsigned int lat_blocks = (unsigned int)((ne + kLatCols - 1) / kLatCols);
     if (is_f64)
-        lat_kernel<double><<<blocks_for(ne), kAThreads, 0, s>>>(nt, ne, (const double*)egm, lat_out);
+        lat_kernel<double><<<lat_blocks, kLatCols * kLatParts, 0, s>>>(nt, ne, (const double*)egm, lat_out);
     else
-        lat_kernel<float><<<blocks_for(ne), kAThreads, 0, s>>>(nt, ne, (const float*)egm, lat_out);
-    shift_to_zero<<<1, kAThreads, 0, s>>>(ne, lat_out);
+        lat_kernel<float><<<lat_blocks, kLatCols * kLatParts, 0, s>>>(nt, ne, (const float*)egm, lat_out);
+    shift_to_zero<<<1, 1024, 0, s>>>(ne, lat_out);
     PHS_CUDA_TRY(cudaGetLastError());
     PHS_CUDA_TRY(cudaStreamSynchronize(s));
     return PHS_OK;
@@ -454,12 +661,13 @@ int phs_activation_times(int64_t S, int64_t n, const void* hist, int64_t ld, int
         (max_per_voxel > 0 && !times))
         return PHS_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    const unsigned int blocks = (unsigned int)std::min<long long>((n + 255) / 256, 65535);
+    // small CTAs: the voxels of one instance are few waves of large ones
+    const unsigned int blocks = (unsigned int)std::min<long long>((n + kActThreads - 1) / kActThreads, 1 << 20);
     if (is_f64)
-        activation_kernel<double><<<blocks, 256, 0, s>>>(S, n, (const double*)hist, ld, threshold, max_per_voxel,
+        activation_kernel<double><<<blocks, kActThreads, 0, s>>>(S, n, (const double*)hist, ld, threshold, max_per_voxel,
                                                          times, counts);
     else
-        activation_kernel<float><<<blocks, 256, 0, s>>>(S, n, (const float*)hist, ld, (float)threshold,
+        activation_kernel<float><<<blocks, kActThreads, 0, s>>>(S, n, (const float*)hist, ld, (float)threshold,
                                                         max_per_voxel, times, counts);
     PHS_CUDA_TRY(cudaGetLastError());
     return PHS_OK;
@@ -470,6 +678,27 @@ int phs_conduction_velocity(int64_t ne, const double* xyz, const double* lat, do
     if (ne <= 0 || ne > (1 << 20) || !xyz || !lat || !v_vec || !v_mag || !(radius >= 0.0)) return PHS_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     const double r2 = radius * radius;
+    {
+        // one warp per electrode; the general form below only when a
+        // neighbourhood does not fit its shared memory
+        unsigned int* big = nullptr;
+        unsigned int h_big = 0;
+        cudaError_t e = dev_alloc((void**)&big, sizeof(unsigned int), s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(big, 0, sizeof(unsigned int), s);
+        if (e == cudaSuccess) {
+            cv_warp<<<(unsigned int)((ne + kCvWarps - 1) / kCvWarps), 32 * kCvWarps, 0, s>>>(ne, xyz, lat, r2, v_vec,
+                                                                                             v_mag, big);
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&h_big, big, sizeof(h_big), cudaMemcpyDeviceToHost, s);
+        dev_free(big, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) {
+            set_last_error("phs_conduction_velocity", e);
+            return e == cudaErrorMemoryAllocation ? PHS_ERR_OOM : PHS_ERR_CUDA;
+        }
+        if (!h_big) return PHS_OK;
+    }
     int32_t* counts = nullptr;
     long long* off = nullptr;
     double* ws = nullptr;
