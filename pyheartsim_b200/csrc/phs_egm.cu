@@ -22,157 +22,300 @@ namespace phs {
 
 // Mt[e][w] = sum over incoming gradient terms (v, +-(d+1)) of
 //            +-c_v / l^3 * (D_v^T l)_d / (2 Delta),  l = x_v - x_e, |l| clamped to >= 1.
-__global__ void leadfield_kernel(int64_t n_v, int64_t n_e, const double* __restrict__ xyz,
-                                 const double* __restrict__ exyz, const double* __restrict__ c,
-                                 const double* __restrict__ D0, const int32_t* __restrict__ in_ptr,
-                                 const int32_t* __restrict__ in_src, const int8_t* __restrict__ in_dir,
-                                 double inv2d, double* __restrict__ Mt) {
-    const int64_t e = blockIdx.y;
-    const double ex = exyz[3 * e], ey = exyz[3 * e + 1], ez = exyz[3 * e + 2];
-    for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < n_v;
-         w += (int64_t)gridDim.x * blockDim.x) {
-        double acc = 0.0;
+// A thread keeps the first kLfTerms terms of its voxel (a lattice voxel has six
+// at most) in registers and walks a chunk of electrodes, so a term costs its
+// arithmetic only; that bounds the kernel (FP64), so 1 / l^3 comes from one
+// rsqrt in place of a square root and a division.  91k voxels x 64 electrodes:
+// 174 us with the terms read again for every electrode, now 99 us; the error of
+// the electrogram against 64-bit reference sums is unchanged (1e-14).
+constexpr int kLfTerms = 6, kLfElectrodes = 16;
+template <bool TENSOR>
+__global__ void __launch_bounds__(128) leadfield_kernel(int64_t n_v, int64_t n_e, const double* __restrict__ xyz,
+                                                        const double* __restrict__ exyz, const double* __restrict__ c,
+                                                        const double* __restrict__ D0,
+                                                        const int32_t* __restrict__ in_ptr,
+                                                        const int32_t* __restrict__ in_src,
+                                                        const int8_t* __restrict__ in_dir, double inv2d,
+                                                        double* __restrict__ Mt) {
+    __shared__ double se[kLfElectrodes][3];
+    const int64_t e0 = (int64_t)blockIdx.y * kLfElectrodes;
+    const int ne = (int)((n_e - e0 < kLfElectrodes) ? n_e - e0 : kLfElectrodes);
+    if ((int)threadIdx.x < 3 * ne) se[threadIdx.x / 3][threadIdx.x % 3] = exyz[3 * e0 + threadIdx.x];
+    __syncthreads();
+    for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < n_v; w += (int64_t)gridDim.x * blockDim.x) {
         const int32_t b0 = in_ptr[w], b1 = in_ptr[w + 1];
-        for (int32_t q = b0; q < b1; ++q) {
+        // a term: the source's position and the scaled row D_v^T e_d (identity: its
+        // one component and which)
+        auto load = [&](int32_t q, double (&x)[3], double (&p)[3], int& d) {
             const int32_t v = in_src[q];
             const int dd = in_dir[q];
-            const int d = (dd > 0 ? dd : -dd) - 1;
-            const double lx = xyz[3 * v] - ex, ly = xyz[3 * v + 1] - ey, lz = xyz[3 * v + 2] - ez;
-            double l = sqrt(lx * lx + ly * ly + lz * lz);
-            if (l < 1.0) l = 1.0;
-            double proj;
-            if (D0) {
-                const double* Dv = D0 + 9 * (int64_t)v;
-                proj = Dv[0 + d] * lx + Dv[3 + d] * ly + Dv[6 + d] * lz;
+            d = (dd > 0 ? dd : -dd) - 1;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) x[i] = xyz[3 * (int64_t)v + i];
+            const double s = (dd > 0) ? c[v] * inv2d : -(c[v] * inv2d);
+            if (TENSOR) {
+#pragma unroll
+                for (int i = 0; i < 3; ++i) p[i] = s * D0[9 * (int64_t)v + 3 * i + d];
             } else {
-                proj = (d == 0) ? lx : (d == 1 ? ly : lz);
+                p[0] = s;
             }
-            const double g = c[v] / (l * l * l) * proj * inv2d;
-            acc += (dd > 0) ? g : -g;
+        };
+        auto value = [&](const double (&x)[3], const double (&p)[3], int d, const double* pe) {
+            const double lx = x[0] - pe[0], ly = x[1] - pe[1], lz = x[2] - pe[2];
+            const double l2 = lx * lx + ly * ly + lz * lz;
+            const double r = (l2 < 1.0) ? 1.0 : rsqrt(l2);
+            const double proj = TENSOR ? p[0] * lx + p[1] * ly + p[2] * lz : p[0] * (d == 0 ? lx : (d == 1 ? ly : lz));
+            return proj * (r * r * r);
+        };
+        double x[kLfTerms][3], p[kLfTerms][3];
+        int d[kLfTerms];
+#pragma unroll
+        for (int t = 0; t < kLfTerms; ++t)
+            if (b0 + t < b1) load(b0 + t, x[t], p[t], d[t]);
+        for (int e = 0; e < ne; ++e) {
+            double acc = 0.0;
+#pragma unroll
+            for (int t = 0; t < kLfTerms; ++t)
+                if (b0 + t < b1) acc += value(x[t], p[t], d[t], se[e]);
+            for (int32_t q = b0 + kLfTerms; q < b1; ++q) {
+                double xq[3], pq[3];
+                int dq;
+                load(q, xq, pq, dq);
+                acc += value(xq, pq, dq, se[e]);
+            }
+            Mt[(e0 + e) * n_v + w] = acc;
         }
-        Mt[e * n_v + w] = acc;
     }
 }
 
-// FP64 C[t][e] = sum_k A[t][k] * B[e][k] over one K-split; tile 64x64, K-step 16,
-// 256 threads with a 4x4 micro-tile each.  Partials go to P[split][t][e].
-constexpr int DG_BM = 64, DG_BN = 64, DG_BK = 16;
-__global__ void __launch_bounds__(256)
+// FP64 C[t][e] = sum_k A[t][k] * B[e][k] over one K-split; partials go to
+// P[split][t][e].  128 x 64 output tile, K-steps of 16 staged through a ring of
+// three shared-memory stages by cp.async, 8 warps of 32 x 32 each on the FP64
+// matrix instruction (mma.m16n8k8; tcgen05 has no FP64 form).  The bound is the
+// FP64 units: a warp's K-step of 8 costs 16 shared-memory loads for 128 clocks
+// of matrix work.  Rows of 16 + 4 doubles keep those loads free of bank
+// conflicts.  Copies are 16 bytes where both operands' rows start on such
+// boundaries, else 8.  (64 x 64 tiles with 4 x 4 values per thread read shared
+// memory once per two multiply-adds: 1000 x 64 x 91k took 1.25 ms = 9.4
+// TFLOP/s, now 0.47 ms = 25 TFLOP/s.)
+constexpr int DG_BM = 128, DG_BN = 64, DG_BK = 16, DG_STAGES = 3, DG_LD = DG_BK + 4;
+constexpr size_t DG_SMEM = (size_t)DG_STAGES * (DG_BM + DG_BN) * DG_LD * sizeof(double);
+
+template <int BYTES>
+__device__ __forceinline__ void cp_async(double* dst, const double* src, int valid) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid) : "memory");
+}
+
+// D += A (16x8, row) * B (8x8, col): lane l holds a: rows l/4 and l/4 + 8, k l%4
+// (a[0], a[1]) and l%4 + 4 (a[2], a[3]); b: column l/4, the same k; d: rows
+// l/4 (d[0], d[1]) and l/4 + 8 (d[2], d[3]), columns 2 (l%4) and + 1.
+__device__ __forceinline__ void mma_f64(double (&d)[4], const double (&a)[4], const double (&b)[2]) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+
+template <int BYTES>
+__global__ void __launch_bounds__(256, 2)
 dgemm_tn_kernel(int64_t M, int64_t N, int64_t K, const double* __restrict__ A, int64_t lda,
                 const double* __restrict__ B, int64_t ldb, double* __restrict__ P, int64_t kchunk) {
-    __shared__ double As[DG_BK][DG_BM + 1];
-    __shared__ double Bs[DG_BK][DG_BN + 1];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    extern __shared__ __align__(16) double dg_smem[];
+    constexpr int STAGE = (DG_BM + DG_BN) * DG_LD;
+    constexpr int VAL = BYTES / 8;                              // values per copy
+    constexpr int PER_ROW = DG_BK / VAL;
     const int64_t m0 = (int64_t)blockIdx.x * DG_BM, n0 = (int64_t)blockIdx.y * DG_BN;
     const int64_t k_beg = (int64_t)blockIdx.z * kchunk;
-    const int64_t k_end = std::min<int64_t>(K, k_beg + kchunk);
-    double acc[4][4] = {};
-    for (int64_t k0 = k_beg; k0 < k_end; k0 += DG_BK) {
-        // 64x16 tiles: 1024 values each, 4 per thread
-        for (int i = threadIdx.x; i < DG_BM * DG_BK; i += 256) {
-            const int r = i / DG_BK, kk = i % DG_BK;
-            const int64_t gm = m0 + r, gk = k0 + kk;
-            As[kk][r] = (gm < M && gk < k_end) ? A[gm * lda + gk] : 0.0;
-            const int64_t gn = n0 + r;
-            Bs[kk][r] = (gn < N && gk < k_end) ? B[gn * ldb + gk] : 0.0;
+    const int64_t k_end = (K < k_beg + kchunk) ? K : k_beg + kchunk;
+    const int steps = (int)((k_end - k_beg + DG_BK - 1) / DG_BK);
+    // rows past M or N and k past k_end are filled with zeros (nothing is read)
+    auto stage_in = [&](int step) {
+        double* st = dg_smem + (step % DG_STAGES) * STAGE;
+        const int64_t k0 = k_beg + (int64_t)step * DG_BK;
+#pragma unroll
+        for (int i = 0; i < (DG_BM + DG_BN) * PER_ROW / 256; ++i) {
+            const int q = i * 256 + threadIdx.x;
+            const int row = q / PER_ROW, kk = (q % PER_ROW) * VAL;
+            const bool is_a = row < DG_BM;
+            const int64_t g = is_a ? m0 + row : n0 + (row - DG_BM);
+            const int64_t left = k_end - (k0 + kk);
+            int valid = (left >= VAL) ? BYTES : (left > 0 ? (int)left * 8 : 0);
+            if (g >= (is_a ? M : N)) valid = 0;
+            const double* src = is_a ? A : B;
+            if (valid) src += g * (is_a ? lda : ldb) + k0 + kk;
+            cp_async<BYTES>(st + row * DG_LD + kk, src, valid);
         }
-        __syncthreads();
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int wm = (warp & 3) * 32, wn = (warp >> 2) * 32;
+    const int g = lane >> 2, t = lane & 3;
+    double acc[2][4][4] = {};
+    for (int s = 0; s < DG_STAGES - 1; ++s) {
+        if (s < steps) stage_in(s);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int s = 0; s < steps; ++s) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(DG_STAGES - 2) : "memory");
+        __syncthreads();                       // stage s is in; stage s - 1 is no longer read
+        if (s + DG_STAGES - 1 < steps) stage_in(s + DG_STAGES - 1);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        const double* As = dg_smem + (s % DG_STAGES) * STAGE;
+        const double* Bs = As + DG_BM * DG_LD;
 #pragma unroll
-        for (int kk = 0; kk < DG_BK; ++kk) {
-            double a[4], b[4];
+        for (int kk = 0; kk < DG_BK; kk += 8) {
+            double a[2][4], b[4][2];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
+            for (int i = 0; i < 2; ++i) {
+                const double* p = As + (wm + 16 * i + g) * DG_LD + kk + t;
+                a[i][0] = p[0];
+                a[i][1] = p[8 * DG_LD];
+                a[i][2] = p[4];
+                a[i][3] = p[8 * DG_LD + 4];
+            }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
+            for (int j = 0; j < 4; ++j) {
+                const double* p = Bs + (wn + 8 * j + g) * DG_LD + kk + t;
+                b[j][0] = p[0];
+                b[j][1] = p[4];
+            }
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < 2; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < 4; ++j) mma_f64(acc[i][j], a[i], b[j]);
         }
-        __syncthreads();
     }
     double* Pz = P + (int64_t)blockIdx.z * M * N;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int64_t gm = m0 + ty + 16 * i;
-        if (gm >= M) continue;
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int64_t gn = n0 + tx + 16 * j;
-            if (gn < N) Pz[gm * N + gn] = acc[i][j];
-        }
-    }
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int64_t gm = m0 + wm + 16 * i + g + (r >> 1) * 8, gn = n0 + wn + 8 * j + 2 * t + (r & 1);
+                if (gm < M && gn < N) Pz[gm * N + gn] = acc[i][j][r];
+            }
 }
 
-// Sum split-K partials in split order (deterministic).
+// Sum split-K partials (deterministic): eight threads per value add an eighth of
+// the splits each, in order, and the eighths are added in order.
 template <typename TO>
-__global__ void splitk_reduce_kernel(int64_t MN, int splits, const double* __restrict__ P, TO* __restrict__ C) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < MN; i += (int64_t)gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int z = 0; z < splits; ++z) s += P[(int64_t)z * MN + i];
-        C[i] = (TO)s;
-    }
-}
-
-// ptp[e] = max_t egm[t][e] - min_t egm[t][e]
-template <typename T>
-__global__ void ptp_kernel(int64_t Tn, int64_t n_e, const T* __restrict__ egm, double* __restrict__ ptp) {
-    const int64_t e = blockIdx.x;
-    double mx = -INFINITY, mn = INFINITY;
-    for (int64_t t = threadIdx.x; t < Tn; t += blockDim.x) {
-        double v = (double)egm[t * n_e + e];
-        mx = fmax(mx, v);
-        mn = fmin(mn, v);
-    }
-    __shared__ double smx[256], smn[256];
-    smx[threadIdx.x] = mx;
-    smn[threadIdx.x] = mn;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s) {
-            smx[threadIdx.x] = fmax(smx[threadIdx.x], smx[threadIdx.x + s]);
-            smn[threadIdx.x] = fmin(smn[threadIdx.x], smn[threadIdx.x + s]);
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(int64_t MN, int splits, const double* __restrict__ P,
+                                                            TO* __restrict__ C) {
+    __shared__ double s[8][32];
+    const int col = threadIdx.x & 31, part = threadIdx.x >> 5;
+    const int per = (splits + 7) / 8;
+    const int z0 = part * per, z1 = (z0 + per < splits) ? z0 + per : splits;
+    for (int64_t i0 = (int64_t)blockIdx.x * 32; i0 < MN; i0 += (int64_t)gridDim.x * 32) {
+        const int64_t i = i0 + col;
+        double a = 0.0;
+        if (i < MN) {
+#pragma unroll 8
+            for (int z = z0; z < z1; ++z) a += P[(int64_t)z * MN + i];
+        }
+        s[part][col] = a;
+        __syncthreads();
+        if (part == 0 && i < MN) {
+            for (int q = 1; q < 8; ++q) a += s[q][col];
+            C[i] = (TO)a;
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) ptp[e] = smx[0] - smn[0];
 }
 
-// egm *= 1 / mean_e(ptp); every block recomputes the mean in the same order.
+// ptp[e] = max_t egm[t][e] - min_t egm[t][e].  A CTA takes 32 adjacent
+// electrodes (whole sectors of each time step's row) and deals the time steps to
+// 32 groups of threads.  (A CTA per electrode read one value out of each sector:
+// 118 us with scale_kernel for 1000 x 2048 FP32; now 30 us.)
+constexpr int kPtpCols = 32, kPtpParts = 32;
 template <typename T>
-__global__ void scale_kernel(int64_t total, int64_t n_e, const double* __restrict__ ptp, T* __restrict__ egm) {
-    __shared__ double s_scale;
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int64_t e = 0; e < n_e; ++e) s += ptp[e];
-        s_scale = 1.0 / (s / (double)n_e);
+__global__ void __launch_bounds__(kPtpCols* kPtpParts) ptp_kernel(int64_t Tn, int64_t n_e, const T* __restrict__ egm,
+                                                                  double* __restrict__ ptp) {
+    __shared__ double smx[kPtpParts][kPtpCols], smn[kPtpParts][kPtpCols];
+    const int col = threadIdx.x % kPtpCols, part = threadIdx.x / kPtpCols;
+    const int64_t e = (int64_t)blockIdx.x * kPtpCols + col;
+    double mx = -INFINITY, mn = INFINITY;
+    if (e < n_e) {
+#pragma unroll 8
+        for (int64_t t = part; t < Tn; t += kPtpParts) {
+            const double v = (double)egm[t * n_e + e];
+            mx = fmax(mx, v);
+            mn = fmin(mn, v);
+        }
     }
+    smx[part][col] = mx;
+    smn[part][col] = mn;
     __syncthreads();
-    const double sc = s_scale;
+    if (part != 0 || e >= n_e) return;
+    for (int q = 1; q < kPtpParts; ++q) {
+        mx = fmax(mx, smx[q][col]);
+        mn = fmin(mn, smn[q][col]);
+    }
+    ptp[e] = mx - mn;
+}
+
+// egm *= 1 / mean_e(ptp); every block recomputes the mean in the same order
+// (threads over the electrodes, then a tree).
+template <typename T>
+__global__ void __launch_bounds__(256) scale_kernel(int64_t total, int64_t n_e, const double* __restrict__ ptp,
+                                                    T* __restrict__ egm) {
+    __shared__ double s[256];
+    double a = 0.0;
+    for (int64_t e = threadIdx.x; e < n_e; e += 256) a += ptp[e];
+    s[threadIdx.x] = a;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+        if ((int)threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
+        __syncthreads();
+    }
+    const double sc = 1.0 / (s[0] / (double)n_e);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
         egm[i] = (T)((double)egm[i] * sc);
+}
+
+// Split-K plan: about two CTAs per SM, at least 256 of K each, at most
+// max_partials partial values.
+static void contract_plan(int64_t T, int64_t n_v, int64_t n_e, int64_t max_partials, int64_t* splits, int64_t* kchunk) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int64_t tiles = ((T + DG_BM - 1) / DG_BM) * ((n_e + DG_BN - 1) / DG_BN);
+    const int64_t target = 2LL * sms;
+    // whole waves of the chip: the splits that fit, not one more
+    int64_t s = std::max<int64_t>(1, std::min<int64_t>(std::max<int64_t>(1, target / tiles), (n_v + 255) / 256));
+    s = std::min<int64_t>(s, max_partials / (T * n_e));
+    int64_t kc = (n_v + s - 1) / s;
+    kc = ((kc + DG_BK - 1) / DG_BK) * DG_BK;
+    *kchunk = kc;
+    *splits = (n_v + kc - 1) / kc;
+}
+
+static cudaError_t contract_launch(int64_t T, int64_t n_v, int64_t n_e, const double* V, int64_t ldv, const double* Mt,
+                                   double* egm, double* P, int64_t splits, int64_t kchunk, cudaStream_t stream) {
+    const dim3 grid((unsigned)((T + DG_BM - 1) / DG_BM), (unsigned)((n_e + DG_BN - 1) / DG_BN), (unsigned)splits);
+    const bool wide = (((uintptr_t)V | (uintptr_t)Mt) & 15) == 0 && ldv % 2 == 0 && n_v % 2 == 0;
+    const auto fn = wide ? dgemm_tn_kernel<16> : dgemm_tn_kernel<8>;
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DG_SMEM);
+    if (e != cudaSuccess) return e;
+    fn<<<grid, 256, DG_SMEM, stream>>>(T, n_e, n_v, V, ldv, Mt, n_v, P, kchunk);
+    const int64_t MN = T * n_e;
+    splitk_reduce_kernel<double><<<(unsigned)std::min<int64_t>((MN + 31) / 32, 4736), 256, 0, stream>>>(MN, (int)splits,
+                                                                                                       P, egm);
+    return cudaGetLastError();
 }
 
 int contract_f64(int64_t T, int64_t n_v, int64_t n_e, const double* V, int64_t ldv, const double* Mt,
                  double* egm, cudaStream_t stream) {
     if (T <= 0 || n_v <= 0 || n_e <= 0 || ldv < n_v) return PHS_ERR_BAD_ARG;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t tm = (T + DG_BM - 1) / DG_BM, tn = (n_e + DG_BN - 1) / DG_BN;
-    const int64_t target = 2LL * sms;
-    int64_t splits = std::max<int64_t>(1, std::min<int64_t>((target + tm * tn - 1) / (tm * tn), (n_v + 255) / 256));
-    int64_t kchunk = (n_v + splits - 1) / splits;
-    kchunk = ((kchunk + DG_BK - 1) / DG_BK) * DG_BK;
-    splits = (n_v + kchunk - 1) / kchunk;
+    int64_t splits = 1, kchunk = 0;
+    contract_plan(T, n_v, n_e, INT64_MAX, &splits, &kchunk);
     double* P = nullptr;
     PHS_CUDA_TRY(dev_alloc((void**)&P, (size_t)splits * T * n_e * sizeof(double), stream));
-    dim3 grid((unsigned)tm, (unsigned)tn, (unsigned)splits);
-    dgemm_tn_kernel<<<grid, 256, 0, stream>>>(T, n_e, n_v, V, ldv, Mt, n_v, P, kchunk);
-    const int64_t MN = T * n_e;
-    splitk_reduce_kernel<double><<<(unsigned)std::min<int64_t>((MN + 255) / 256, 4096), 256, 0, stream>>>(
-        MN, (int)splits, P, egm);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = contract_launch(T, n_v, n_e, V, ldv, Mt, egm, P, splits, kchunk, stream);
     dev_free(P, stream);
     if (e != cudaSuccess) { set_last_error("contract_f64", e); return PHS_ERR_CUDA; }
     return PHS_OK;
@@ -184,22 +327,9 @@ int contract_f64(int64_t T, int64_t n_v, int64_t n_e, const double* V, int64_t l
 int contract_f64_into(int64_t T, int64_t n_v, int64_t n_e, const double* V, int64_t ldv, const double* Mt,
                       double* egm, double* P, int64_t max_partials, cudaStream_t stream) {
     if (T <= 0 || n_v <= 0 || n_e <= 0 || ldv < n_v || T * n_e > max_partials) return PHS_ERR_BAD_ARG;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t tm = (T + DG_BM - 1) / DG_BM, tn = (n_e + DG_BN - 1) / DG_BN;
-    const int64_t target = 2LL * sms;
-    int64_t splits = std::max<int64_t>(1, std::min<int64_t>((target + tm * tn - 1) / (tm * tn), (n_v + 255) / 256));
-    splits = std::min<int64_t>(splits, max_partials / (T * n_e));
-    int64_t kchunk = (n_v + splits - 1) / splits;
-    kchunk = ((kchunk + DG_BK - 1) / DG_BK) * DG_BK;
-    splits = (n_v + kchunk - 1) / kchunk;
-    dim3 grid((unsigned)tm, (unsigned)tn, (unsigned)splits);
-    dgemm_tn_kernel<<<grid, 256, 0, stream>>>(T, n_e, n_v, V, ldv, Mt, n_v, P, kchunk);
-    const int64_t MN = T * n_e;
-    splitk_reduce_kernel<double><<<(unsigned)std::min<int64_t>((MN + 255) / 256, 4096), 256, 0, stream>>>(
-        MN, (int)splits, P, egm);
-    cudaError_t e = cudaGetLastError();
+    int64_t splits = 1, kchunk = 0;
+    contract_plan(T, n_v, n_e, max_partials, &splits, &kchunk);
+    cudaError_t e = contract_launch(T, n_v, n_e, V, ldv, Mt, egm, P, splits, kchunk, stream);
     if (e != cudaSuccess) { set_last_error("contract_f64_into", e); return PHS_ERR_CUDA; }
     return PHS_OK;
 }
@@ -208,12 +338,13 @@ int normalize(int64_t T, int64_t n_e, void* egm, bool is_f64, cudaStream_t strea
     double* ptp = nullptr;
     PHS_CUDA_TRY(dev_alloc((void**)&ptp, (size_t)n_e * sizeof(double), stream));
     const int64_t total = T * n_e;
-    const unsigned blocks = (unsigned)std::min<int64_t>((total + 255) / 256, 2048);
+    const unsigned blocks = (unsigned)std::min<int64_t>((total + 255) / 256, 1184);
+    const unsigned cols = (unsigned)((n_e + kPtpCols - 1) / kPtpCols);
     if (is_f64) {
-        ptp_kernel<double><<<(unsigned)n_e, 256, 0, stream>>>(T, n_e, (const double*)egm, ptp);
+        ptp_kernel<double><<<cols, kPtpCols * kPtpParts, 0, stream>>>(T, n_e, (const double*)egm, ptp);
         scale_kernel<double><<<blocks, 256, 0, stream>>>(total, n_e, ptp, (double*)egm);
     } else {
-        ptp_kernel<float><<<(unsigned)n_e, 256, 0, stream>>>(T, n_e, (const float*)egm, ptp);
+        ptp_kernel<float><<<cols, kPtpCols * kPtpParts, 0, stream>>>(T, n_e, (const float*)egm, ptp);
         scale_kernel<float><<<blocks, 256, 0, stream>>>(total, n_e, ptp, (float*)egm);
     }
     cudaError_t e = cudaGetLastError();
@@ -243,9 +374,14 @@ int phs_egm_leadfield_f64(int64_t n_v, int64_t n_e, const double* voxel_xyz, con
                           const int8_t* in_dir, double inv_two_delta, double* Mt, void* stream) {
     if (n_v <= 0 || n_e <= 0 || n_e > 65535 || !voxel_xyz || !electrode_xyz || !c_voxel || !in_ptr || !Mt)
         return PHS_ERR_BAD_ARG;
-    dim3 grid((unsigned)std::min<int64_t>((n_v + 255) / 256, 1024), (unsigned)n_e);
-    leadfield_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(n_v, n_e, voxel_xyz, electrode_xyz, c_voxel, D0,
-                                                            in_ptr, in_src, in_dir, inv_two_delta, Mt);
+    const dim3 grid((unsigned)std::min<int64_t>((n_v + 127) / 128, 65535),
+                    (unsigned)((n_e + kLfElectrodes - 1) / kLfElectrodes));
+    if (D0)
+        leadfield_kernel<true><<<grid, 128, 0, (cudaStream_t)stream>>>(n_v, n_e, voxel_xyz, electrode_xyz, c_voxel, D0,
+                                                                      in_ptr, in_src, in_dir, inv_two_delta, Mt);
+    else
+        leadfield_kernel<false><<<grid, 128, 0, (cudaStream_t)stream>>>(n_v, n_e, voxel_xyz, electrode_xyz, c_voxel, D0,
+                                                                       in_ptr, in_src, in_dir, inv_two_delta, Mt);
     PHS_CUDA_TRY(cudaGetLastError());
     return PHS_OK;
 }

@@ -1,0 +1,110 @@
+"""The electrogram's kernels at the edges of their tiles, copies and alignments,
+against the same sums in plain torch FP64."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from pyheartsim_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def _p(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+# 128 x 64 output tiles, K-steps of 16, at least 256 of K per split; odd leading
+# dimensions and bases off a 16-byte boundary take the 8-byte copies
+@pytest.mark.parametrize("T,n_e,n_v,pad,shift", [(1, 1, 1, 0, 0), (127, 63, 15, 1, 0), (128, 64, 16, 0, 0),
+                                                 (129, 65, 17, 1, 1), (100, 16, 20001, 0, 0), (257, 130, 4096, 2, 1),
+                                                 (300, 70, 1001, 3, 0)])
+def test_fp64_contraction_edges(T, n_e, n_v, pad, shift, cuda_device):
+    import torch
+    g = torch.Generator(device=cuda_device).manual_seed(T + n_e + n_v)
+    ld = n_v + pad
+    store = torch.randn(T * ld + shift, dtype=torch.float64, device=cuda_device, generator=g)
+    V = store[shift:].view(T, ld)
+    Mt = torch.randn(n_e, n_v, dtype=torch.float64, device=cuda_device, generator=g)
+    out = torch.full((T, n_e), float("nan"), dtype=torch.float64, device=cuda_device)
+    _lib.check(_lib.lib().phs_egm_contract_f64(T, n_v, n_e, _p(V), ld, _p(Mt), _p(out), None), "phs_egm_contract_f64")
+    torch.cuda.synchronize()
+    want = V[:, :n_v] @ Mt.T
+    # both are FP64 sums of n_v products: n_v eps sum |v m| at most, and that is far
+    # above what either order loses
+    bound = 2 * n_v * 2.2e-16 * (V[:, :n_v].abs() @ Mt.abs().T)
+    assert bool(((out - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("terms,n_e,tensor", [(6, 1, False), (6, 16, True), (6, 17, False), (9, 33, True)])
+def test_leadfield_terms_and_chunks(terms, n_e, tensor, cuda_device):
+    """Any CSR of gradient terms, more than six to a voxel among them."""
+    import torch
+    rng = np.random.default_rng(terms * 100 + n_e)
+    n = 300
+    xyz, exyz = rng.uniform(0, 20, (n, 3)), rng.uniform(0, 20, (n_e, 3))
+    exyz[0] = xyz[0] + 0.1                                        # within the 1 mm clamp
+    c, D0 = rng.uniform(0, 2, n), rng.normal(size=(n, 3, 3)) if tensor else None
+    cnt = rng.integers(0, terms + 1, n)
+    ptr = np.zeros(n + 1, np.int32)
+    np.cumsum(cnt, out=ptr[1:])
+    src = rng.integers(0, n, ptr[-1]).astype(np.int32)
+    dirs = (rng.integers(1, 4, ptr[-1]) * rng.choice([-1, 1], ptr[-1])).astype(np.int8)
+    d = lambda a: None if a is None else torch.as_tensor(np.ascontiguousarray(a), device=cuda_device)
+    t = [d(a) for a in (xyz, exyz, c, D0, ptr, src, dirs)]
+    Mt = torch.empty((n_e, n), dtype=torch.float64, device=cuda_device)
+    q = lambda x: None if x is None else _p(x)
+    _lib.check(_lib.lib().phs_egm_leadfield_f64(n, n_e, q(t[0]), q(t[1]), q(t[2]), q(t[3]), q(t[4]), q(t[5]), q(t[6]),
+                                                1.25, _p(Mt), None), "phs_egm_leadfield_f64")
+    torch.cuda.synchronize()
+    want, mag = np.zeros((n_e, n)), np.zeros((n_e, n))
+    for w in range(n):
+        for k in range(ptr[w], ptr[w + 1]):
+            v, a = src[k], abs(int(dirs[k])) - 1
+            l = xyz[v] - exyz
+            proj = l[:, a] if D0 is None else l @ D0[v][:, a]
+            val = np.sign(dirs[k]) * c[v] * proj / np.maximum(np.linalg.norm(l, axis=1), 1.0) ** 3 * 1.25
+            want[:, w] += val
+            full = np.abs(l).sum(axis=1) * (1.0 if D0 is None else np.abs(D0[v]).max())
+            mag[:, w] += c[v] * full / np.maximum(np.linalg.norm(l, axis=1), 1.0) ** 3 * 1.25
+    # a term has some 20 roundings
+    assert np.all(np.abs(Mt.cpu().numpy() - want) <= 40 * 2.2e-16 * mag)
+
+
+@pytest.mark.parametrize("is64", [False, True])
+@pytest.mark.parametrize("rows,cols,ld,rows_out,ld_out", [(1, 1, 1, 1, 1), (3, 63, 63, 128, 64), (5, 64, 67, 5, 66),
+                                                          (2, 1023, 1024, 4, 1088), (7, 130, 131, 9, 131)])
+def test_split_is_exact_by_element(rows, cols, ld, rows_out, ld_out, is64, cuda_device):
+    import torch
+    g = torch.Generator(device=cuda_device).manual_seed(rows * 1000 + cols)
+    src = torch.randn((rows, ld), dtype=torch.float64, device=cuda_device, generator=g)
+    src = src if is64 else src.float()
+    hi = torch.full((rows_out, ld_out), 7, dtype=torch.uint16, device=cuda_device)
+    lo = hi.clone()
+    _lib.check(_lib.lib().phs_split_bf16(rows, cols, _p(src), ld, int(is64), _p(hi), _p(lo), rows_out, ld_out, None),
+               "phs_split_bf16")
+    torch.cuda.synchronize()
+    want_hi = torch.zeros((rows_out, ld_out), dtype=torch.bfloat16, device=cuda_device)
+    want_lo = want_hi.clone()
+    x = src[:, :cols]
+    want_hi[:rows, :cols] = x.float().bfloat16()
+    want_lo[:rows, :cols] = (x.double() - want_hi[:rows, :cols].double()).float().bfloat16()
+    assert torch.equal(hi.view(torch.bfloat16), want_hi) and torch.equal(lo.view(torch.bfloat16), want_lo)
+
+
+@pytest.mark.parametrize("is64", [False, True])
+@pytest.mark.parametrize("T,n_e", [(1, 5), (31, 1), (33, 31), (100, 33), (64, 600)])
+def test_normalise(T, n_e, is64, cuda_device):
+    import torch
+    g = torch.Generator(device=cuda_device).manual_seed(T * 1000 + n_e)
+    egm = torch.randn((T, n_e), dtype=torch.float64, device=cuda_device, generator=g)
+    egm = egm if is64 else egm.float()
+    want = egm.double()
+    want = want / (want.max(0).values - want.min(0).values).mean()
+    _lib.check(_lib.lib().phs_egm_normalize(T, n_e, _p(egm), int(is64), None), "phs_egm_normalize")
+    torch.cuda.synchronize()
+    if T == 1:                                   # no range to scale by: 1 / 0, as before
+        assert not bool(torch.isfinite(egm).any())
+        return
+    # one product per value and a mean of n_e: a few eps of the type
+    assert bool(((egm.double() - want).abs() <= (1e-14 if is64 else 3e-7) * want.abs()).all())
