@@ -78,15 +78,19 @@ __global__ void __launch_bounds__(kLatCols* kLatParts) lat_kernel(long long nt, 
     if (e < ne && t0 < t1) {
         const T* p = egm + t0 * ne + e;
         T prev = *p;
-#pragma unroll 8
-        for (long long t = t0; t < t1; ++t) {
-            p += ne;
-            const T cur = *p;
-            const T d = neg_diff<T>(cur, prev);
-            prev = cur;
-            if (found_nan) continue;               // the first NaN is the argmax
-            if (isnan(d)) { found_nan = true; at = (int)t; continue; }
-            if (at == INT32_MIN || d > best) { best = d; at = (int)t; }
+        for (long long t = t0; t < t1; t += 8) {   // eight loads in flight, the last few too
+            T cur[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) cur[q] = (t + q < t1) ? p[(t + q - t0 + 1) * ne] : T(0);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                if (t + q >= t1) break;
+                const T d = neg_diff<T>(cur[q], prev);
+                prev = cur[q];
+                if (found_nan) continue;           // the first NaN is the argmax
+                if (isnan(d)) { found_nan = true; at = (int)(t + q); continue; }
+                if (at == INT32_MIN || d > best) { best = d; at = (int)(t + q); }
+            }
         }
     }
     s_best[part][col] = best;
@@ -148,7 +152,14 @@ __global__ void activation_kernel(long long S, long long n, const T* __restrict_
 #pragma unroll
             for (int i = 0; i < kRows; ++i) look(u[i], s + i);
         }
-        for (; s < S; ++s, p += ld) look(*p, s);
+        if (s < S) {                       // the last rows, also together
+            T u[kRows];
+#pragma unroll
+            for (int i = 0; i < kRows; ++i) u[i] = (s + i < S) ? __ldcs(p + i * ld) : T(0);
+#pragma unroll
+            for (int i = 0; i < kRows; ++i)
+                if (s + i < S) look(u[i], s + i);
+        }
         counts[v] = c;
     }
 }

@@ -214,8 +214,13 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(int64_t MN, int spli
         const int64_t i = i0 + col;
         double a = 0.0;
         if (i < MN) {
-#pragma unroll 8
-            for (int z = z0; z < z1; ++z) a += P[(int64_t)z * MN + i];
+            for (int z = z0; z < z1; z += 8) {         // eight loads in flight, the last few too
+                double v[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v[q] = (z + q < z1) ? P[(int64_t)(z + q) * MN + i] : 0.0;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) a += v[q];
+            }
         }
         s[part][col] = a;
         __syncthreads();
@@ -240,11 +245,18 @@ __global__ void __launch_bounds__(kPtpCols* kPtpParts) ptp_kernel(int64_t Tn, in
     const int64_t e = (int64_t)blockIdx.x * kPtpCols + col;
     double mx = -INFINITY, mn = INFINITY;
     if (e < n_e) {
-#pragma unroll 8
-        for (int64_t t = part; t < Tn; t += kPtpParts) {
-            const double v = (double)egm[t * n_e + e];
-            mx = fmax(mx, v);
-            mn = fmin(mn, v);
+        for (int64_t t = part; t < Tn; t += 8 * kPtpParts) {   // eight loads in flight
+            T v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int64_t at = t + q * kPtpParts;
+                v[q] = egm[(at < Tn ? at : t) * n_e + e];
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                mx = fmax(mx, (double)v[q]);
+                mn = fmin(mn, (double)v[q]);
+            }
         }
     }
     smx[part][col] = mx;
