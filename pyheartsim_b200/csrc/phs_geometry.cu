@@ -7,10 +7,11 @@
 // (simulation/simulation_gpu.py:138-225).  Here the same tables come from
 // three device passes:
 //
-//   phs_lattice_neighbors  dense occupancy grid over the bounding box of the
-//                          integer lattice coordinates: scatter voxel ids,
-//                          gather the 18 neighbours; a scan over the grid in
-//                          (z, y, x) order gives the row order of the voxels
+//   phs_lattice_neighbors  one bit per cell of the bounding box of the integer
+//                          lattice coordinates; the running count of set bits
+//                          in (z, y, x) order is a voxel's rank, so a cell's
+//                          voxel is order[rank], and 18 cells give a voxel's
+//                          neighbours
 //   phs_equation_parts     P_2d, FP64, in the reference's operation order
 //                          (no contraction), so it is bit-identical
 //   phs_operator_tables    the compacted operator of compile_instance in device
@@ -22,6 +23,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <limits.h>
+#include <algorithm>
 
 #include "../../include/phs.h"
 #include "phs_common.cuh"
@@ -48,28 +50,45 @@ unsigned int grid_for(long long n) {
     return (unsigned int)b;
 }
 
-__global__ void bbox_kernel(const int32_t* __restrict__ ijk, long long n, int* mm) {
+// Bounding box.  Two CTAs per SM and one set of atomics per CTA: with a set per
+// warp of a grid of one voxel per thread, 190,000 atomics on six words took 131
+// of the call's 290 us for 1M voxels.
+constexpr unsigned int kBoxBlocks = 296;
+__global__ void __launch_bounds__(kGeoThreads) bbox_kernel(const int32_t* __restrict__ ijk, long long n, int* mm) {
+    __shared__ int s[6][kGeoThreads / 32];
     int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
+    const long long step = (long long)gridDim.x * blockDim.x;
+    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += 4 * step) {
+        int c[4][3];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const int c = ijk[3 * v + d];
-            lo[d] = min(lo[d], c);
-            hi[d] = max(hi[d], c);
+        for (int i = 0; i < 4; ++i) {          // four voxels' loads together
+            const long long q = (v + i * step < n) ? v + i * step : v;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) c[i][d] = ijk[3 * q + d];
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                lo[d] = min(lo[d], c[i][d]);
+                hi[d] = max(hi[d], c[i][d]);
+            }
     }
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[d] = min(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-            hi[d] = max(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+        const int a = __reduce_min_sync(0xffffffffu, lo[d]), b = __reduce_max_sync(0xffffffffu, hi[d]);
+        if ((threadIdx.x & 31) == 0) {
+            s[d][threadIdx.x >> 5] = a;
+            s[3 + d][threadIdx.x >> 5] = b;
         }
     }
-    if ((threadIdx.x & 31) == 0) {
-        for (int d = 0; d < 3; ++d) {
-            atomicMin(mm + d, lo[d]);
-            atomicMax(mm + 3 + d, hi[d]);
-        }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        int r = s[threadIdx.x][0];
+        for (int w = 1; w < kGeoThreads / 32; ++w)
+            r = (threadIdx.x < 3) ? min(r, s[threadIdx.x][w]) : max(r, s[threadIdx.x][w]);
+        if (threadIdx.x < 3) atomicMin(mm + threadIdx.x, r);
+        else atomicMax(mm + threadIdx.x, r);
     }
 }
 
@@ -87,97 +106,144 @@ __global__ void fill_i32(int32_t* p, long long n, int32_t v) {
         p[i] = v;
 }
 
-__global__ void scatter_kernel(const int32_t* __restrict__ ijk, long long n, Box b, int32_t* grid, unsigned int* err) {
+// Occupancy as one bit per cell of the box, 32 cells of a (z, y, x) run to a
+// word: a 1M-voxel shell's 41M cells take 5 MB, and its running counts as much,
+// so the 18 million cell reads stay in L2.  (A dense int32 grid of voxel ids, as
+// before, was 165 MB to fill, to gather from and to scan twice, and its chunk
+// counts were scanned by one CTA with a load at a time: 530 us per call, now
+// 165, 106 of them in these kernels.)
+__global__ void scatter_bits(const int32_t* __restrict__ ijk, long long n, Box b, unsigned int* bits, unsigned int* err) {
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
         const long long c = cell_of(b, ijk[3 * v], ijk[3 * v + 1], ijk[3 * v + 2]);
-        if (atomicCAS(grid + c, -1, (int32_t)v) != -1) atomicOr(err, 1u);   // two voxels in one cell
+        const unsigned int bit = 1u << (c & 31);
+        if (atomicOr(bits + (c >> 5), bit) & bit) atomicOr(err, 1u);   // two voxels in one cell
     }
 }
 
-__global__ void gather_kernel(const int32_t* __restrict__ ijk, long long n, Box b, const int32_t* __restrict__ grid,
-                              int32_t* __restrict__ nb18) {
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
-        const int x = ijk[3 * v], y = ijk[3 * v + 1], z = ijk[3 * v + 2];
+// Running counts of set bits, in three passes over chunks of kChunkWords words:
+// counts per chunk, their scan by one CTA, then each chunk's words.
+constexpr int kWordsPerThread = 8;
+constexpr int kChunkWords = kGeoThreads * kWordsPerThread;
+
+__device__ __forceinline__ int block_sum(int v, int* s) {   // every thread gets the sum; s: 8 ints
+    v = __reduce_add_sync(0xffffffffu, v);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+    __syncthreads();
+    int t = 0;
 #pragma unroll
-        for (int k = 0; k < 18; ++k)   // the padding keeps every neighbour cell inside the grid
-            nb18[18 * v + k] = grid[cell_of(b, x + c_off[k][0], y + c_off[k][1], z + c_off[k][2])];
+    for (int w = 0; w < kGeoThreads / 32; ++w) t += s[w];
+    return t;
+}
+// exclusive prefix over the CTA's threads of v; s: 8 ints
+__device__ __forceinline__ int block_prefix(int v, int* s) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
     }
+    __syncthreads();
+    if (lane == 31) s[warp] = x;
+    __syncthreads();
+    int before = 0;
+#pragma unroll
+    for (int w = 0; w < kGeoThreads / 32; ++w)
+        if (w < warp) before += s[w];
+    return before + x - v;
 }
 
-// Row order: rank of a voxel = occupied cells before its cell in (z, y, x)
-// order.  Three passes over the grid in chunks of kChunkCells.
-constexpr int kChunkCells = kGeoThreads * 4;
-
-__global__ void chunk_count(const int32_t* __restrict__ grid, long long cells, int32_t* counts) {
+__global__ void __launch_bounds__(kGeoThreads) chunk_count(const unsigned int* __restrict__ bits, long long words,
+                                                           int32_t* counts) {
     __shared__ int s[kGeoThreads / 32];
-    const long long base = (long long)blockIdx.x * kChunkCells;
+    const long long base = (long long)blockIdx.x * kChunkWords + threadIdx.x;
     int c = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const long long q = base + i * kGeoThreads + threadIdx.x;
-        if (q < cells && grid[q] >= 0) ++c;
+    for (int i = 0; i < kWordsPerThread; ++i) {
+        const long long q = base + (long long)i * kGeoThreads;
+        if (q < words) c += __popc(bits[q]);
     }
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0;
-        for (int w = 0; w < kGeoThreads / 32; ++w) t += s[w];
-        counts[blockIdx.x] = t;
+    c = block_sum(c, s);
+    if (threadIdx.x == 0) counts[blockIdx.x] = c;
+}
+
+// exclusive scan of `m` chunk counts by one CTA, 256 at a time
+__global__ void __launch_bounds__(kGeoThreads) scan_counts(int32_t* counts, long long m) {
+    __shared__ int s[kGeoThreads / 32], t[kGeoThreads / 32];
+    int run = 0;
+    for (long long a = 0; a < m; a += kGeoThreads) {
+        const long long i = a + threadIdx.x;
+        const int c = i < m ? counts[i] : 0;
+        const int p = block_prefix(c, s), all = block_sum(c, t);
+        if (i < m) counts[i] = run + p;
+        run += all;
     }
 }
 
-// exclusive scan of `m` chunk counts, one CTA (sequential over its threads' slices)
-__global__ void scan_counts(int32_t* counts, long long m) {
-    __shared__ long long part[kGeoThreads];
-    const long long per = (m + kGeoThreads - 1) / kGeoThreads;
-    const long long a = threadIdx.x * per, e = min(a + per, m);
-    long long s = 0;
-    for (long long i = a; i < e; ++i) s += counts[i];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        long long run = 0;
-        for (int t = 0; t < kGeoThreads; ++t) {
-            const long long x = part[t];
-            part[t] = run;
-            run += x;
+// prefix[word] = set bits before it
+__global__ void __launch_bounds__(kGeoThreads) chunk_prefix(const unsigned int* __restrict__ bits, long long words,
+                                                            const int32_t* __restrict__ offsets,
+                                                            int32_t* __restrict__ prefix) {
+    __shared__ int s[kGeoThreads / 32];
+    // thread t owns words 8t .. 8t+7 of the chunk
+    const long long base = (long long)blockIdx.x * kChunkWords + (long long)kWordsPerThread * threadIdx.x;
+    int p[kWordsPerThread], c = 0;
+#pragma unroll
+    for (int i = 0; i < kWordsPerThread; ++i) {
+        p[i] = c;
+        c += (base + i < words) ? __popc(bits[base + i]) : 0;
+    }
+    const int off = offsets[blockIdx.x] + block_prefix(c, s);
+#pragma unroll
+    for (int i = 0; i < kWordsPerThread; ++i)
+        if (base + i < words) prefix[base + i] = off + p[i];
+}
+
+// order[rank] = voxel, the rank being the count of occupied cells before its own
+__global__ void rank_kernel(const int32_t* __restrict__ ijk, long long n, Box b, const unsigned int* __restrict__ bits,
+                            const int32_t* __restrict__ prefix, int32_t* __restrict__ order) {
+    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
+        const long long c = cell_of(b, ijk[3 * v], ijk[3 * v + 1], ijk[3 * v + 2]);
+        const unsigned int below = bits[c >> 5] & ((1u << (c & 31)) - 1u);
+        order[prefix[c >> 5] + __popc(below)] = (int32_t)v;   // a duplicate cell's two voxels share a rank < n
+    }
+}
+
+// The 18 neighbours of each voxel; the rows go out through shared memory, a
+// CTA's 256 of them as one run.
+__global__ void __launch_bounds__(kGeoThreads) gather_kernel(const int32_t* __restrict__ ijk, long long n, Box b,
+                                                             const unsigned int* __restrict__ bits,
+                                                             const int32_t* __restrict__ prefix,
+                                                             const int32_t* __restrict__ order,
+                                                             int32_t* __restrict__ nb18) {
+    __shared__ int32_t s[kGeoThreads * 18];
+    for (long long v0 = (long long)blockIdx.x * kGeoThreads; v0 < n; v0 += (long long)gridDim.x * kGeoThreads) {
+        const long long v = v0 + threadIdx.x;
+        if (v < n) {
+            // the padding keeps every neighbour cell inside the box
+            const long long c0 = cell_of(b, ijk[3 * v], ijk[3 * v + 1], ijk[3 * v + 2]);
+            long long c[18];
+            unsigned int w[18];
+#pragma unroll
+            for (int k = 0; k < 18; ++k) {
+                c[k] = c0 + ((long long)c_off[k][2] * b.sy + c_off[k][1]) * b.sx + c_off[k][0];
+                w[k] = bits[c[k] >> 5];
+            }
+            int32_t r[18];
+#pragma unroll
+            for (int k = 0; k < 18; ++k) {
+                const unsigned int bit = 1u << (c[k] & 31);
+                r[k] = (w[k] & bit) ? prefix[c[k] >> 5] + __popc(w[k] & (bit - 1u)) : -1;
+            }
+#pragma unroll
+            for (int k = 0; k < 18; ++k) s[threadIdx.x * 18 + k] = (r[k] >= 0) ? order[r[k]] : -1;
         }
-    }
-    __syncthreads();
-    long long run = part[threadIdx.x];
-    for (long long i = a; i < e; ++i) {
-        const long long x = counts[i];
-        counts[i] = (int32_t)run;
-        run += x;
-    }
-}
-
-__global__ void chunk_order(const int32_t* __restrict__ grid, long long cells, const int32_t* __restrict__ offsets,
-                            int32_t* __restrict__ order) {
-    // cells of the chunk in order: thread t owns cells 4t .. 4t+3
-    __shared__ int s[kGeoThreads];
-    const long long base = (long long)blockIdx.x * kChunkCells + 4ll * threadIdx.x;
-    int32_t g[4];
-    int c = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        g[i] = (base + i < cells) ? grid[base + i] : -1;
-        c += (g[i] >= 0);
-    }
-    s[threadIdx.x] = c;
-    __syncthreads();
-    // exclusive scan over the CTA's threads (Hillis-Steele on shared memory)
-    for (int o = 1; o < kGeoThreads; o <<= 1) {
-        const int x = (threadIdx.x >= o) ? s[threadIdx.x - o] : 0;
         __syncthreads();
-        s[threadIdx.x] += x;
+        const int rows = (int)((n - v0 < kGeoThreads) ? n - v0 : kGeoThreads);
+        for (int i = threadIdx.x; i < rows * 18; i += kGeoThreads) nb18[18 * v0 + i] = s[i];
         __syncthreads();
     }
-    int r = offsets[blockIdx.x] + s[threadIdx.x] - c;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-        if (g[i] >= 0) order[r++] = g[i];
 }
 
 // ---- P_2d, simulation/equation_parts.py:36-114 ---------------------------------
@@ -334,12 +400,14 @@ int phs_lattice_neighbors(int64_t n, const int32_t* ijk, int32_t* nb18, int32_t*
     int h_mm[6] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN};
     int* d_mm = nullptr;
     unsigned int* d_err = nullptr;
-    int32_t* grid = nullptr;
-    int32_t* counts = nullptr;
+    unsigned int* bits = nullptr;
+    int32_t *prefix = nullptr, *counts = nullptr, *own_order = nullptr;
     int rc = PHS_OK;
     auto cleanup = [&]() {
         dev_free(counts, s);
-        dev_free(grid, s);
+        dev_free(prefix, s);
+        dev_free(own_order, s);
+        dev_free(bits, s);
         dev_free(d_err, s);
         dev_free(d_mm, s);
         cudaStreamSynchronize(s);
@@ -357,7 +425,7 @@ int phs_lattice_neighbors(int64_t n, const int32_t* ijk, int32_t* nb18, int32_t*
     GEO_TRY(dev_alloc((void**)&d_err, sizeof(unsigned int), s));
     GEO_TRY(cudaMemcpyAsync(d_mm, h_mm, sizeof(h_mm), cudaMemcpyHostToDevice, s));
     GEO_TRY(cudaMemsetAsync(d_err, 0, sizeof(unsigned int), s));
-    bbox_kernel<<<grid_for(n), kGeoThreads, 0, s>>>(ijk, n, d_mm);
+    bbox_kernel<<<std::min(grid_for(n), kBoxBlocks), kGeoThreads, 0, s>>>(ijk, n, d_mm);
     GEO_TRY(cudaGetLastError());
     GEO_TRY(cudaMemcpyAsync(h_mm, d_mm, sizeof(h_mm), cudaMemcpyDeviceToHost, s));
     GEO_TRY(cudaStreamSynchronize(s));
@@ -381,19 +449,22 @@ int phs_lattice_neighbors(int64_t n, const int32_t* ijk, int32_t* nb18, int32_t*
         return PHS_ERR_UNSUPPORTED;
     }
     const long long cells = span[0] * span[1] * span[2];
-    GEO_TRY(dev_alloc((void**)&grid, (size_t)cells * sizeof(int32_t), s));
-    fill_i32<<<grid_for(cells), kGeoThreads, 0, s>>>(grid, cells, -1);
-    scatter_kernel<<<grid_for(n), kGeoThreads, 0, s>>>(ijk, n, b, grid, d_err);
-    gather_kernel<<<grid_for(n), kGeoThreads, 0, s>>>(ijk, n, b, grid, nb18);
+    const long long words = (cells + 31) / 32, chunks = (words + kChunkWords - 1) / kChunkWords;
+    if (!order) GEO_TRY(dev_alloc((void**)&own_order, (size_t)n * sizeof(int32_t), s));
+    int32_t* const od = order ? order : own_order;
+    GEO_TRY(dev_alloc((void**)&bits, (size_t)words * sizeof(unsigned int), s));
+    GEO_TRY(dev_alloc((void**)&prefix, (size_t)words * sizeof(int32_t), s));
+    GEO_TRY(dev_alloc((void**)&counts, (size_t)chunks * sizeof(int32_t), s));
+    GEO_TRY(cudaMemsetAsync(bits, 0, (size_t)words * sizeof(unsigned int), s));
+    scatter_bits<<<grid_for(n), kGeoThreads, 0, s>>>(ijk, n, b, bits, d_err);
+    chunk_count<<<(unsigned int)chunks, kGeoThreads, 0, s>>>(bits, words, counts);
+    scan_counts<<<1, kGeoThreads, 0, s>>>(counts, chunks);
+    chunk_prefix<<<(unsigned int)chunks, kGeoThreads, 0, s>>>(bits, words, counts, prefix);
+    rank_kernel<<<grid_for(n), kGeoThreads, 0, s>>>(ijk, n, b, bits, prefix, od);
+    // (with duplicate cells some ranks hold no voxel: the call fails below, and
+    // the table it leaves is not used)
+    gather_kernel<<<grid_for(n), kGeoThreads, 0, s>>>(ijk, n, b, bits, prefix, od, nb18);
     GEO_TRY(cudaGetLastError());
-    if (order) {
-        const long long chunks = (cells + kChunkCells - 1) / kChunkCells;
-        GEO_TRY(dev_alloc((void**)&counts, (size_t)chunks * sizeof(int32_t), s));
-        chunk_count<<<(unsigned int)chunks, kGeoThreads, 0, s>>>(grid, cells, counts);
-        scan_counts<<<1, kGeoThreads, 0, s>>>(counts, chunks);
-        chunk_order<<<(unsigned int)chunks, kGeoThreads, 0, s>>>(grid, cells, counts, order);
-        GEO_TRY(cudaGetLastError());
-    }
     unsigned int h_err = 0;
     GEO_TRY(cudaMemcpyAsync(&h_err, d_err, sizeof(h_err), cudaMemcpyDeviceToHost, s));
     GEO_TRY(cudaStreamSynchronize(s));
