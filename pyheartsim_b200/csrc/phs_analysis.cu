@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(kAThreads) cv_solve(long long ne, const long l
 // 2048 electrodes; now 0.2 ms, call and transfers included.  An electrode with
 // more than kCvRows rows sets *big and the caller falls back to that form, which
 // has no limit.
-constexpr int kCvRows = 512, kCvWarps = 2;
+constexpr int kCvRows = 512, kCvWarps = 2, kCvAhead = 4;
 __global__ void __launch_bounds__(32 * kCvWarps) cv_warp(long long ne, const double* __restrict__ xyz,
                                                          const double* __restrict__ lat, double r2,
                                                          double* __restrict__ vvec, double* __restrict__ vmag,
@@ -478,26 +478,29 @@ __global__ void __launch_bounds__(32 * kCvWarps) cv_warp(long long ne, const dou
     if (i >= ne) return;                       // whole warps
     const double c[3] = {xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2]};
     int m = 0;
-    for (long long j0 = 0; j0 < ne; j0 += 32) {
-        const long long j = j0 + lane;
-        double p[3] = {0.0, 0.0, 0.0};
-        bool in = false;
-        if (j < ne) {
-            p[0] = xyz[3 * j];
-            p[1] = xyz[3 * j + 1];
-            p[2] = xyz[3 * j + 2];
-            in = dist2(c, p) <= r2;
+    for (long long j0 = 0; j0 < ne; j0 += 32 * kCvAhead) {
+        double p[kCvAhead][3];
+#pragma unroll
+        for (int a = 0; a < kCvAhead; ++a) {           // kCvAhead candidates' loads together
+            const long long j = j0 + 32 * a + lane, jj = (j < ne) ? j : i;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) p[a][d] = xyz[3 * jj + d];
         }
-        const unsigned int mask = __ballot_sync(0xffffffffu, in);
-        const int at = m + __popc(mask & ((1u << lane) - 1u));
-        if (in && at < kCvRows) {
-            col[0][at] = p[0];
-            col[1][at] = p[1];
-            col[2][at] = p[2];
-            col[3][at] = 1.0;
-            col[4][at] = lat[j];
+#pragma unroll
+        for (int a = 0; a < kCvAhead; ++a) {
+            const long long j = j0 + 32 * a + lane;
+            const bool in = j < ne && dist2(c, p[a]) <= r2;
+            const unsigned int mask = __ballot_sync(0xffffffffu, in);
+            const int at = m + __popc(mask & ((1u << lane) - 1u));
+            if (in && at < kCvRows) {
+                col[0][at] = p[a][0];
+                col[1][at] = p[a][1];
+                col[2][at] = p[a][2];
+                col[3][at] = 1.0;
+                col[4][at] = lat[j];
+            }
+            m += __popc(mask);
         }
-        m += __popc(mask);
     }
     if (m > kCvRows) {
         if (lane == 0) atomicOr(big, 1u);
@@ -580,7 +583,7 @@ __global__ void __launch_bounds__(32 * kCvWarps) cv_warp(long long ne, const dou
                 ++rotated;
                 const double zeta = (be - al) / (2.0 * ga);
                 const double t = copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-                const double cs = 1.0 / sqrt(1.0 + t * t), sn = cs * t;
+                const double cs = rsqrt(1.0 + t * t), sn = cs * t;
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
                     const double x = R[r][p], w = R[r][q], vx = V[r][p], vw = V[r][q];
