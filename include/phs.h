@@ -165,10 +165,8 @@ int64_t phs_engine_launch_count(phs_engine* eng);
                                     many as the grid holds).  Each wave is one launch over the whole
                                     grid for the same steps, one wave after another, so a wave's
                                     instances have the L2 to themselves                             */
-#define PHS_CFG_GROUP_SUMS 7  /* FP64 engines: 1 (default) combines the per-tile partial sums of
-                                 every reduction in fixed groups of 8 consecutive tiles before the
-                                 leader CTA sums the groups; 0: the leader sums every tile.  The
-                                 order is fixed either way (results do not depend on team size) */
+#define PHS_CFG_GROUP_SUMS 7  /* accepted, without effect: partial sums are kept per group of
+                                 consecutive tiles, in an order that does not depend on team size */
 #define PHS_CFG_COMPACT_NB 9  /* 1 (default): an instance whose present neighbours of slots 0 and 1
                                  are n+1 and n-1 (the +-x ones in the lattice row order) and whose
                                  other slots' offsets fit int16 around a base per 512-voxel block
@@ -201,8 +199,10 @@ int phs_engine_rebalance(phs_engine* eng);
  * phase C, [5] its barrier, [6] update, [7] residual check, [8] its barrier,
  * [9] final copy, [10] RHS pass 1 (reaction); [11] steps and
  * [12] Arnoldi iterations counted; [13] CTAs in the team at the last launch;
- * [14] nanoseconds in the leader bodies of the team's barriers (whichever CTA
- * led) and [15] team barriers passed.                                          */
+ * [14] nanoseconds between the end of a barrier and its decision (sums of the
+ * partials, solver scalars) and [15] team barriers passed.  [2] and [3] are the
+ * column passes and their barriers in the Chebyshev basis, [4] and [5] stay 0
+ * there.                                                                       */
 int phs_instance_profile(phs_engine* eng, int slot, uint64_t* out16);
 /* Bytes per voxel of the neighbour table the instance's compact-table variants
  * read: 8 (compact form, PHS_CFG_COMPACT_NB) or 24 (int32 table).              */
@@ -250,8 +250,10 @@ int phs_egm_contract_bf16x3(int64_t T, int64_t n_e, int64_t T_pad, int64_t n_e_p
                             const uint16_t* Vhi, const uint16_t* Vlo, const uint16_t* Mhi,
                             const uint16_t* Mlo, float* egm, void* work, void* stream);
 /* phs_egm_contract_bf16x3 with a tile configuration, 0 .. count-1 (output tile
- * 128 x 128 or 128 x 256, K blocks of 64 or 32 per pipeline stage); the
- * workspace size above covers every configuration.  For the autotuner.         */
+ * 128 x 128, 128 x 256 or, by pairs of CTAs, 256 x 256; K blocks of 64 or 32 per
+ * pipeline stage; a T_pad that is not a multiple of 256 takes 128 x 256 in the
+ * place of pairs); the workspace size above covers every configuration.  For the
+ * autotuner.                                                                   */
 int phs_egm_contract_bf16x3_cfg(int64_t T, int64_t n_e, int64_t T_pad, int64_t n_e_pad, int64_t K_pad,
                                 const uint16_t* Vhi, const uint16_t* Vlo, const uint16_t* Mhi,
                                 const uint16_t* Mlo, float* egm, void* work, int config, void* stream);
@@ -297,7 +299,7 @@ int phs_electrogram(int64_t T, int64_t n_v, int64_t n_e, const double* V, const 
  * reference's column order with -1 for an absent neighbour.  order (may be NULL)
  * receives the voxels sorted by (z, y, x), x fastest: order[r] = voxel of rank r.
  * PHS_ERR_BAD_TABLE: two voxels share coordinates; PHS_ERR_UNSUPPORTED: the
- * bounding box exceeds 2^31 cells.  Works in a temporary dense grid over the box. */
+ * bounding box exceeds 2^31 cells.  Works in a temporary bit per cell of the box. */
 int phs_lattice_neighbors(int64_t n, const int32_t* ijk, int32_t* nb18, int32_t* order, void* stream);
 
 /* P_2d [n][21] (FP64), bit-identical to the reference, from nb18, D0 [n][3][3]

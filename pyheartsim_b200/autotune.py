@@ -14,8 +14,8 @@ rounded to a power of two, instance count): in the process, and in a JSON file
 (``PHS_AUTOTUNE_CACHE``, default ``~/.cache/pyheartsim_b200/autotune.json``)
 so later processes on the same machine start from the same choice.
 
-:func:`tune_electrogram` picks the tile configuration (output tile 128 x 128 or
-128 x 256, K stage width and depth) of the BF16x3 electrogram contraction.
+:func:`tune_electrogram` picks the tile configuration (output tile 128 x 128,
+128 x 256 or 256 x 256 by CTA pairs, K stage width and depth) of the BF16x3 electrogram contraction.
 """
 import json
 import math
@@ -110,7 +110,7 @@ def tune(engine, steps=10, stream=None, cps_options=None, repeats=5, use_file=Tr
 
 
 _EGM_CACHE = {}
-EGM_TILE_NAMES = ("128x128 BK64 x3", "128x256 BK64 x2", "128x256 BK32 x4", "128x128 BK32 x6")
+EGM_TILE_NAMES = ("128x128 BK64 x3", "128x256 BK64 x2", "128x256 BK32 x4", "256x256 BK64 x3 (CTA pairs)")
 
 
 def tune_electrogram(T, n_e, T_pad, E_pad, K_pad, vh, vl, mh, ml, out, work, stream=None, repeats=3):

@@ -19,12 +19,11 @@
 //   warps 0..3      epilogue: tcgen05.ld 32x32b.x32 -> FP32 partial tile in HBM
 // Tile configurations (kTcConfigs; every one uses 192 KB of shared memory):
 // 128 x 128 with 3 stages of BK 64, 128 x 256 with 2 stages of BK 64, 128 x 256
-// with 4 stages of BK 32, 128 x 128 with 6 stages of BK 32.  The 256-wide tiles
-// read 0.75 of the operand bytes per FLOP of the 128-wide ones (the operands
-// stream from L2); the BK-32 rings keep more, smaller stages in flight ahead of
-// the MMAs (measured slower: their 64-byte TMA rows move less per request).
-// phs_egm_contract_bf16x3 uses kTcDefaultConfig;
-// phs_egm_contract_bf16x3_cfg takes a configuration (the autotuner's choice).
+// with 4 stages of BK 32 (slower: its 64-byte TMA rows move less per request) and
+// 256 x 256 by pairs of CTAs (egm_bf16x3_pair_kernel), the default where T_pad
+// is a multiple of 256.  The operands stream from L2, and the wider a tile the
+// fewer of their bytes it reads per FLOP.  phs_egm_contract_bf16x3_cfg takes a
+// configuration (the autotuner's choice).
 // Split-K partials are summed in split order by a second kernel.
 //
 // Every wait is bounded (kTcWaitNs); on timeout the CTA records an error word,
@@ -286,6 +285,173 @@ egm_bf16x3_kernel(const __grid_constant__ CUtensorMap map_vhi, const __grid_cons
     }
 }
 
+// The paired form: a cluster of two CTAs computes a 256 (t) x 256 (e) tile with
+// tcgen05.mma.cta_group::2 (M = 256, N = 256).  Each CTA stages its own 128 rows
+// of V and half of the 256 rows of M, 64 KB per K block of 64 in place of the
+// 96 KB a CTA of the 128 x 256 form reads, so the operands' L2 -> shared-memory
+// traffic, which bounds that form, falls by a third and three stages fit.  Each
+// CTA's loads are counted on the even CTA's "full" barrier; its thread issues
+// the MMAs for both and commits each stage to both CTAs' "empty" barriers.  The
+// accumulator's rows of a CTA lie in its own TMEM.  K blocks, products and splits
+// are those of the 128 x 256 form, in the same order, so the sums are the same.
+constexpr int TP_STAGES = 3, TP_BK = 64, TP_BN = 256;
+constexpr int TP_TILE_BYTES = TC_BM * TP_BK * 2;           // 128 rows of one part
+constexpr int TP_STAGE_BYTES = 4 * TP_TILE_BYTES;          // V hi, lo and M hi, lo of one CTA
+constexpr size_t TP_SMEM = (size_t)TP_STAGES * TP_STAGE_BYTES + 1024 + 256;
+constexpr uint32_t kLeaderMask = 0xFEFFFFFFu;              // a shared address of the pair -> the even CTA's
+
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(dst), "l"((uint64_t)map), "r"(bar & kLeaderMask), "r"(c0), "r"(c1)
+        : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(acc)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+        "h"((uint16_t)3)
+        : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
+egm_bf16x3_pair_kernel(const __grid_constant__ CUtensorMap map_vhi, const __grid_constant__ CUtensorMap map_vlo,
+                       const __grid_constant__ CUtensorMap map_mhi, const __grid_constant__ CUtensorMap map_mlo,
+                       int nkb_total, int kb_per_split, int T_pad, int part_cols, float* __restrict__ part,
+                       int* __restrict__ err) {
+    extern __shared__ __align__(1024) uint8_t tc_smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* bars = (uint64_t*)(smem + (size_t)TP_STAGES * TP_STAGE_BYTES);
+    // bars[0..S) full (the even CTA's are used), bars[S..2S) empty, bars[2S] done;  tmem base after them
+    uint32_t* tmem_slot = (uint32_t*)(bars + 2 * TP_STAGES + 1);
+    __shared__ int s_fail;
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const bool leader = (blockIdx.x & 1) == 0;
+    const int t0 = blockIdx.x * TC_BM;
+    const int e0 = blockIdx.y * TP_BN;
+    const int kb0 = blockIdx.z * kb_per_split;
+    const int nkb = max(0, min(nkb_total, kb0 + kb_per_split) - kb0);
+
+    if (threadIdx.x == 0) {
+        s_fail = 0;
+        for (int i = 0; i < 2 * TP_STAGES + 1; ++i) mbar_init(smem_u32(&bars[i]), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(TP_BN)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_sync();                // both CTAs' barriers and TMEM are there
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
+    const uint32_t done_bar = smem_u32(&bars[2 * TP_STAGES]);
+
+    if (warp == 0 && lane == 0) {
+        // ------------------------------------------------ TMA producer of this CTA's tiles
+        int issued = 0;
+        const int er = e0 + (leader ? 0 : 128);
+        for (int i = 0; i < nkb; ++i) {
+            const int s = i % TP_STAGES;
+            const int r = i / TP_STAGES;
+            if (r > 0 && !mbar_wait(smem_u32(&bars[TP_STAGES + s]), (uint32_t)((r - 1) & 1))) {
+                atomicExch(&s_fail, 1);
+                break;
+            }
+            if (*(volatile int*)&s_fail) break;
+            const uint32_t fb = smem_u32(&bars[s]);
+            uint8_t* st = smem + (size_t)s * TP_STAGE_BYTES;
+            if (leader) mbar_expect_tx(fb, 2 * TP_STAGE_BYTES);
+            const int kc = (kb0 + i) * TP_BK;
+            tma_load_2d_pair(smem_u32(st), &map_vhi, fb, kc, t0);
+            tma_load_2d_pair(smem_u32(st + TP_TILE_BYTES), &map_vlo, fb, kc, t0);
+            tma_load_2d_pair(smem_u32(st + 2 * TP_TILE_BYTES), &map_mhi, fb, kc, er);
+            tma_load_2d_pair(smem_u32(st + 3 * TP_TILE_BYTES), &map_mlo, fb, kc, er);
+            issued = i + 1;
+        }
+        // drain after a failure: the even CTA's barriers count both CTAs' loads, and
+        // neither CTA leaves before the cluster barrier below
+        if (leader && *(volatile int*)&s_fail) {
+            for (int i = max(0, issued - TP_STAGES); i < issued; ++i)
+                mbar_wait(smem_u32(&bars[i % TP_STAGES]), (uint32_t)((i / TP_STAGES) & 1));
+        }
+    } else if (leader && warp == 1 && lane == 0) {
+        // ------------------------------------------------ MMA issuer for the pair
+        const uint32_t idesc = umma_idesc_bf16(2 * TC_BM, TP_BN);
+        constexpr uint32_t SBO = 8u * TP_BK * 2u;
+        for (int i = 0; i < nkb; ++i) {
+            const int s = i % TP_STAGES;
+            const int r = i / TP_STAGES;
+            if (!mbar_wait(smem_u32(&bars[s]), (uint32_t)(r & 1))) {
+                atomicExch(&s_fail, 1);
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            uint8_t* st = smem + (size_t)s * TP_STAGE_BYTES;
+            const uint64_t dAh = umma_desc(smem_u32(st), SBO, 2);
+            const uint64_t dAl = umma_desc(smem_u32(st + TP_TILE_BYTES), SBO, 2);
+            const uint64_t dBh = umma_desc(smem_u32(st + 2 * TP_TILE_BYTES), SBO, 2);
+            const uint64_t dBl = umma_desc(smem_u32(st + 3 * TP_TILE_BYTES), SBO, 2);
+#pragma unroll
+            for (int kk = 0; kk < TP_BK / 16; ++kk) {
+                const uint64_t adv = (uint64_t)(kk * 32) >> 4;  // 16 bf16 = 32 B along K
+                umma_bf16_pair(tmem, dAh + adv, dBh + adv, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+                umma_bf16_pair(tmem, dAh + adv, dBl + adv, idesc, 1u);
+                umma_bf16_pair(tmem, dAl + adv, dBh + adv, idesc, 1u);
+            }
+            umma_commit_pair(smem_u32(&bars[TP_STAGES + s]));  // the stage is free in both CTAs
+        }
+        umma_commit_pair(done_bar);  // accumulators complete (also after a failure: drains issued MMAs)
+    }
+    __syncwarp();
+
+    // ------------------------------------------------ epilogue (all four warps): this CTA's 128 rows
+    const bool ok = mbar_wait(done_bar, 0u);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (!ok) atomicExch(&s_fail, 1);
+    __syncthreads();
+    const int row = t0 + warp * 32 + lane;
+    float* out = part + ((size_t)blockIdx.z * T_pad + row) * part_cols + e0;
+    if (!s_fail && nkb > 0) {
+#pragma unroll 1
+        for (int c = 0; c < TP_BN / 32; ++c) {
+            uint32_t r[32];
+            tmem_ld_32x32b_x32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c * 32), r);
+            float4* o4 = (float4*)(out + c * 32);
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                o4[q] = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
+                                    __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
+        }
+    } else if (nkb == 0) {
+        for (int c = 0; c < TP_BN; ++c) out[c] = 0.0f;
+    }
+    if (s_fail && threadIdx.x == 0) atomicExch(err, 1);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_sync();                // neither CTA's memory is in use by the other any more
+    if (warp == 0) {
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TP_BN) : "memory");
+    }
+}
+
 // egm[t][e] = sum_z part[z][t][e] (split order, FP64), t < T, e < n_e.
 __global__ void tc_reduce_kernel(int64_t T, int64_t n_e, int64_t T_pad, int64_t part_cols, int splits,
                                  const float* __restrict__ part, float* __restrict__ egm) {
@@ -400,17 +566,23 @@ struct TcConfig {
     int bn, bk, stages;
     const void* fn;
     size_t smem;
+    int box_b;      // rows of M a CTA loads
+    bool pair;      // two CTAs along t per tile
 };
 template <int BN, int BK, int ST>
 constexpr TcConfig tc_config() {
-    return TcConfig{BN, BK, ST, (const void*)egm_bf16x3_kernel<BN, BK, ST>, TcShape<BN, BK, ST>::SMEM};
+    return TcConfig{BN, BK, ST, (const void*)egm_bf16x3_kernel<BN, BK, ST>, TcShape<BN, BK, ST>::SMEM, BN, false};
 }
 const TcConfig kTcConfigs[] = {tc_config<128, 64, 3>(), tc_config<256, 64, 2>(), tc_config<256, 32, 4>(),
-                               tc_config<128, 32, 6>()};
+                               TcConfig{TP_BN, TP_BK, TP_STAGES, (const void*)egm_bf16x3_pair_kernel, TP_SMEM, TP_BN / 2, true}};
 constexpr int kTcNumConfigs = 4;
-// 128 x 256 tiles, 2 stages of BK 64: the fastest at 1000 x 519,533 x 2048
-// (5.09 ms against 5.78 ms for 128 x 128; the BK-32 rings took 8.7 and 10.7 ms).
-constexpr int kTcDefaultConfig = 1;
+constexpr int kTcSingle = 1, kTcPair = 3;
+// The configuration a launch uses: by default pairs of CTAs where T_pad holds a
+// whole number of them, else the 128 x 256 form (also when a pair is asked for).
+int tc_choice(int config, int64_t T_pad) {
+    if (config < 0) config = kTcPair;
+    return (config == kTcPair && (T_pad / TC_BM) % 2 != 0) ? kTcSingle : config;
+}
 
 // Columns of the split-K partial tiles: n_e_pad rounded up to the tile width.
 int64_t partial_cols(int64_t E_pad, int bn) { return (E_pad + bn - 1) / bn * bn; }
@@ -467,8 +639,8 @@ int split_bf16(int64_t rows, int64_t cols, const void* src, int64_t ld, bool src
 int contract_bf16x3(int64_t T, int64_t n_e, int64_t T_pad, int64_t E_pad, int64_t K_pad, const uint16_t* Vhi,
                     const uint16_t* Vlo, const uint16_t* Mhi, const uint16_t* Mlo, float* egm, void* work,
                     cudaStream_t stream, int config) {
-    if (config < 0) config = kTcDefaultConfig;
     if (config >= kTcNumConfigs) return PHS_ERR_BAD_ARG;
+    config = tc_choice(config, T_pad);
     const TcConfig& c = kTcConfigs[config];
     if (T <= 0 || n_e <= 0 || T > T_pad || n_e > E_pad || T_pad % TC_BM || E_pad % 128 || K_pad % 64 ||
         K_pad <= 0 || !Vhi || !Vlo || !Mhi || !Mlo || !egm || !work)
@@ -479,7 +651,7 @@ int contract_bf16x3(int64_t T, int64_t n_e, int64_t T_pad, int64_t E_pad, int64_
     if (((uintptr_t)Vhi | (uintptr_t)Vlo | (uintptr_t)Mhi | (uintptr_t)Mlo) & 15) return PHS_ERR_BAD_ARG;
     CUtensorMap mv_hi, mv_lo, mm_hi, mm_lo;
     if (!make_map(&mv_hi, Vhi, T_pad, K_pad, TC_BM, c.bk) || !make_map(&mv_lo, Vlo, T_pad, K_pad, TC_BM, c.bk) ||
-        !make_map(&mm_hi, Mhi, E_pad, K_pad, c.bn, c.bk) || !make_map(&mm_lo, Mlo, E_pad, K_pad, c.bn, c.bk))
+        !make_map(&mm_hi, Mhi, E_pad, K_pad, c.box_b, c.bk) || !make_map(&mm_lo, Mlo, E_pad, K_pad, c.box_b, c.bk))
         return PHS_ERR_CUDA;
     int splits = 1, per = 1;
     splits_for(c, T_pad, E_pad, K_pad, &splits, &per);

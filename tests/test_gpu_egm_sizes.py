@@ -108,3 +108,33 @@ def test_normalise(T, n_e, is64, cuda_device):
         return
     # one product per value and a mean of n_e: a few eps of the type
     assert bool(((egm.double() - want).abs() <= (1e-14 if is64 else 3e-7) * want.abs()).all())
+
+
+# pairs of CTAs (configuration 3) against single ones (1): the same products in
+# the same order; T_pad an odd number of 128-row tiles falls back to single ones,
+# n_e_pad 128 leaves half of a pair's columns empty, K_pad 64 is one stage
+@pytest.mark.parametrize("T,E,K", [(200, 40, 64), (256, 256, 192), (100, 300, 1000), (500, 130, 9000),
+                                   (1000, 600, 20000)])
+def test_contraction_by_pairs_equals_single(T, E, K, cuda_device):
+    import torch
+    L = _lib.lib()
+    up = lambda x, m: -(-x // m) * m
+    Tp, Ep, Kp = up(T, 128), up(E, 128), up(K, 64)
+    g = torch.Generator(device=cuda_device).manual_seed(T + E + K)
+    pad = lambda r, c, rp: torch.nn.functional.pad(
+        torch.randn((r, c), device=cuda_device, generator=g), (0, Kp - c, 0, rp - r)).bfloat16()
+    vh, vl, mh, ml = pad(T, K, Tp), pad(T, K, Tp) * 2 ** -8, pad(E, K, Ep), pad(E, K, Ep) * 2 ** -8
+    work = torch.empty(L.phs_egm_bf16x3_workspace(Tp, Ep, Kp), dtype=torch.uint8, device=cuda_device)
+    out = []
+    for cfg in (1, 3):
+        o = torch.full((T, E), float("nan"), device=cuda_device)
+        _lib.check(L.phs_egm_contract_bf16x3_cfg(T, E, Tp, Ep, Kp, _p(vh), _p(vl), _p(mh), _p(ml), _p(o), _p(work), cfg,
+                                                 None), "phs_egm_contract_bf16x3_cfg")
+        _lib.check(L.phs_egm_bf16x3_status(_p(work), None), "phs_egm_bf16x3_status")
+        out.append(o)
+    d = lambda t: t[:, :K].double()
+    want = d(vh)[:T] @ d(mh)[:E].T + d(vh)[:T] @ d(ml)[:E].T + d(vl)[:T] @ d(mh)[:E].T
+    # FP32 accumulation of 3 K products of sizes around 1: K eps of their magnitude
+    bound = 3 * K * 6e-8 * (d(vh)[:T].abs() @ d(mh)[:E].abs().T)
+    assert bool(((out[0].double() - want).abs() <= bound).all())
+    assert torch.equal(out[0], out[1])
