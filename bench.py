@@ -32,12 +32,12 @@ sys.path.insert(0, ROOT)
 METRIC = "voxel-steps/s batched FP32 vs plain FP64 on 1 B200 at LAT err<=dt; p99 latency"
 DEFAULT_F32_VARIANT = 7        # the engine's FP32 default when the autotuner is off
 # DRAM bytes per voxel-step of step_kernel measured by ncu (dram__bytes_read.sum +
-# dram__bytes_write.sum of the two timed full-size launches of this batch, 2.71
-# Arnoldi steps per step, profiles/step_kernel_64shells_dram_fullsize.md), for
+# dram__bytes_write.sum of two full-size launches of a 64-shell batch, 2.98
+# columns per step, profiles/step_kernel_64shells_dram_fullsize.md), for
 # the variants that read the int32 neighbour table and those that read the
 # compact one; multiplied by the voxels and steps of one launch below.
-STEP_TRAFFIC_BYTES_PER_VOXEL_STEP = {"int32": 267.0, "compact": 201.0}
-STEP_TRAFFIC_ARNOLDI_PER_STEP = 2.71
+STEP_TRAFFIC_BYTES_PER_VOXEL_STEP = {"int32": 210.4, "compact": 144.8}
+STEP_TRAFFIC_ARNOLDI_PER_STEP = 2.98
 BALANCE_LAUNCHES = 10   # launches per team-balancing round in the pre-steps
 WORKLOAD = "64 shells, 50k-400k voxels log-uniform, scar 0-30%, focal pacing, MS+AP, FP32 state / FP64 dots"
 
@@ -287,13 +287,12 @@ def run_b200(args):
     k_sq = np.array([b["arnoldi_sq"] - a["arnoldi_sq"] for a, b in zip(info0, info1)], dtype=np.float64)
     solves = np.array([b["solves"] - a["solves"] for a, b in zip(info0, info1)], dtype=np.float64)
     iso = [x.cw is not None for x in insts]
-    gs = [bool(x.guess) for x in insts]
     # neighbour-table bytes per row: the compact table where the variant reads it
     from pyheartsim_b200.engine import step_variant_layout
     reads_compact = step_variant_layout(_lib.PREC_F32)[step_variant_of(tune)][1]
     nbb = [roofline.COMPACT_NB if (reads_compact and eng.table_bytes(s) == 8) else 24 for s in slots]
-    alg_bytes = float(sum(roofline.algorithmic_bytes(4, int(n), K, ks, kq, sv, io, g, nb=nb)
-                          for n, ks, kq, sv, io, g, nb in zip(ns, k_sum, k_sq, solves, iso, gs, nbb)))
+    alg_bytes = float(sum(roofline.chebyshev_bytes(4, int(n), K, ks, kq, io, nb=nb)
+                          for n, ks, kq, io, nb in zip(ns, k_sum, k_sq, iso, nbb)))
     local_vs = float(ns.sum()) * K
     total_vs = local_vs * world
     value = total_vs / (ms_max / 1e3)
@@ -528,8 +527,8 @@ def dropin_c1_leg(dev):
 def plain_leg(args, cases, fast_value, dev):
     """Plain FP64 drop-in semantics (full GMRES(50) cycles, FP64) on the median
     instance of the batch, one instance on the whole GPU: throughput, the byte
-    model's roofline (k = m = 50 Arnoldi steps per cycle, one true-residual test
-    per cycle) and the device phase times."""
+    model's roofline (one true-residual test per solve) and the device phase
+    times."""
     import torch
     from pyheartsim_b200 import _lib, roofline, workloads
     from pyheartsim_b200.engine import BatchedEngine
@@ -555,8 +554,8 @@ def plain_leg(args, cases, fast_value, dev):
     info = eng.info(slot)
     k_sum = info["arnoldi_steps"] - info0["arnoldi_steps"]
     k_sq = info["arnoldi_sq"] - info0["arnoldi_sq"]
-    cycles = k_sum / 50.0
-    alg = roofline.algorithmic_bytes(8, meta["n"], steps, k_sum, k_sq, iso=inst.cw is not None, checks=cycles)
+    solves = info["solves"] - info0["solves"]     # a true-residual test ends each
+    alg = roofline.chebyshev_bytes(8, meta["n"], steps, k_sum, k_sq, iso=inst.cw is not None, checks=solves)
     # device phase times over 4 more steps
     eng.set_profile(True)
     eng.advance(4, stream=stream, sync=True)
@@ -574,7 +573,7 @@ def plain_leg(args, cases, fast_value, dev):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
                          "frac": achieved / pk["hbm_gbs"], "peak_source": pk_src,
                          "bytes_per_voxel_step": alg / (meta["n"] * steps),
-                         "note": "the 51-column FP64 Krylov basis of this instance fits in L2"},
+                         "note": "the FP64 Krylov columns of this instance fit in L2"},
             "phases_ms_per_step": {**{k: round(v_ / st, 4) for k, v_ in prof.items()},
                                    "barriers_per_step": round(nbar / st, 2)},
             "speedup_batched_fp32": (fast_value / v) if fast_value else None}
@@ -675,8 +674,8 @@ def aniso_leg(args, dev, tune=None, count=16):
     k_sum = np.array([b["arnoldi_steps"] - a["arnoldi_steps"] for a, b in zip(info0, info1)], dtype=np.float64)
     k_sq = np.array([b["arnoldi_sq"] - a["arnoldi_sq"] for a, b in zip(info0, info1)], dtype=np.float64)
     solves = np.array([b["solves"] - a["solves"] for a, b in zip(info0, info1)], dtype=np.float64)
-    alg = float(sum(roofline.algorithmic_bytes(4, int(n), K, ks, kq, sv, x.cw is not None, bool(x.guess), edge=True)
-                    for n, ks, kq, sv, x in zip(ns, k_sum, k_sq, solves, insts)))
+    alg = float(sum(roofline.chebyshev_bytes(4, int(n), K, ks, kq, x.cw is not None, edge=True, nb=roofline.COMPACT_NB)
+                    for n, ks, kq, x in zip(ns, k_sum, k_sq, insts)))
     pk, pk_src = peaks()
     achieved = alg / (ms / 1e3) / 1e9
     return {"value": float(ns.sum()) * K / (ms / 1e3), "unit": "voxel-steps/s", "instances": int(count),

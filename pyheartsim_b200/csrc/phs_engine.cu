@@ -10,21 +10,23 @@
 //               right-hand side b = u* + dt/2 L u*  (simulation/simulation_gpu.py:245)
 //               and the initial residual r0 = b - A x0  (A = I - dt/2 L, :321-322)
 //   GMRES       restarted GMRES on A (CuPy semantics of the reference's call at
-//               simulation/simulation_gpu.py:253): classical Gram-Schmidt, the
-//               Hessenberg least-squares solved by Givens rotations on device,
-//               FP64 dot products and norms whatever the storage type
+//               simulation/simulation_gpu.py:253): one pass and one barrier per
+//               column in a Chebyshev basis, or Arnoldi with classical
+//               Gram-Schmidt for stiff steps; FP64 dot products and norms
+//               whatever the storage type
 //   update      x += V y, then either the true-residual test of the next cycle
-//               (full_cycles = 1, CuPy semantics) or the Givens estimate
+//               (full_cycles = 1, CuPy semantics) or the residual estimate
 //               (full_cycles = 0, early exit)
 //
 // The Laplacian is applied matrix-free from a compacted table of six neighbour
 // indices and six premultiplied coefficients per voxel, which is the CSR matrix
 // of simulation/simulation_gpu.py:138-225 without the explicit zeros.
 //
-// Reductions are deterministic: every tile of kThreads*VPT voxels writes its
-// own FP64 partials and the last CTA of the team to arrive at the barrier sums
-// the tiles in index order.  The result therefore does not depend on the team
-// size, so an instance gives bit-identical results alone and in a batch.
+// Reductions are deterministic: every group of consecutive tiles of
+// kThreads*VPT voxels has its own FP64 partials, and every CTA of the team sums
+// the groups after the barrier in an order of their number alone.  The result
+// therefore does not depend on the team size, so an instance gives
+// bit-identical results alone and in a batch.
 #include <cuda_runtime.h>
 #include <cuda/atomic>
 #include <climits>

@@ -1,5 +1,9 @@
 """Algorithmic DRAM bytes of the step kernel, per voxel-step.
 
+The kernel's solves use a Chebyshev Krylov basis (one pass per column,
+:func:`chebyshev_bytes`); the model of its Arnoldi form, which stiff steps keep,
+follows.
+
 Counts every array the kernel must stream once per phase; s = bytes per stored
 value (4 FP32, 8 FP64), cb = coefficient bytes per row (5 for isotropic rows:
 one value + a presence byte; 6 s otherwise).  Neighbour values read by the
@@ -69,3 +73,19 @@ def algorithmic_bytes(s, voxels, steps, k_sum, k_sq_sum, solves=None, iso=True, 
 
 def per_voxel_step(s, k, iso=True, nb=24):
     return algorithmic_bytes(s, 1, 1, k, k * k, iso=iso, nb=nb)
+
+
+def chebyshev_bytes(s, voxels, steps, k_sum, k_sq_sum, iso=True, edge=False, checks=0, nb=24):
+    """Bytes of ``steps`` steps whose solves took ``k_sum`` columns in total in
+    the Chebyshev basis.  Per voxel, with r the bytes of a row (neighbours,
+    coefficients, edge pairs):
+
+      right-hand side  read the pair (u*, increment), the row; write K_0  = 3 s + r
+      column j         read K_0..K_j, the row; write K_{j+1}              = (j + 2) s + r
+      update           read the pair, K_0..K_{k-1}, h, flags; write u, the
+                       pair and h (the next step's reaction is in it)     = (k + 7) s + 1
+
+    and for each true-residual test of a full cycle (``checks``) x and b written
+    and read, the row, K_0 and u written: 6 s + r."""
+    r = nb + coef_bytes(s, iso) + (edge_bytes(s) if edge else 0)
+    return voxels * (steps * (10 * s + r + 1) + k_sum * (r + 3 * s) + s * (k_sq_sum - k_sum) / 2 + checks * (6 * s + r))
