@@ -59,9 +59,18 @@ void set_threshold(DevicePool& d) {
     cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
 }
 
+// While it lives, this thread's calls neither fail for nor disturb a stream
+// capture that another thread has under way.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // The current device's pool, made on first use; nullptr when there is none to
 // be had (the default pool serves then).  g_pool_mu held.
 DevicePool* current_pool() {
+    RelaxedCapture relaxed;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
     if (cudaFree(nullptr) != cudaSuccess) return nullptr;   // the context exists from here on
@@ -73,13 +82,8 @@ DevicePool* current_pool() {
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
-    // making a pool must not disturb a capture another thread has under way
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
     cudaMemPool_t pool = nullptr;
-    const cudaError_t e = cudaMemPoolCreate(&pool, &props);
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    if (e != cudaSuccess) {
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }

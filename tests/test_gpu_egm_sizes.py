@@ -138,3 +138,39 @@ def test_contraction_by_pairs_equals_single(T, E, K, cuda_device):
     bound = 3 * K * 6e-8 * (d(vh)[:T].abs() @ d(mh)[:E].abs().T)
     assert bool(((out[0].double() - want).abs() <= bound).all())
     assert torch.equal(out[0], out[1])
+
+
+def test_contractions_and_normalisation_under_capture(cuda_device):
+    """Captured in a graph after a first call outside (as the allocation-free form
+    asks), replayed on new inputs; the workspaces of the others belong to the graph."""
+    import torch
+    L = _lib.lib()
+    T, n_e, n = 130, 70, 3001
+    g = torch.Generator(device=cuda_device).manual_seed(5)
+    V = torch.randn((T, n), dtype=torch.float64, device=cuda_device, generator=g)
+    Mt = torch.randn((n_e, n), dtype=torch.float64, device=cuda_device, generator=g)
+    a, b = (torch.empty((T, n_e), dtype=torch.float64, device=cuda_device) for _ in range(2))
+
+    def call():
+        s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        _lib.check(L.phs_egm_contract_f64(T, n, n_e, _p(V), n, _p(Mt), _p(a), s), "phs_egm_contract_f64")
+        _lib.check(L.phs_egm_contract_f64_noalloc(T, n, n_e, _p(V), n, _p(Mt), _p(b), s), "noalloc")
+        _lib.check(L.phs_egm_normalize(T, n_e, _p(a), 1, s), "phs_egm_normalize")
+        _lib.check(L.phs_egm_normalize(T, n_e, _p(b), 1, s), "phs_egm_normalize")
+
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call()
+    V.copy_(torch.randn((T, n), dtype=torch.float64, device=cuda_device, generator=g))
+    graph.replay()
+    torch.cuda.synchronize()
+    got = a.clone(), b.clone()
+    call()
+    torch.cuda.synchronize()
+    assert torch.equal(got[0], a) and torch.equal(got[1], b)
+    want = V @ Mt.T
+    want = want / (want.max(0).values - want.min(0).values).mean()
+    # n products a value, normalised: far within 1e-11 of values around 1
+    assert float((a - want).abs().max()) < 1e-11 and float((b - want).abs().max()) < 1e-11
