@@ -190,7 +190,7 @@ int phs_step_variant_vpt(int precision, int32_t count, int32_t* vpt);
 int phs_step_variant_layout(int precision, int32_t count, int32_t* ring_bytes, int32_t* compact_table);
 /* Re-split the CTAs over the instances in proportion to their cost since the
  * last rebalance: the measured team time per step x team CTAs when the phase
- * timers (PHS_CFG_PROFILE) are on, else voxels x (1.6 + Arnoldi iterations per
+ * timers (PHS_CFG_PROFILE) are on, else voxels x (2.3 + Arnoldi iterations per
  * step).  Synchronises the device; the next advance() rebuilds its plan.        */
 int phs_engine_rebalance(phs_engine* eng);
 /* Phase timers of an instance (PHS_CFG_PROFILE on): 16 counters, nanoseconds

@@ -616,11 +616,12 @@ __device__ __forceinline__ double warp_sums(double (&v)[N], int lane) {
 }
 __host__ __device__ constexpr int log2_of(int n) { return n <= 1 ? 0 : 1 + log2_of(n / 2); }
 
-// Basis vectors whose loads are issued together: FP32 tiles hold two or four
-// voxels per thread (as many loads per vector), FP64 tiles one, and the FP64
-// plain form passes over some twenty vectors per column.
+// Basis vectors whose loads and sums are taken together: FP32 tiles hold two or
+// four voxels per thread (as many loads per vector), FP64 tiles one, and the FP64
+// plain form passes over some twenty vectors per column (160k voxels, 30 steps:
+// 9.9 ms by eights, 10.7 by sixteens with their spills, 10.2 by fours).
 template <typename T>
-constexpr int kChunkOf = sizeof(T) == 8 ? 16 : 4;
+constexpr int kChunkOf = sizeof(T) == 8 ? 8 : 4;
 // A full GMRES cycle ends early once its residual estimate is at most this
 // fraction of ||b||: half a unit roundoff of the stored type.  A is I - dt/2 L
 // with eigenvalues of 1 and above, so what the remaining columns could add to x
@@ -1959,7 +1960,7 @@ struct InstHost {
     InstState* st = nullptr;
     unsigned long long* prof = nullptr;
     InstState st_host{};
-    double kavg = 4.0;           // recent Arnoldi steps per step (cost model)
+    double kavg = 4.0;           // recent columns per step (cost model)
     long long ref_arnoldi = 0;   // counters at the last rebalance
     long long ref_step = 0;
     double weight = 0.0;         // measured CTA-time per step (0: use the model)
@@ -2403,6 +2404,11 @@ int add_instance(phs_engine* e, const phs_instance_desc* d, int* slot) {
         if (dev_alloc((void**)&h.prof, kProfSlots * sizeof(unsigned long long), 0) == cudaSuccess)
             cudaMemset(h.prof, 0, kProfSlots * sizeof(unsigned long long));
     }
+    // columns per step until they are known (cost model of the first launch): the
+    // batches' Mitchell-Schaeffer shells (hg 0.94) take 4.7, the Aliev-Panfilov
+    // ones (hg 0.6) 1.8
+    const double hg = std::min(1.0, 0.25 * d->dt * h.bound);
+    h.kavg = d->full_cycles ? 10.0 + 15.0 * hg : 1.0 + 4.4 * hg * hg * hg;
     e->inst[s] = h;
     pool_update(0);
     e->dirty = true;
@@ -2497,12 +2503,16 @@ InstDev<T> make_dev(const InstHost& h, int vpt, bool compact_nb) {
 // time proportional to (cost per tile) x ceil(tiles / P): its CTAs walk their
 // tiles one after another and the one with the most tiles sets the pace.  The
 // cost of an instance is `weight` (voxels times the cost of a step in units of
-// one Arnoldi iteration, or the measured CTA-time per step), per tile weight /
+// one column, or the measured CTA-time per step), per tile weight /
 // tiles.  Starting from one CTA each, the instance with the longest time
 // receives the fewest CTAs that lower its tiles-per-CTA count, until the CTAs
 // run out or the longest one cannot be helped; CTAs left over (when every team
 // already has one CTA per tile, or the longest would need more than remain) go
 // to no one.  Never more CTAs than tiles.
+// A step costs as much as this many columns beside its columns (right-hand side,
+// update, reaction: 12 against 5.3 CTA-ns per voxel in a batch of 24 shells, for
+// both models).
+constexpr double kStepCost = 2.3;
 std::vector<int> team_sizes(const std::vector<int>& tiles, const std::vector<double>& weight, int G) {
     const int A = (int)tiles.size();
     std::vector<int> P(A, 1);
@@ -2636,7 +2646,7 @@ int build_plan(phs_engine* e, int cps, bool edge) {
         for (size_t i = w0; i < w1; ++i) {
             const InstHost& h = e->inst[act[i]];
             tiles.push_back(groups_of<T>(tiles_of(h.n, vpt)));
-            weight.push_back(measured ? h.weight : (double)h.n * (1.6 + h.kavg));
+            weight.push_back(measured ? h.weight : (double)h.n * (kStepCost + h.kavg));
         }
         std::vector<int> P = team_sizes(tiles, weight, G);
         for (size_t i = w0; i < w1; ++i) e->inst[act[i]].team = P[i - w0];
