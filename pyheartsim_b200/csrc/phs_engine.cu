@@ -413,7 +413,7 @@ struct SharedCtl {
 // the partials, in the same order and so to the same bits.  That takes three
 // dependent L2 round trips out of a barrier (the leader's read of the partials,
 // its release and the waiters' read of its results): 5.3-7.5 us with a leader
-// that reduced, 3.0-4.2 us now, the reduction included (40 to 157 CTAs).
+// that reduced, 3.8-4.3 us now with sums and decision (7 to 157 CTAs).
 //
 // Ordering: the arrival is a release RMW after a CTA barrier (cumulative over
 // the CTA's writes), the poll an acquire load, followed by a CTA barrier.
@@ -671,8 +671,8 @@ constexpr double kPivot = 1e-12;
 //  ||z||^2.  The iterates, estimates and column counts are those of Arnoldi
 //  GMRES (FP32: solutions agree to 1e-8, estimates to 3 digits at tol 1e-7;
 //  FP64: to 1e-15), which needed two passes and two barriers per column, the
-//  second pass to orthogonalise.  200 x 200 sheet: FP32 70 -> 33 us per step of
-//  3 columns, FP64 460 -> 190 us per step of 21.
+//  second pass to orthogonalise.  200 x 200 sheet: FP32 70 -> 24 us per step of
+//  3 columns, FP64 460 -> 157 us per step of 22.
 //
 //  Arnoldi with classical Gram-Schmidt (the others: stiff steps with long
 //  cycles): phase A applies A and takes the dots, phase C orthogonalises.
