@@ -18,7 +18,8 @@ void set_last_error(const char* where, cudaError_t e);
 void set_last_message(const char* msg);
 
 // Device memory from the library's pool of the current device, ordered on
-// `stream` (phs_pool.cu); dev_free accepts null.
+// `stream` (phs_pool.cu); dev_free accepts null.  Memory allocated or filled on
+// one stream is used on another only after a synchronisation or an event wait.
 cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t stream);
 void dev_free(void* p, cudaStream_t stream);
 // Sets how much the pool keeps; `engines`: engines made (+1) or destroyed (-1).

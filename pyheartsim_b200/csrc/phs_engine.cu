@@ -2671,6 +2671,10 @@ int build_plan(phs_engine* e, int cps, bool edge) {
         e->d_map_n = map_all.size();
     }
     PHS_CUDA_TRY(cudaMemcpy(e->d_map, map_all.data(), map_all.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    // The launch may be on a stream that does not wait for the legacy one (any
+    // non-blocking stream), on which the two arrays were allocated and filled, and
+    // a copy from pageable memory may return before its transfer has landed.
+    PHS_CUDA_TRY(cudaStreamSynchronize(0));
     return PHS_OK;
 }
 
