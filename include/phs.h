@@ -87,7 +87,11 @@ typedef struct phs_instance_desc {
                                  there as on a breakdown); 0: Givens early exit             */
     double u0, h0;            /* initial state (MS: 0,1; AP: 0,0)                           */
     double tol, atol;         /* stop when ||r|| <= max(atol, tol*||b||)                    */
-    int32_t maxiter;          /* Arnoldi steps per solve before giving up (reference 10000) */
+    int32_t maxiter;          /* columns per solve before giving up, counted in whole cycles of
+                                 restart columns (reference 10000); an early-exit cycle that the
+                                 loss of its Gram matrix cut short is not counted, and once such
+                                 cycles add up to maxiter columns the solve goes on in Arnoldi
+                                 form                                                      */
     int32_t guess;            /* 0: start each solve from u* (the reference's x0); 1: from u*
                                  plus the previous step's diffusion increment (same stopping
                                  test, fewer iterations)                                    */

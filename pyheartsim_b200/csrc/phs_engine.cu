@@ -403,6 +403,7 @@ struct SharedCtl {
     int k;            // basis vectors of the update that follows
     int settled;      // the cycle's estimate is below rounding level (kSettled)
     double bnorm, atol_eff;
+    double rnorm;     // residual at the start of the cycle
     double sj;        // Arnoldi: scale of the column the next pass applies A to
     double sz;        // Chebyshev basis: sum of z_i^2
 };
@@ -792,7 +793,7 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
     const int gt = I.gt, n_groups = I.n_groups, n_tiles = I.n_tiles;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    const bool cheb = I.cheb != 0;
+    bool cheb = false;       // form of the cycle under way (I.cheb at the start of a solve)
     long long step = sh_step0;
     long long step_end = step + n_steps_launch;
     if (step_end > I.n_steps) step_end = I.n_steps;
@@ -978,7 +979,8 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
     const size_t ldV = (size_t)I.ldv;
 
     // ---- what every CTA decides from the sums of a barrier ------------------
-    int iters_solve = 0, iters_cap = 0, cols = 0;   // columns: of the solve, CuPy's count, of the cycle
+    // columns: of the solve, CuPy's count, of the cycle, of the early exit's short cycles
+    int iters_solve = 0, iters_cap = 0, cols = 0, iters_short = 0;
     bool refined = false;
     auto fail = [&]() {
         ctl.action = ACT_FAIL;
@@ -996,6 +998,7 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
     auto start_cycle = [&](double r2) {
         ctl.action = ACT_CYCLE;
         const double w0 = rsqrt(r2);
+        ctl.rnorm = r2 * w0;
         if (cheb) {
             tm[0] = w0;            // W
             va[0] = w0;            // z
@@ -1219,7 +1222,18 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
         const double rn = sqrt(gsum[0]);
         const bool more = cheb && I.full_cycles && left > 0 && rn > kRefine<T> * ctl.bnorm && !refined;
         if (more && ctl.settled) refined = true;
-        if (!more) iters_cap += I.m;
+        // early exit, the Gram matrix gave out: such a short cycle is not one of those
+        // that maxiter counts (m columns each), so the solve has as many whole cycles
+        // as Arnoldi's would, from a smaller residual.  The form stays while short
+        // cycles halve the residual and add up to less than maxiter columns (one pass
+        // per column: 64 x 64 sheet, plane front, half width 60, restart 20, tol 1e-5:
+        // 44 passes per solve, 67 with Arnoldi from the first short cycle on)
+        const bool cut = cheb && !I.full_cycles && left > 0;
+        if (cut) {
+            iters_short += cols;
+            if (iters_short >= I.maxiter || rn > 0.5 * ctl.rnorm) cheb = false;
+        }
+        if (!more && !cut) iters_cap += I.m;
         bool over = false;
         csync<ST>();
         if (threadIdx.x == 0) {
@@ -1359,8 +1373,10 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
         if (!barrier_sums(2)) { aborted = true; break; }
         iters_solve = 0;
         iters_cap = 0;
+        iters_short = 0;
         cols = 0;
         refined = false;
+        cheb = I.cheb != 0;
         decide_rhs();
         int act = ctl.action;
         mark(PF_RHS_WAIT);
@@ -2419,11 +2435,14 @@ int add_instance(phs_engine* e, const phs_instance_desc* d, int* slot) {
 }
 
 // Which solves use the Chebyshev basis.  hg: the half width of the interval
-// of A - I.  Its Gram matrix stays positive definite in FP64 for about 25
-// columns on the stiff side (hg 3 and 15: lost at column 22-30) and longer
-// than a solve needs where it converges by 4 and more per column.  Early exit:
-// restarts of up to 20 columns stay clear of that at any hg (hg 15, 20 columns:
-// estimate within 0.5 % of Arnoldi's).  Full cycles want rounding level: up to
+// of A - I.  Its Gram matrix stays positive definite in FP64 longer than a solve
+// needs where it converges by 4 and more per column; on the stiff side it is lost
+// after 22-30 columns (hg 3 and 15, discs and rough residuals) or, for plane
+// fronts, after 10-17 (FP32 from hg 5, FP64 from hg 3 on at tol 1e-9).  Early
+// exit: with restarts of up to 20 columns a lost matrix costs little, the cycle
+// ends in a true residual and the solve goes on (64 x 64 sheet, plane front,
+// columns against Arnoldi's: none more at hg 3, 5 % at hg 5, 28 % at hg 15, 18 % at
+// hg 60, at half the passes per column).  Full cycles want rounding level: up to
 // hg 1.25 (Mitchell-Schaeffer at 0.05 ms and 0.4 mm: 0.94) that takes 21-28
 // columns; beyond, Arnoldi.
 bool cheb_rule(bool full_cycles, int m, double hg) {
