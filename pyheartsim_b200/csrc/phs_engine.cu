@@ -404,6 +404,10 @@ struct SharedCtl {
     int settled;      // the cycle's estimate is below rounding level (kSettled)
     double bnorm, atol_eff;
     double rnorm;     // residual at the start of the cycle
+    int cheb;         // form of the solve's cycles from here on: Chebyshev basis, else Arnoldi
+    int iters_cap;    // columns of the solve as maxiter counts them
+    int iters_short;  // columns of the early exit's short cycles, which it does not
+    int refined;      // the columns after a settled full cycle have run
     double sj;        // Arnoldi: scale of the column the next pass applies A to
     double sz;        // Chebyshev basis: sum of z_i^2
 };
@@ -793,7 +797,7 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
     const int gt = I.gt, n_groups = I.n_groups, n_tiles = I.n_tiles;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    bool cheb = false;       // form of the cycle under way (I.cheb at the start of a solve)
+    const bool cheb = I.cheb != 0;
     long long step = sh_step0;
     long long step_end = step + n_steps_launch;
     if (step_end > I.n_steps) step_end = I.n_steps;
@@ -979,9 +983,7 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
     const size_t ldV = (size_t)I.ldv;
 
     // ---- what every CTA decides from the sums of a barrier ------------------
-    // columns: of the solve, CuPy's count, of the cycle, of the early exit's short cycles
-    int iters_solve = 0, iters_cap = 0, cols = 0, iters_short = 0;
-    bool refined = false;
+    int iters_solve = 0, cols = 0;   // columns of the solve, of the cycle
     auto fail = [&]() {
         ctl.action = ACT_FAIL;
         if (rank == 0) I.st->status = PHS_ERR_NONFINITE;
@@ -999,7 +1001,7 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
         ctl.action = ACT_CYCLE;
         const double w0 = rsqrt(r2);
         ctl.rnorm = r2 * w0;
-        if (cheb) {
+        if (cheb && ctl.cheb) {
             tm[0] = w0;            // W
             va[0] = w0;            // z
             vb[0] = 1.0;           // t
@@ -1012,6 +1014,8 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
     };
     auto decide_rhs = [&]() {
         if (threadIdx.x == 0) {
+            ctl.cheb = cheb;
+            ctl.iters_cap = ctl.iters_short = ctl.refined = 0;
             const double bn = sqrt(gsum[0]), rn = sqrt(gsum[1]);
             const double atol_eff = fmax(I.atol, I.tol * bn);
             ctl.bnorm = bn;
@@ -1219,47 +1223,43 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
         // columns the logical cycle of I.m still has: when its Gram matrix gave out
         // early, or once more when it ended settled (kRefine)
         const int left = I.m - cols;
+        const bool basis = cheb && ctl.cheb;
         const double rn = sqrt(gsum[0]);
-        const bool more = cheb && I.full_cycles && left > 0 && rn > kRefine<T> * ctl.bnorm && !refined;
-        if (more && ctl.settled) refined = true;
-        // early exit, the Gram matrix gave out: such a short cycle is not one of those
-        // that maxiter counts (m columns each), so the solve has as many whole cycles
-        // as Arnoldi's would, from a smaller residual.  The form stays while short
-        // cycles halve the residual and add up to less than maxiter columns (one pass
-        // per column: 64 x 64 sheet, plane front, half width 60, restart 20, tol 1e-5:
-        // 44 passes per solve, 67 with Arnoldi from the first short cycle on)
-        const bool cut = cheb && !I.full_cycles && left > 0;
-        if (cut) {
-            iters_short += cols;
-            if (iters_short >= I.maxiter || rn > 0.5 * ctl.rnorm) cheb = false;
-        }
-        if (!more && !cut) iters_cap += I.m;
-        bool over = false;
+        const bool more = basis && I.full_cycles && left > 0 && rn > kRefine<T> * ctl.bnorm && !ctl.refined;
         csync<ST>();
         if (threadIdx.x == 0) {
+            // early exit, the Gram matrix gave out: such a short cycle is not one of those
+            // that maxiter counts (m columns each), so the solve has as many whole cycles
+            // as Arnoldi's would, from a smaller residual.  The form stays while short
+            // cycles halve the residual and add up to less than maxiter columns (one pass
+            // per column: 64 x 64 sheet, plane front, half width 60, restart 20, tol 1e-5:
+            // 44 passes per solve, 67 with Arnoldi from the first short cycle on)
+            if (more) {
+                if (ctl.settled) ctl.refined = 1;
+            } else if (basis && !I.full_cycles && left > 0) {
+                ctl.iters_short += cols;
+                if (ctl.iters_short >= I.maxiter || rn > 0.5 * ctl.rnorm) ctl.cheb = 0;
+            } else {
+                ctl.iters_cap += I.m;
+                ctl.refined = 0;
+            }
             if (!isfinite(rn)) {
                 fail();
             } else if (more) {
                 start_cycle(gsum[0]);
             } else if (rn <= ctl.atol_eff) {
                 ctl.action = ACT_DONE;
-            } else if (iters_cap >= I.maxiter) {
+            } else if (ctl.iters_cap >= I.maxiter) {
                 ctl.action = ACT_DONE;
-                over = true;
+                st_nonconv += 1;
+                if (rank == 0 && I.st->status == PHS_OK) I.st->status = PHS_WARN_NO_CONVERGE;
             } else {
                 start_cycle(gsum[0]);
             }
         }
         decided();
-        if (!more) {
-            cols = 0;
-            refined = false;
-        }
+        if (!more) cols = 0;
         if (ctl.action == ACT_DONE) account_solve();
-        if (over) {
-            st_nonconv += 1;
-            if (rank == 0 && I.st->status == PHS_OK) I.st->status = PHS_WARN_NO_CONVERGE;
-        }
     };
 
     // ---- sample / activation bookkeeping of the state in u (after step s-1)
@@ -1372,11 +1372,7 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
         mark(PF_RHS);
         if (!barrier_sums(2)) { aborted = true; break; }
         iters_solve = 0;
-        iters_cap = 0;
-        iters_short = 0;
         cols = 0;
-        refined = false;
-        cheb = I.cheb != 0;
         decide_rhs();
         int act = ctl.action;
         mark(PF_RHS_WAIT);
@@ -1392,7 +1388,7 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
         if (act == ACT_CYCLE) {
             bool first_cycle = true;
             for (;;) {
-                if (cheb) {
+                if (cheb && ctl.cheb) {
                     const int cycle_cols = I.m - cols;
                     for (int j = 0;; ++j) {
                         // ======== column j: K_{j+1} = 2/delta (A - theta) K_j - K_{j-1}, dots
@@ -1494,25 +1490,27 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
                                 for (int v = 0; v < VPT; ++v) own[v] = Vj[n0 + v * kThreads];
                                 tile_lap<T, VPT, EDGE, NB>(I, Vj, n0, tb, own, lap);
 #pragma unroll
-                                for (int v = 0; v < VPT; ++v) {
-                                    wr[v] = sj * (own[v] - I.half_dt * lap[v]);
-                                    Vn[n0 + v * kThreads] = wr[v];
-                                }
+                                for (int v = 0; v < VPT; ++v) wr[v] = sj * (own[v] - I.half_dt * lap[v]);
                                 for (int i0 = 0; i0 <= j; i0 += kChunk) {
+                                    T vv[kChunk][VPT];
                                     double s[kChunk];
+#pragma unroll
+                                    for (int e = 0; e < kChunk; ++e)
+#pragma unroll
+                                        for (int v = 0; v < VPT; ++v)
+                                            vv[e][v] = (i0 + e <= j) ? Vb[(size_t)(i0 + e) * ldV + n0 + v * kThreads] : T(0);
 #pragma unroll
                                     for (int e = 0; e < kChunk; ++e) {
                                         s[e] = 0.0;
 #pragma unroll
-                                        for (int v = 0; v < VPT; ++v)
-                                            if (i0 + e <= j)
-                                                s[e] += (double)Vb[(size_t)(i0 + e) * ldV + n0 + v * kThreads] *
-                                                        (double)wr[v];
+                                        for (int v = 0; v < VPT; ++v) s[e] += (double)vv[e][v] * (double)wr[v];
                                     }
                                     const double w = warp_sums<kChunk>(s, lane);
                                     const int i = i0 + (lane >> (5 - log2_of(kChunk)));
                                     if ((lane & (32 / kChunk - 1)) == 0 && i <= j) put(ns, i, w, first);
                                 }
+#pragma unroll
+                                for (int v = 0; v < VPT; ++v) Vn[n0 + v * kThreads] = wr[v];
                             }
                             group_done(ns);
                         }
@@ -1528,12 +1526,19 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
                                 double acc[VPT], s[1] = {0.0};
 #pragma unroll
                                 for (int v = 0; v < VPT; ++v) acc[v] = (double)Vn[n0 + v * kThreads];
-#pragma unroll 4
-                                for (int i = 0; i <= j; ++i) {
-                                    const double cf = shc[i];
+                                for (int i0 = 0; i0 <= j; i0 += kChunk) {
+                                    T vv[kChunk][VPT];
 #pragma unroll
-                                    for (int v = 0; v < VPT; ++v)
-                                        acc[v] -= cf * (double)Vb[(size_t)i * ldV + n0 + v * kThreads];
+                                    for (int e = 0; e < kChunk; ++e)
+#pragma unroll
+                                        for (int v = 0; v < VPT; ++v)
+                                            vv[e][v] = (i0 + e <= j) ? Vb[(size_t)(i0 + e) * ldV + n0 + v * kThreads] : T(0);
+#pragma unroll
+                                    for (int e = 0; e < kChunk; ++e) {
+                                        const double cf = (i0 + e <= j) ? shc[i0 + e] : 0.0;
+#pragma unroll
+                                        for (int v = 0; v < VPT; ++v) acc[v] -= cf * (double)vv[e][v];
+                                    }
                                 }
 #pragma unroll
                                 for (int v = 0; v < VPT; ++v) {
