@@ -657,6 +657,12 @@ constexpr int kRedDoubles = 16 * kSlots;      // warp sums a CTA holds back befo
 constexpr int kTri = (kMaxRestart + 1) * (kMaxRestart + 2) / 2;
 __device__ __forceinline__ int tri(int row) { return row * (row + 1) / 2; }
 
+// A solve whose squared residual norm is below this (||r|| < 1e-50: resting tissue
+// long after its last wave, solved to a tolerance without an absolute part) is
+// Arnoldi's, whose vectors are normalised: the Chebyshev form sums squares of
+// 1 / ||r||, which leave the range of FP64 as the estimate passes 1e-154.
+constexpr double kTinySquare = 1e-100;
+
 // Below this share of <K_j, K_j> the part of K_j outside the span of the
 // earlier vectors is zero (breakdown) or lost to rounding.
 constexpr double kPivot = 1e-12;
@@ -1014,7 +1020,7 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
     };
     auto decide_rhs = [&]() {
         if (threadIdx.x == 0) {
-            ctl.cheb = cheb;
+            ctl.cheb = cheb && !(gsum[1] < kTinySquare);
             ctl.iters_cap = ctl.iters_short = ctl.refined = 0;
             const double bn = sqrt(gsum[0]), rn = sqrt(gsum[1]);
             const double atol_eff = fmax(I.atol, I.tol * bn);
@@ -1243,6 +1249,7 @@ step_kernel(const InstDev<T>* __restrict__ insts, const int4* __restrict__ cta_m
                 ctl.iters_cap += I.m;
                 ctl.refined = 0;
             }
+            if (gsum[0] < kTinySquare) ctl.cheb = 0;
             if (!isfinite(rn)) {
                 fail();
             } else if (more) {
