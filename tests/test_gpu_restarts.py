@@ -3,9 +3,11 @@ restarted solves."""
 import numpy as np
 import pytest
 
+from oracle import simulation_fp64
 from pyheartsim_b200 import _lib, instance, synthetic
 from pyheartsim_b200.engine import BatchedEngine
 from pyheartsim_b200.simulation import simulation_gpu
+from tests import gpu_cases
 
 pytestmark = pytest.mark.gpu
 
@@ -68,3 +70,67 @@ def test_tiny_states_are_solved_like_small_ones(exponent, full, tol, cuda_device
     assert 0.0 < a.min() < 0.9 * a.max()                   # a field with something to solve
     # both residuals are at most tol ||b|| (full cycles: far below), |A^-1| <= 1; rounding 1e-14
     np.testing.assert_allclose(b, a, rtol=0, atol=max(1e-14, (0.0 if full else 2 * tol) * np.linalg.norm(a)))
+
+
+def _steps(case, dtype, restart, steps, *, full=False, variant=None, tol=1e-6, atol=1e-12):
+    """(u after ``steps`` steps, info) of one case in an engine of its own."""
+    (n, P, geom, sp, ap), pdur = case
+    inst = instance.compile_instance(n, P, geom, dict(sp), dict(ap), full_cycles=full, tol=tol, atol=atol, restart=restart,
+                                     pacing_duration=pdur, max_steps=steps)
+    with BatchedEngine(_lib.PREC_F32 if dtype == np.float32 else _lib.PREC_F64) as eng:
+        if variant is not None:
+            eng.configure(variant=variant)
+        s = eng.add(inst)
+        eng.advance(steps)
+        u, _, _ = eng.state(s)
+        return u.astype(np.float64), eng.info(s)
+
+
+_CASES = {"sheet": lambda: gpu_cases.sheet_ms(), "shell": lambda: gpu_cases.small_shell_ms(),
+          "fibres": lambda: gpu_cases.small_shell_ms_fibres()}
+
+
+# Early exit in several cycles: the update into x, the check that takes b from the
+# pairs, the next cycle from its residual.  Variants 5 and 6 (FP32) stage the update.
+@pytest.mark.parametrize("name", list(_CASES))
+@pytest.mark.parametrize("dtype,variant", [(np.float32, None), (np.float32, 0), (np.float32, 5), (np.float32, 6),
+                                           (np.float64, None)])
+@pytest.mark.parametrize("restart", [2, 3, 4])
+def test_restarted_early_exit(name, dtype, variant, restart, cuda_device):
+    case, steps, tol = _CASES[name](), 8, 1e-6
+    u, info = _steps(case, dtype, restart, steps, variant=variant, tol=tol)
+    uo, io = _steps(case, np.float64, 50, steps, full=True, tol=1e-13, atol=0.0)
+    assert info["max_arnoldi"] > restart and info["nonconverged"] == 0 and info["status"] == 0
+    assert io["nonconverged"] == 0
+    # a step is off by at most tol ||b|| (|A^-1| near 1), ||b|| <= sqrt(excited voxels);
+    # the upstroke amplifies an error by exp(0.05 / 0.3) a step at most (tau_in 0.3), the
+    # sum of 8 steps is below 16; FP32 rounding is 6e-8 a step
+    excited = np.count_nonzero(uo > 1e-3)
+    assert 0 < excited and uo.max() <= 1.0
+    eps = 6e-8 if dtype == np.float32 else 1e-16
+    np.testing.assert_allclose(u, uo, rtol=0, atol=16 * (tol * np.sqrt(excited) + eps))
+
+
+# One full-cycle step from rest, random voxels paced (r0 of the order of b, so the
+# cycle that ends at rounding level is followed by a few columns more), and one
+# whose cycles are too short to get there: the true residual of the result
+@pytest.mark.parametrize("name", list(_CASES))
+@pytest.mark.parametrize("restart", [50, 30, 8])
+def test_full_cycles_true_residual(name, restart, cuda_device):
+    (n, P, geom, sp, ap), _ = _CASES[name]()
+    s1 = np.flatnonzero(np.random.default_rng(3).random(n) < 0.3)
+    ap = dict(ap, s1_pacing_voxel_id=s1)
+    u, info = _steps(((n, P, geom, sp, ap), 1.0), np.float64, restart, 1, full=True, tol=1e-13, atol=0.0)
+    assert info["nonconverged"] == 0 and info["solves"] == 1
+    J = np.zeros(n)
+    J[s1] = 1.0
+    us, _ = simulation_fp64.rk4(0, np.zeros(n), np.ones(n), P, J, sp["dt"])
+    L = simulation_fp64.laplacian(P, geom["neighbor_id_2d"], geom["Delta"])
+    b = us + sp["dt"] / 2 * (L @ us)
+    r = b - (u - sp["dt"] / 2 * (L @ u))
+    r0 = b - (us - sp["dt"] / 2 * (L @ us))
+    assert np.linalg.norm(r0) > 0.1 * np.linalg.norm(b)
+    # restart 8 stops at tol; the others at the rounding of the residual itself (a row adds up
+    # to 20 terms of |A| |u|, below 4 |b|: 20 * 1.1e-16 * 4 would be the worst row, the norm over
+    # random signs is sqrt(20) of it) and of u* on the two sides
+    np.testing.assert_array_less(np.linalg.norm(r), (2e-15 if restart > 8 else 2e-13) * np.linalg.norm(b))
