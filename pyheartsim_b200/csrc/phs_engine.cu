@@ -628,9 +628,11 @@ __host__ __device__ constexpr int log2_of(int n) { return n <= 1 ? 0 : 1 + log2_
 template <typename T>
 constexpr int kChunkOf = sizeof(T) == 8 ? 8 : 4;
 // A full GMRES cycle ends early once its residual estimate is at most this
-// fraction of ||b||: half a unit roundoff of the stored type.  A is I - dt/2 L
-// with eigenvalues of 1 and above, so what the remaining columns could add to x
-// is below a rounding of x; besides, classical Gram-Schmidt has lost the basis'
+// fraction of ||b||: half a unit roundoff of the stored type.  With isotropic rows
+// A is I - dt/2 L with eigenvalues of 1 and above, so what the remaining columns
+// could add to x is below a rounding of x (anisotropic rows: unproven, but ||A^-1||
+// is near 1 there too, and the true-residual test follows either way); besides,
+// classical Gram-Schmidt has lost the basis'
 // orthogonality by then (|v_0 . v_j| of 0.1 to 1 where the estimate passes this
 // line) and those columns are rounding noise.  On the sheet and shell runs the
 // line is crossed after 18-26 of 50 columns with the error against the exact
@@ -672,8 +674,9 @@ constexpr double kPivot = 1e-12;
 //
 //  Chebyshev basis (I.cheb, the rule is cheb_rule's): the Krylov vectors are
 //  K_j = T_j((A - theta) / delta) r0 for the interval [theta - delta, theta +
-//  delta] that Gershgorin's theorem gives for A, a basis well enough conditioned
-//  to be used without orthogonalising it.  Column j is ONE pass over the voxels
+//  delta] that Gershgorin's theorem gives for A (isotropic rows; a heuristic for
+//  anisotropic ones, see make_dev), a basis well enough conditioned to be used
+//  without orthogonalising it.  Column j is ONE pass over the voxels
 //  (K_{j+1} from K_j and K_{j-1}, and its dots with every K_i) and ONE team
 //  barrier.  From the Gram matrix G of the dots (FP64) every CTA keeps
 //  W = R^-T, G = R^T R, and z = W t, t_i = T_i(-theta / delta): with the
@@ -2121,7 +2124,7 @@ __global__ void nb_slot_kinds(long long n, const int32_t* nb, const T* coef, con
 }
 
 // Largest over the rows of (diagonal of -L) + (sum of its off-diagonal
-// magnitudes), the bound Gershgorin's theorem gives for the eigenvalues of -L;
+// magnitudes), the upper bound Gershgorin's theorem gives for the eigenvalues of -L;
 // rounded up to FP32, whose bit patterns of non-negative values order as
 // integers (NaN above all).
 template <typename T>
@@ -2516,7 +2519,12 @@ InstDev<T> make_dev(const InstHost& h, int vpt, bool compact_nb) {
     I.stride = h.d.sample_stride;
     I.n_samples = h.d.n_samples;
     I.save_h = h.d.save_h;
-    // A = I - dt/2 L has its eigenvalues in 1 + [0, 2 hg]
+    // Isotropic rows: A = I - dt/2 L has its eigenvalues in 1 + [0, 2 hg] (its rows are
+    // those of a symmetric matrix scaled by c_n >= 0).  With cross terms the
+    // off-diagonal magnitudes exceed the diagonal and the rows are not symmetric, so
+    // eigenvalues below 1 or off the real axis are not excluded: the interval is a
+    // heuristic there, the columns may grow outside it, and the test for a lost Gram
+    // matrix is what guards the solve (fibre shells: column counts are Arnoldi's)
     const double hg = 0.5 * (0.5 * h.d.dt) * h.bound;
     const double delta = std::max(hg, 1.0 / 16), theta = 1.0 + hg;
     I.cheb = cheb_rule(h.d.full_cycles != 0, h.m, hg) ? 1 : 0;

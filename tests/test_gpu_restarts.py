@@ -134,3 +134,20 @@ def test_full_cycles_true_residual(name, restart, cuda_device):
     # to 20 terms of |A| |u|, below 4 |b|: 20 * 1.1e-16 * 4 would be the worst row, the norm over
     # random signs is sqrt(20) of it) and of u* on the two sides
     np.testing.assert_array_less(np.linalg.norm(r), (2e-15 if restart > 8 else 2e-13) * np.linalg.norm(b))
+
+
+# Anisotropic rows, where the interval of the Chebyshev basis is a heuristic: the
+# columns and the results of Arnoldi (restart 21, early exit, dt 0.2: beyond the rule)
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_chebyshev_and_arnoldi_agree_on_fibre_rows(dtype, cuda_device):
+    steps = 20
+    (n, P, geom, sp, ap), pdur = gpu_cases.small_shell_ms(dt=0.2, fibres=True)
+    ub, ib = _steps(((n, P, geom, sp, ap), pdur), dtype, 21, steps, tol=1e-7, atol=1e-5)
+    ua, ia = _steps(((n, P, geom, sp, ap), pdur), dtype, 20, steps, tol=1e-7, atol=1e-5)
+    assert ia["nonconverged"] == ib["nonconverged"] == 0 and ia["max_arnoldi"] <= 20
+    # the same spaces and the same test: the counts differ where an estimate falls on the tolerance
+    assert abs(ia["arnoldi_steps"] - ib["arnoldi_steps"]) <= max(2, 0.02 * ib["arnoldi_steps"])
+    # each solve leaves a residual of at most 1e-5 (atol) or 1e-7 ||b||, below 1e-5: twice that per step
+    # and an upstroke's growth of exp(0.2 / 0.3) a step, in sum below 1.2e6 over 20 steps at worst; the
+    # excited voxels here take under 5 steps to rise, 60 in sum
+    np.testing.assert_allclose(ua, ub, rtol=0, atol=20 * 60 * 2e-5)
