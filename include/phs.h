@@ -146,8 +146,16 @@ int phs_instance_read_history(phs_engine* eng, int slot, int32_t s0, int32_t cou
 /* Copy the current state u, h ([n] each, engine precision) and the activation
  * step table lat ([n] int32, -1 = not activated) to host.  Any may be NULL.    */
 int phs_instance_read_state(phs_engine* eng, int slot, void* u_dst, void* h_dst, int32_t* lat_dst);
-/* Device pointers of an instance's state (for device-side consumers). */
+/* Device pointers of an instance's state (for device-side consumers).  The first
+ * call for an instance moves the three arrays into cudaMalloc memory of their own
+ * (after a device synchronisation; the addresses stay until the instance is
+ * removed), so that they can be read by peers (cudaDeviceEnablePeerAccess) and
+ * exported (cudaIpcGetMemHandle).                                              */
 int phs_instance_device_ptrs(phs_engine* eng, int slot, void** u, void** hist_u, int32_t** lat);
+/* The same addresses where they are, for use by this process on the engine's
+ * device: the arrays may lie in the library's memory pool, and a later
+ * phs_instance_device_ptrs moves them.                                          */
+int phs_instance_device_views(phs_engine* eng, int slot, void** u, void** hist_u, int32_t** lat);
 /* Number of kernel launches the engine issued since creation. */
 int64_t phs_engine_launch_count(phs_engine* eng);
 /* Engine settings.  PHS_CFG_VARIANT: step-kernel variant index (-1 = default);

@@ -152,6 +152,8 @@ SIGNATURES = {
                                                c_int32_p]),
     "phs_instance_device_ptrs": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.POINTER(ctypes.c_void_p),
                                                 ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(c_int32_p)]),
+    "phs_instance_device_views": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.POINTER(ctypes.c_void_p),
+                                                ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(c_int32_p)]),
     "phs_engine_launch_count": (ctypes.c_int64, [ctypes.c_void_p]),
     "phs_engine_config": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_int64]),
     "phs_step_variants": (ctypes.c_int, [ctypes.c_int, c_int32_p, c_int32_p, c_int32_p]),

@@ -1958,6 +1958,7 @@ const void* step_fn(int variant, bool edge = false) {
 struct InstHost {
     bool used = false;
     bool finished = false;
+    bool exported = false;       // u, hist_u and lat are allocations of their own (export_arrays)
     phs_instance_desc d{};
     long long n = 0;
     long long ldv = 0;           // padded voxel count: length of every per-voxel array
@@ -2012,6 +2013,13 @@ struct DeviceGuard {
 };
 
 void free_inst(InstHost& h) {
+    if (h.exported) {
+        cudaFree(h.u);
+        cudaFree(h.hist_u);
+        cudaFree(h.lat);
+        h.u = h.hist_u = nullptr;
+        h.lat = nullptr;
+    }
     void* ptrs[] = {h.nb, h.nbr, h.nbase, h.coef, h.cw, h.m6, h.enb, h.ecf, h.ud, h.vflags, h.vparams, h.stim, h.u, h.h0, h.h1, h.x, h.b, h.V,
                     h.hist_u, h.hist_h, h.lat, h.part, h.sync, h.st, h.prof};
     for (void* p : ptrs) dev_free(p, 0);
@@ -2808,6 +2816,39 @@ int advance_impl(phs_engine* e, long long n_steps, int ctas_per_sm, cudaStream_t
     return worst;
 }
 
+// Moves the arrays whose addresses the caller asked for out of the pool into
+// cudaMalloc memory, which peers can be given access to and other processes a
+// handle of; pool memory has neither.  Only then: three cudaMalloc and cudaFree
+// calls per instance cost more than adding it otherwise does.  Where there is no
+// memory for them the arrays stay in the pool.
+void export_arrays(phs_engine* e, InstHost& h) {
+    if (h.exported) return;
+    DeviceGuard guard(e->device);
+    // a stream capture that another thread has under way is not disturbed
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const size_t es = (e->prec == PHS_PREC_F64) ? 8 : 4;
+    void* old[3] = {h.u, h.hist_u, h.lat};
+    const size_t bytes[3] = {(size_t)h.ldv * es, (size_t)std::max(h.d.n_samples, 1) * h.n * es, (size_t)h.ldv * 4};
+    void* p[3] = {nullptr, nullptr, nullptr};
+    cudaError_t ce = cudaDeviceSynchronize();
+    for (int i = 0; i < 3 && ce == cudaSuccess; ++i) ce = cudaMalloc(&p[i], bytes[i]);
+    for (int i = 0; i < 3 && ce == cudaSuccess; ++i) ce = cudaMemcpyAsync(p[i], old[i], bytes[i], cudaMemcpyDeviceToDevice, 0);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(0);
+    if (ce == cudaSuccess) {
+        for (void* q : old) dev_free(q, 0);
+        h.u = p[0];
+        h.hist_u = p[1];
+        h.lat = (int32_t*)p[2];
+        h.exported = true;
+        e->dirty = true;       // the launch plan holds the old addresses
+    } else {
+        for (void* q : p) cudaFree(q);
+        cudaGetLastError();
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+}
+
 }  // namespace
 
 // ====================================================================== C ABI
@@ -2932,9 +2973,19 @@ int phs_instance_read_state(phs_engine* e, int slot, void* u_dst, void* h_dst, i
     return PHS_OK;
 }
 
+int phs_instance_device_views(phs_engine* e, int slot, void** u, void** hist_u, int32_t** lat) {
+    if (!e || slot < 0 || slot >= (int)e->inst.size() || !e->inst[slot].used) return PHS_ERR_BAD_ARG;
+    const InstHost& h = e->inst[slot];
+    if (u) *u = h.u;
+    if (hist_u) *hist_u = h.hist_u;
+    if (lat) *lat = h.lat;
+    return PHS_OK;
+}
+
 int phs_instance_device_ptrs(phs_engine* e, int slot, void** u, void** hist_u, int32_t** lat) {
     if (!e || slot < 0 || slot >= (int)e->inst.size() || !e->inst[slot].used) return PHS_ERR_BAD_ARG;
     InstHost& h = e->inst[slot];
+    export_arrays(e, h);
     if (u) *u = h.u;
     if (hist_u) *hist_u = h.hist_u;
     if (lat) *lat = h.lat;

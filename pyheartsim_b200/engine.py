@@ -131,8 +131,8 @@ class BatchedEngine:
         u = ctypes.c_void_p()
         hist = ctypes.c_void_p()
         lat = _lib.c_int32_p()
-        _lib.check(_lib.lib().phs_instance_device_ptrs(self._h, slot, ctypes.byref(u), ctypes.byref(hist),
-                                                       ctypes.byref(lat)), "phs_instance_device_ptrs")
+        _lib.check(_lib.lib().phs_instance_device_views(self._h, slot, ctypes.byref(u), ctypes.byref(hist),
+                                                        ctypes.byref(lat)), "phs_instance_device_views")
         n = int(inst.n_voxel)
         tdt = torch.float32 if self.precision == _lib.PREC_F32 else torch.float64
         dev = torch.device("cuda", torch.cuda.current_device())
@@ -180,8 +180,8 @@ class BatchedEngine:
         u = ctypes.c_void_p()
         hist = ctypes.c_void_p()
         lat = _lib.c_int32_p()
-        _lib.check(_lib.lib().phs_instance_device_ptrs(self._h, slot, ctypes.byref(u), ctypes.byref(hist),
-                                                       ctypes.byref(lat)), "phs_instance_device_ptrs")
+        _lib.check(_lib.lib().phs_instance_device_views(self._h, slot, ctypes.byref(u), ctypes.byref(hist),
+                                                        ctypes.byref(lat)), "phs_instance_device_views")
         n = int(inst.n_voxel)
         S = int(info["samples"])
         dev = torch.device("cuda", torch.cuda.current_device())
