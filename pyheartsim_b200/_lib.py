@@ -5,6 +5,7 @@ fallback: if the library is missing every call raises, so a missing CUDA
 extension can never be mistaken for a working one.
 """
 import ctypes
+import hashlib
 import os
 import threading
 
@@ -212,6 +213,7 @@ SIGNATURES = {
 
 _lib = None
 _lock = threading.Lock()
+_revisions = {}
 
 
 class PhsError(RuntimeError):
@@ -245,6 +247,16 @@ def lib():
                 f.argtypes = args
             _lib = h
     return _lib
+
+
+def revision():
+    """Short digest of the library's file: names the kernels that a measurement
+    kept for later was made with."""
+    path = LIB_PATH
+    if path not in _revisions:
+        with open(path, "rb") as f:
+            _revisions[path] = hashlib.file_digest(f, "sha256").hexdigest()[:12]
+    return _revisions[path]
 
 
 def status_string(status):

@@ -9,7 +9,8 @@ way every run) and leaves the engine configured with it.  Each option is timed `
 its graph) and ranked by the median.  Tuning advances the instances like any
 other call (the steps are real work).
 
-Results are cached per GPU name and workload bucket (precision, total voxels
+Results are cached per GPU name, library (a digest of its file: a choice holds
+for the kernels it was measured with) and workload bucket (precision, total voxels
 rounded to a power of two, instance count): in the process, and in a JSON file
 (``PHS_AUTOTUNE_CACHE``, default ``~/.cache/pyheartsim_b200/autotune.json``)
 so later processes on the same machine start from the same choice.
@@ -59,7 +60,7 @@ def _store_file(key, best):
 
 def _bucket(engine):
     n = sum(engine.instance(s).n_voxel for s in engine.slots())
-    return "|".join(str(x) for x in (torch.cuda.get_device_name(), engine.precision,
+    return "|".join(str(x) for x in (torch.cuda.get_device_name(), _lib.revision(), engine.precision,
                                       1 << max(0, int(math.log2(max(n, 1)))), len(engine.slots())))
 
 
