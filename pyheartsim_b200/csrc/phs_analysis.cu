@@ -319,13 +319,14 @@ __global__ void cv_count(long long ne, const double* __restrict__ xyz, double r2
     }
 }
 
-// rows of electrode i at [off[i], off[i] + counts[i]) of five planes: x, y, z, 1, lat
-__global__ void cv_fill(long long ne, const double* __restrict__ xyz, const double* __restrict__ lat, double r2,
-                        const long long* __restrict__ off, const int32_t* __restrict__ counts, long long total,
-                        double* __restrict__ ws) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ne; i += (long long)gridDim.x * blockDim.x) {
+// rows of the b-th electrode of the list, i = ids[b], at [off[b], off[b] + counts[i])
+// of five planes: x, y, z, 1, lat
+__global__ void cv_fill(long long ne, long long nb, const int32_t* __restrict__ ids, const double* __restrict__ xyz,
+                        const double* __restrict__ lat, double r2, const long long* __restrict__ off,
+                        const int32_t* __restrict__ counts, long long total, double* __restrict__ ws) {
+    for (long long b = blockIdx.x * (long long)blockDim.x + threadIdx.x; b < nb; b += (long long)gridDim.x * blockDim.x) {
         long long k = 0;
-        const long long o = off[i], cnt = counts[i];
+        const long long i = ids[b], o = off[b], cnt = counts[i];
         for (long long j = 0; j < ne && k < cnt; ++j) {
             if (dist2(xyz + 3 * i, xyz + 3 * j) <= r2) {
                 const long long r = o + k;
@@ -360,16 +361,17 @@ __device__ __forceinline__ void block_sum3(double& a, double& b, double& c, doub
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kAThreads) cv_solve(long long ne, const long long* __restrict__ off,
+__global__ void __launch_bounds__(kAThreads) cv_solve(long long nb, const int32_t* __restrict__ ids,
+                                                      const long long* __restrict__ off,
                                                       const int32_t* __restrict__ counts, long long total,
                                                       double* __restrict__ ws, double* __restrict__ vvec,
                                                       double* __restrict__ vmag) {
     __shared__ double red[3][kAThreads];
     __shared__ double V[4][4];
     __shared__ double rot[2];
-    const long long i = blockIdx.x;
-    if (i >= ne) return;
-    const long long m = counts[i], o = off[i];
+    const long long b = blockIdx.x;
+    if (b >= nb) return;
+    const long long i = ids[b], m = counts[i], o = off[b];
     if (m < 4) {
         if (threadIdx.x == 0) {
             vvec[3 * i] = vvec[3 * i + 1] = vvec[3 * i + 2] = nan("");
@@ -463,14 +465,20 @@ __global__ void __launch_bounds__(kAThreads) cv_solve(long long ne, const long l
 // Jacobi SVD of R, whose singular values are those of the system.  Before, a
 // count, a download of the counts, an upload of offsets, a fill and a CTA-wide
 // Jacobi over the m rows (a block reduction per column pair) took 1.08 ms for
-// 2048 electrodes; now 0.2 ms, call and transfers included.  An electrode with
-// more than kCvRows rows sets *big and the caller falls back to that form, which
-// has no limit.
+// 2048 electrodes; now 0.2 ms, call and transfers included.  counts[i] is the
+// number of rows; an electrode with more than kCvRows of them sets *big and is
+// left to that form, which has no limit.
 constexpr int kCvRows = 512, kCvWarps = 2, kCvAhead = 4;
+// Most electrodes for which the warps search: every warp reads all candidates, a
+// thread of cv_count shares its reads with its warp.  Call, ms, this form (with the
+// general one for the electrodes above kCvRows) and the general one alone: 131072
+// electrodes with 60 neighbours 40 / 59, 262144 158 / 179, 524288 624 / 584 and with
+// 600 neighbours 1091 / 726; 65536 with 600 neighbours 37 / 44.
+constexpr long long kCvWarpElectrodes = 1 << 17;
 __global__ void __launch_bounds__(32 * kCvWarps) cv_warp(long long ne, const double* __restrict__ xyz,
                                                          const double* __restrict__ lat, double r2,
                                                          double* __restrict__ vvec, double* __restrict__ vmag,
-                                                         unsigned int* __restrict__ big) {
+                                                         int32_t* __restrict__ counts, unsigned int* __restrict__ big) {
     __shared__ double sm[kCvWarps][5][kCvRows];
     const int lane = threadIdx.x & 31;
     double(*col)[kCvRows] = sm[threadIdx.x >> 5];
@@ -502,6 +510,7 @@ __global__ void __launch_bounds__(32 * kCvWarps) cv_warp(long long ne, const dou
             m += __popc(mask);
         }
     }
+    if (lane == 0) counts[i] = m;
     if (m > kCvRows) {
         if (lane == 0) atomicOr(big, 1u);
         return;
@@ -692,68 +701,67 @@ int phs_conduction_velocity(int64_t ne, const double* xyz, const double* lat, do
     if (ne <= 0 || ne > (1 << 20) || !xyz || !lat || !v_vec || !v_mag || !(radius >= 0.0)) return PHS_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     const double r2 = radius * radius;
-    {
-        // one warp per electrode; the general form below only when a
-        // neighbourhood does not fit its shared memory
-        unsigned int* big = nullptr;
-        unsigned int h_big = 0;
-        cudaError_t e = dev_alloc((void**)&big, sizeof(unsigned int), s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(big, 0, sizeof(unsigned int), s);
+    int32_t *counts = nullptr, *ids = nullptr;   // counts[ne]: the word that cv_warp sets
+    long long* off = nullptr;
+    double* ws = nullptr;
+    auto done = [&](cudaError_t e) {
+        dev_free(ws, s);
+        dev_free(off, s);
+        dev_free(ids, s);
+        dev_free(counts, s);
+        const cudaError_t se = cudaStreamSynchronize(s);
+        if (e == cudaSuccess) e = se;
+        if (e == cudaSuccess) return (int)PHS_OK;
+        set_last_error("phs_conduction_velocity", e);
+        return (int)(e == cudaErrorMemoryAllocation ? PHS_ERR_OOM : PHS_ERR_CUDA);
+    };
+    const bool warps = ne <= kCvWarpElectrodes;
+    unsigned int h_big = 1;
+    cudaError_t e = dev_alloc((void**)&counts, ((size_t)ne + 1) * sizeof(int32_t), s);
+    if (e == cudaSuccess && warps) {
+        unsigned int* big = (unsigned int*)(counts + ne);
+        e = cudaMemsetAsync(big, 0, sizeof(unsigned int), s);
         if (e == cudaSuccess) {
             cv_warp<<<(unsigned int)((ne + kCvWarps - 1) / kCvWarps), 32 * kCvWarps, 0, s>>>(ne, xyz, lat, r2, v_vec,
-                                                                                             v_mag, big);
+                                                                                             v_mag, counts, big);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(&h_big, big, sizeof(h_big), cudaMemcpyDeviceToHost, s);
-        dev_free(big, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
-            set_last_error("phs_conduction_velocity", e);
-            return e == cudaErrorMemoryAllocation ? PHS_ERR_OOM : PHS_ERR_CUDA;
-        }
-        if (!h_big) return PHS_OK;
-    }
-    int32_t* counts = nullptr;
-    long long* off = nullptr;
-    double* ws = nullptr;
-    auto done = [&](int rc) {
-        dev_free(ws, s);
-        dev_free(off, s);
-        dev_free(counts, s);
-        cudaStreamSynchronize(s);
-        return rc;
-    };
-    cudaError_t e = dev_alloc((void**)&counts, (size_t)ne * sizeof(int32_t), s);
-    if (e == cudaSuccess) {
+    } else if (e == cudaSuccess) {
         cv_count<<<blocks_for(ne), kAThreads, 0, s>>>(ne, xyz, r2, counts);
         e = cudaGetLastError();
     }
-    std::vector<int32_t> h_counts((size_t)ne);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_counts.data(), counts, (size_t)ne * sizeof(int32_t),
-                                              cudaMemcpyDeviceToHost, s);
+    if (e != cudaSuccess) return done(e);
+    if (!h_big) {                  // the stream has finished
+        dev_free(counts, s);
+        return PHS_OK;
+    }
+    // the general form, for the electrodes that are left
+    std::vector<int32_t> h_counts((size_t)ne), h_ids;
+    e = cudaMemcpyAsync(h_counts.data(), counts, (size_t)ne * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) { set_last_error("phs_conduction_velocity", e); return done(PHS_ERR_CUDA); }
-    std::vector<long long> h_off((size_t)ne);
+    if (e != cudaSuccess) return done(e);
+    std::vector<long long> h_off;
     long long total = 0;
     for (long long i = 0; i < ne; ++i) {
-        h_off[(size_t)i] = total;
+        if (warps && h_counts[(size_t)i] <= kCvRows) continue;
+        h_ids.push_back((int32_t)i);
+        h_off.push_back(total);
         total += h_counts[(size_t)i];
     }
-    e = dev_alloc((void**)&off, (size_t)ne * sizeof(long long), s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(off, h_off.data(), (size_t)ne * sizeof(long long),
-                                              cudaMemcpyHostToDevice, s);
+    const long long nb = (long long)h_ids.size();
+    e = dev_alloc((void**)&ids, (size_t)nb * sizeof(int32_t), s);
+    if (e == cudaSuccess) e = dev_alloc((void**)&off, (size_t)nb * sizeof(long long), s);
     if (e == cudaSuccess) e = dev_alloc((void**)&ws, (size_t)(5 * (total > 0 ? total : 1)) * sizeof(double), s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(ids, h_ids.data(), (size_t)nb * sizeof(int32_t), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(off, h_off.data(), (size_t)nb * sizeof(long long), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
-        cv_fill<<<blocks_for(ne), kAThreads, 0, s>>>(ne, xyz, lat, r2, off, counts, total, ws);
-        cv_solve<<<(unsigned int)ne, kAThreads, 0, s>>>(ne, off, counts, total, ws, v_vec, v_mag);
+        cv_fill<<<blocks_for(nb), kAThreads, 0, s>>>(ne, nb, ids, xyz, lat, r2, off, counts, total, ws);
+        cv_solve<<<(unsigned int)nb, kAThreads, 0, s>>>(nb, ids, off, counts, total, ws, v_vec, v_mag);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) {
-        set_last_error("phs_conduction_velocity", e);
-        return done(e == cudaErrorMemoryAllocation ? PHS_ERR_OOM : PHS_ERR_CUDA);
-    }
-    return done(PHS_OK);
+    return done(e);
 }
 
 }  // extern "C"
