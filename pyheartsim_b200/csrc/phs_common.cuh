@@ -22,6 +22,10 @@ void set_last_message(const char* msg);
 // one stream is used on another only after a synchronisation or an event wait.
 cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t stream);
 void dev_free(void* p, cudaStream_t stream);
+// The opt-in of kernel `fn` to `bytes` of dynamic shared memory, which holds per
+// context: made once in each (so a call under capture that follows one outside
+// makes no such call).
+cudaError_t allow_dynamic_smem(const void* fn, size_t bytes);
 // Sets how much the pool keeps; `engines`: engines made (+1) or destroyed (-1).
 void pool_update(int engines);
 

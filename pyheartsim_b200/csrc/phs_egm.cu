@@ -13,7 +13,6 @@
 #include <math.h>
 #include <stdint.h>
 #include <algorithm>
-#include <mutex>
 #include <vector>
 
 #include "../../include/phs.h"
@@ -312,23 +311,10 @@ static cudaError_t contract_launch(int64_t T, int64_t n_v, int64_t n_e, const do
     const dim3 grid((unsigned)((T + DG_BM - 1) / DG_BM), (unsigned)((n_e + DG_BN - 1) / DG_BN), (unsigned)splits);
     const bool wide = (((uintptr_t)V | (uintptr_t)Mt) & 15) == 0 && ldv % 2 == 0 && n_v % 2 == 0;
     const auto fn = wide ? dgemm_tn_kernel<16> : dgemm_tn_kernel<8>;
-    {
-        // both kernels' shared-memory opt-in, once per device (so a call under
-        // capture that follows one outside makes no such call)
-        static std::mutex mu;
-        static bool set[64] = {};
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e != cudaSuccess) return e;
-        std::lock_guard<std::mutex> lk(mu);
-        if (dev < 0 || dev >= 64 || !set[dev]) {
-            e = cudaFuncSetAttribute(dgemm_tn_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DG_SMEM);
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(dgemm_tn_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DG_SMEM);
-            if (e != cudaSuccess) return e;
-            if (dev >= 0 && dev < 64) set[dev] = true;
-        }
-    }
+    // both kernels' opt-in, whichever this call launches
+    cudaError_t e = allow_dynamic_smem((const void*)dgemm_tn_kernel<16>, DG_SMEM);
+    if (e == cudaSuccess) e = allow_dynamic_smem((const void*)dgemm_tn_kernel<8>, DG_SMEM);
+    if (e != cudaSuccess) return e;
     fn<<<grid, 256, DG_SMEM, stream>>>(T, n_e, n_v, V, ldv, Mt, n_v, P, kchunk);
     const int64_t MN = T * n_e;
     splitk_reduce_kernel<double><<<(unsigned)std::min<int64_t>((MN + 31) / 32, 4736), 256, 0, stream>>>(MN, (int)splits,

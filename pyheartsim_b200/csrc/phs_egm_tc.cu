@@ -658,18 +658,7 @@ int contract_bf16x3(int64_t T, int64_t n_e, int64_t T_pad, int64_t E_pad, int64_
     int* err = (int*)work;
     float* part = (float*)((char*)work + kTcHeader);
     PHS_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), stream));
-    // the dynamic shared-memory opt-in is a per-device attribute of each kernel
-    {
-        static std::mutex mu;
-        static bool attr_set[64][kTcNumConfigs] = {};
-        int dev = 0;
-        PHS_CUDA_TRY(cudaGetDevice(&dev));
-        std::lock_guard<std::mutex> lk(mu);
-        if (dev < 0 || dev >= 64 || !attr_set[dev][config]) {
-            PHS_CUDA_TRY(cudaFuncSetAttribute(c.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem));
-            if (dev >= 0 && dev < 64) attr_set[dev][config] = true;
-        }
-    }
+    PHS_CUDA_TRY(allow_dynamic_smem(c.fn, c.smem));
     dim3 grid((unsigned)(T_pad / TC_BM), (unsigned)(Ew / c.bn), (unsigned)splits);
     int nkb_total = (int)(K_pad / c.bk), T_pad_i = (int)T_pad, Ew_i = (int)Ew;
     void* args[] = {(void*)&mv_hi, (void*)&mv_lo, (void*)&mm_hi, (void*)&mm_lo, (void*)&nkb_total, (void*)&per,

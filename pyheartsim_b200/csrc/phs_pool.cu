@@ -1,4 +1,4 @@
-// Device memory of the library: one stream-ordered pool per device.
+// Device memory of the library: one stream-ordered pool per device and context.
 //
 // cudaMalloc and cudaFree cost 0.05-0.2 ms each here and cudaFree now and then
 // much more (an engine of 24 instances, ~30 arrays each, took 170-300 ms to
@@ -11,14 +11,18 @@
 // next synchronisation.
 //
 // The pool is the library's own, so the device's default pool keeps the
-// caller's settings.  It is found by device and context (a device reset makes a
-// new context and so a new pool).  A stream that is being captured allocates
+// caller's settings.  It is found by device and context (a program may have
+// several contexts on a device; a device reset makes a new one, and ids are not
+// used again).  A stream that is being captured allocates
 // from the default pool as any cudaMallocAsync does: the graph owns that
 // memory.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
+#include <map>
 #include <mutex>
+#include <set>
+#include <utility>
 
 #include "../../include/phs.h"
 #include "phs_common.cuh"
@@ -26,17 +30,15 @@
 namespace phs {
 namespace {
 
-constexpr int kMaxDevices = 64;
 constexpr unsigned long long kKeepEngine = 4ull << 30;
 constexpr unsigned long long kKeepIdle = 512ull << 20;
 
 struct DevicePool {
-    unsigned long long ctx = 0;
     cudaMemPool_t pool = nullptr;
     int engines = 0;
 };
 std::mutex g_pool_mu;
-DevicePool g_pool[kMaxDevices];
+std::map<std::pair<int, unsigned long long>, DevicePool> g_pool;   // by device and context
 
 bool context_id(unsigned long long* id) {
     static PFN_cuCtxGetId_v12000 fn = nullptr;
@@ -72,12 +74,12 @@ struct RelaxedCapture {
 DevicePool* current_pool() {
     RelaxedCapture relaxed;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
     if (cudaFree(nullptr) != cudaSuccess) return nullptr;   // the context exists from here on
     unsigned long long ctx = 0;
     if (!context_id(&ctx)) return nullptr;
-    DevicePool& d = g_pool[dev];
-    if (d.pool != nullptr && d.ctx == ctx) return &d;
+    const auto it = g_pool.find({dev, ctx});
+    if (it != g_pool.end()) return &it->second;
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -87,7 +89,8 @@ DevicePool* current_pool() {
         cudaGetLastError();
         return nullptr;
     }
-    d = DevicePool{ctx, pool, 0};
+    DevicePool& d = g_pool[{dev, ctx}];
+    d.pool = pool;
     set_threshold(d);
     return &d;
 }
@@ -109,6 +112,18 @@ cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t stream) {
 
 void dev_free(void* p, cudaStream_t stream) {
     if (p) cudaFreeAsync(p, stream);
+}
+
+cudaError_t allow_dynamic_smem(const void* fn, size_t bytes) {
+    static std::mutex mu;
+    static std::set<std::pair<unsigned long long, const void*>> done;
+    unsigned long long ctx = 0;
+    std::lock_guard<std::mutex> lk(mu);
+    const bool known = context_id(&ctx);
+    if (known && done.count({ctx, fn})) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess && known) done.insert({ctx, fn});
+    return e;
 }
 
 void pool_update(int engines) {
