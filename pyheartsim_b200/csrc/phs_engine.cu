@@ -2335,7 +2335,11 @@ int add_instance(phs_engine* e, const phs_instance_desc* d, int* slot) {
     // a tile's slice of any of them can be copied whole
     const size_t np = (n + kPadVoxels - 1) / kPadVoxels * kPadVoxels;
     h.ldv = (long long)np;
-    auto fail = [&](int code) { free_inst(h); return code; };
+    auto fail = [&](int code) {
+        free_inst(h);
+        cudaStreamSynchronize(0);
+        return code;
+    };
 #define PHS_ALLOC(ptr, bytes)                                            \
     do {                                                                 \
         cudaError_t _e = dev_alloc((void**)&(ptr), (bytes), 0);          \
@@ -2898,6 +2902,7 @@ int phs_engine_destroy(phs_engine* e) {
     dev_free(e->d_desc, 0);
     dev_free(e->d_map, 0);
     pool_update(-1);
+    cudaStreamSynchronize(0);   // the driver has what the pool does not keep
     delete e;
     return PHS_OK;
 }
@@ -2913,6 +2918,7 @@ int phs_instance_remove(phs_engine* e, int slot) {
     cudaDeviceSynchronize();
     free_inst(e->inst[slot]);
     pool_update(0);
+    cudaStreamSynchronize(0);   // the driver has what the pool does not keep
     e->dirty = true;
     e->auto_left = 2;
     e->auto_mark = e->launches;

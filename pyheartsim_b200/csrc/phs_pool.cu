@@ -7,8 +7,9 @@
 // synchronisation, so a contraction that allocates its partial sums paid 4-5 ms
 // per call for 1.5 ms of kernels.  This pool keeps a bounded amount instead:
 // what is allocated plus kKeepEngine bytes while an engine of the device is
-// alive, plus kKeepIdle bytes otherwise; the driver returns the rest at the
-// next synchronisation.
+// alive, plus kKeepIdle bytes otherwise; the driver takes the rest back at the
+// next synchronisation, which the calls that remove an instance or destroy an
+// engine make at their end, so other allocators find it when they return.
 //
 // The pool is the library's own, so the device's default pool keeps the
 // caller's settings.  It is found by device and context (a program may have
