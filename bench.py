@@ -33,7 +33,7 @@ METRIC = "voxel-steps/s batched FP32 vs plain FP64 on 1 B200 at LAT err<=dt; p99
 DEFAULT_F32_VARIANT = 7        # the engine's FP32 default when the autotuner is off
 # DRAM bytes per voxel-step of step_kernel measured by ncu (dram__bytes_read.sum +
 # dram__bytes_write.sum of two full-size launches of a 64-shell batch, 2.98
-# columns per step, profiles/step_kernel_64shells_dram_fullsize.md), for
+# columns per step; the capture's summary is in profiles/), for
 # the variants that read the int32 neighbour table and those that read the
 # compact one; multiplied by the voxels and steps of one launch below.
 STEP_TRAFFIC_BYTES_PER_VOXEL_STEP = {"int32": 210.4, "compact": 144.8}
@@ -348,8 +348,72 @@ def run_b200(args):
         import torch.distributed as dist
         dist.destroy_process_group()
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        print(json.dumps(line), file=sys.stderr, flush=True)       # every leg in full
+        print(json.dumps(short_line(line), allow_nan=False), flush=True)
     return 0
+
+
+# Figures of the legs that go into the printed line, by key path
+LINE_KEYS = {
+    "autotune": ("variant", "ctas_per_sm"),
+    "solver": ("arnoldi_per_step",),
+    "roofline": ("bound", "achieved", "peak", "unit", "frac", "peak_source", "traffic", "kernel", "bytes_per_voxel_step"),
+    "phases_ms_per_step": ("cta_utilization", "barriers_per_step"),
+    "e2e": ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "seconds", "run_only_value"),
+    "e2e_dropin_c1": ("plain_fp64.simulate_s", "fast_fp32.simulate_s"),
+    "plain_fp64": ("value", "ms_per_step", "voxels", "speedup_batched_fp32"),
+    "anisotropic": ("value", "ms_per_step", "voxels"),
+    "geometry": ("device_s", "host_numpy_s"),
+    "serving": ("p50_latency_s", "p99_latency_s", "throughput_voxel_steps_s"),
+    "serving_half_load": ("p50_latency_s", "p99_latency_s", "throughput_voxel_steps_s"),
+    "electrogram": ("bf16x3_ms", "executed_tflops", "fp64_contract_ms", "leadfield_ms", "rel_l2_bf16x3_vs_fp64"),
+    "cpu_baseline": ("value", "unit", "cores", "kind", "sample"),
+}
+
+
+def short_line(line):
+    """The printed line: every scalar and the configuration as they are, of the
+    legs the figures of LINE_KEYS, numbers to seven digits and non-finite ones as
+    null.  The whole of every leg makes a line of tens of kilobytes, which a
+    log that keeps a few thousand characters of output loses the head of."""
+    def num(v):
+        if isinstance(v, dict):
+            return {k: num(x) for k, x in v.items()}
+        if isinstance(v, (list, tuple)):
+            return [num(x) for x in v]
+        if isinstance(v, float):
+            return float(f"{v:.7g}") if np.isfinite(v) else None
+        return v
+
+    out = {}
+    for k, v in line.items():
+        if k == "accuracy":
+            out[k] = accuracy_summary(v)
+        elif k in LINE_KEYS and isinstance(v, dict):
+            out[k] = {}
+            for path in LINE_KEYS[k]:
+                x = v
+                for part in path.split("."):
+                    x = x.get(part) if isinstance(x, dict) else None
+                if x is not None:
+                    out[k][path] = x
+        else:
+            out[k] = v
+    return num(out)
+
+
+def accuracy_summary(acc):
+    """First-activation errors (steps) and max |dVm| of each configuration."""
+    def pick(r):
+        f = r.get("first") or {}
+        return {"first_max_dlat_steps": f.get("max_dlat_steps"), "first_p99_dlat_steps": f.get("p99_dlat_steps"),
+                "max_abs_dvm": r.get("max_abs_dvm_1khz")}
+
+    out = {k: pick(v) for k, v in acc.items() if isinstance(v, dict)}
+    c3 = [r["first_max_dlat_steps"] for r in acc.get("c3_sample", []) if r["first_max_dlat_steps"] is not None]
+    if c3:
+        out["c3_first_max_dlat_steps"] = max(c3)
+    return out
 
 
 def step_variant_of(tune):
