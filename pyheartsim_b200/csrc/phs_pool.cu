@@ -104,11 +104,15 @@ cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t stream) {
         const cudaError_t e = cudaStreamIsCapturing(stream, &cap);
         if (e != cudaSuccess) return e;
     }
+    cudaMemPool_t pool = nullptr;
     if (cap == cudaStreamCaptureStatusNone) {
         std::lock_guard<std::mutex> lk(g_pool_mu);
-        if (DevicePool* d = current_pool()) return cudaMallocFromPoolAsync(p, bytes, d->pool, stream);
+        if (DevicePool* d = current_pool()) pool = d->pool;
     }
-    return cudaMallocAsync(p, bytes, stream);
+    const cudaError_t e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, stream) : cudaMallocAsync(p, bytes, stream);
+    // the caller reports it; the check after a later call's launches must not find it
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    return e;
 }
 
 void dev_free(void* p, cudaStream_t stream) {
