@@ -298,7 +298,10 @@ constexpr int TP_STAGES = 3, TP_BK = 64, TP_BN = 256;
 constexpr int TP_TILE_BYTES = TC_BM * TP_BK * 2;           // 128 rows of one part
 constexpr int TP_STAGE_BYTES = 4 * TP_TILE_BYTES;          // V hi, lo and M hi, lo of one CTA
 constexpr size_t TP_SMEM = (size_t)TP_STAGES * TP_STAGE_BYTES + 1024 + 256;
-constexpr uint32_t kLeaderMask = 0xFEFFFFFFu;              // a shared address of the pair -> the even CTA's
+// In the shared::cluster window bit 24 of an address is the low bit of the CTA's
+// rank: cleared, an address of either CTA of a pair is that of the even one (the form
+// that CUTLASS's public sm100 copies use for the barrier of a cta_group::2 load).
+constexpr uint32_t kLeaderMask = 0xFEFFFFFFu;
 
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
     asm volatile(

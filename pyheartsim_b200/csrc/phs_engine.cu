@@ -50,7 +50,6 @@ struct alignas(128) TeamSync {
 };
 
 enum Action : int {
-    ACT_NONE = 0,
     ACT_ZERO_B = 1,      // ||b|| == 0: the solve returns b
     ACT_DONE = 2,        // residual test passed: the solve returns x
     ACT_CYCLE = 3,       // start an Arnoldi cycle (V0 holds r, s[0] = 1/||r||)
@@ -59,8 +58,6 @@ enum Action : int {
     ACT_UPDATE_CHECK = 6,// x += V y, then the true-residual test
     ACT_FAIL = 7,        // non-finite norm: instance retired with an error
 };
-
-enum Phase : int { PH_PLAIN = 0, PH_RHS = 1, PH_DOTS = 2, PH_NORM = 3, PH_CHECK = 4 };
 
 // Phase timer slots (nanoseconds of globaltimer, summed over steps).
 enum ProfSlot : int {
@@ -2105,7 +2102,7 @@ __global__ void check_tables(long long n, const int32_t* nb, const T* coef, cons
 
 // ---- compact neighbour table (decode_nb)
 // Whether slot k of row v has a neighbour the operator reads: its coefficient
-// is nonzero, the test lap_row makes.
+// is nonzero, the test tile_lap makes.
 template <typename T>
 __device__ __forceinline__ bool nb_present(const T* coef, const T* cw, const uint8_t* m6, long long v, int k) {
     if (cw) return ((m6[v] >> k) & 1u) && cw[v] != T(0);
@@ -2447,9 +2444,11 @@ int add_instance(phs_engine* e, const phs_instance_desc* d, int* slot) {
         if (dev_alloc((void**)&h.prof, kProfSlots * sizeof(unsigned long long), 0) == cudaSuccess)
             cudaMemset(h.prof, 0, kProfSlots * sizeof(unsigned long long));
     }
-    // columns per step until they are known (cost model of the first launch): the
-    // batches' Mitchell-Schaeffer shells (hg 0.94) take 4.7, the Aliev-Panfilov
-    // ones (hg 0.6) 1.8
+    // columns per step until they are known.  A guess for the team sizes of the first
+    // launch only, through the two stiffnesses at hand (Mitchell-Schaeffer shells, hg
+    // 0.94: 4.7, Aliev-Panfilov, hg 0.6: 1.8; 24 and 19 in full cycles): at another
+    // lattice constant or step it may be off by a factor, and the measured costs
+    // take its place at the first rebalancing
     const double hg = std::min(1.0, 0.25 * d->dt * h.bound);
     h.kavg = d->full_cycles ? 10.0 + 15.0 * hg : 1.0 + 4.4 * hg * hg * hg;
     e->inst[s] = h;
