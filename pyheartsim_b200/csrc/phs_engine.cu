@@ -2466,9 +2466,9 @@ int add_instance(phs_engine* e, const phs_instance_desc* d, int* slot) {
 // after 22-30 columns (hg 3 and 15, discs and rough residuals) or, for plane
 // fronts, after 10-17 (FP32 from hg 5, FP64 from hg 3 on at tol 1e-9).  Early
 // exit: with restarts of up to 20 columns a lost matrix costs little, the cycle
-// ends in a true residual and the solve goes on (64 x 64 sheet, plane front,
-// columns against Arnoldi's: none more at hg 3, 5 % at hg 5, 28 % at hg 15, 18 % at
-// hg 60, at half the passes per column).  Full cycles want rounding level: up to
+// ends in a true residual and the solve goes on (64 x 64 sheet, plane front, more
+// columns than Arnoldi's, FP32 at tol 1e-6 / FP64 at 1e-9: 1 / 30 % at hg 3, 6 / 13 %
+// at 5, 21 / 12 % at 15, 17 / 17 % at 60, at half the passes per column).  Full cycles want rounding level: up to
 // hg 1.25 (Mitchell-Schaeffer at 0.05 ms and 0.4 mm: 0.94) that takes 21-28
 // columns; beyond, Arnoldi.
 bool cheb_rule(bool full_cycles, int m, double hg) {
